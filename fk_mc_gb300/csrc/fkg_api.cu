@@ -214,16 +214,21 @@ static void stage_cb(void* c, int stage, int end) {
 
 // Enqueue one batched eigenvalue solve + logZ on ctx->st. Inputs already on the
 // device in ws.desc / ws.diag / ws.beta.
-int enqueue_solve(fkg_ctx* ctx, Workspace& ws, const Layout& L, bool want_exp, const StepIO* io) {
+int enqueue_solve(fkg_ctx* ctx, Workspace& ws, const Layout& L, bool want_exp, const StepIO* io, bool want_q) {
     const ChainDesc* dd = (const ChainDesc*)ws.desc.p;
     double* A = (double*)ws.A.p;
     bool two_stage = false;
     if (ctx->precision == FKG_PREC_F64) {
+        // with eigenvectors A holds the reflectors, else the tiles beyond shared memory
+        if (want_q) {
+            const int rc = ensure_dev(ctx, ws.tiles, sizeof(double) * (size_t)L.a_total);
+            if (rc) return rc;
+        }
         stage_begin(ctx, FKG_STAGE_REDUCE);
-        FKG_CUDA(ctx, launch_sytrd_v3_f64(dd, L.batch, L.max_ld, (const double*)ws.diag.p, A, (double*)ws.d.p,
-                                          (double*)ws.e.p, (double*)ws.tau.p, ctx->st, pick_variant(ctx, L, false),
-                                          (const int*)ws.order.p, (int*)ws.counter.p, ctx->num_sms,
-                                          (int*)ctx->status.p));
+        FKG_CUDA(ctx, launch_sytrd_f64(L.desc.data(), dd, L.batch, L.max_ld, (const double*)ws.diag.p,
+                                       want_q ? A : nullptr, want_q ? ws.tiles.p : ws.A.p, (double*)ws.d.p,
+                                       (double*)ws.e.p, (double*)ws.tau.p, ctx->st, pick_variant(ctx, L, false),
+                                       (const int*)ws.order.p, (int*)ws.counter.p, (int*)ctx->status.p));
         stage_end(ctx, FKG_STAGE_REDUCE);
         ctx->launches++;
     } else {
@@ -284,13 +289,13 @@ int enqueue_solve(fkg_ctx* ctx, Workspace& ws, const Layout& L, bool want_exp, c
     }
     stage_begin(ctx, FKG_STAGE_LOGZ);
     if (io)  // the proposal step: logZ, decision and state update in one launch
-        FKG_CUDA(ctx, launch_logz_accept(dd, L.batch, (const double*)ws.w.p, (const double*)ws.beta.p,
+        FKG_CUDA(ctx, launch_logz_accept(dd, L.batch, (double*)ws.w.p, (const double*)ws.beta.p,
                                          (double*)ws.logz.p, io->site, io->u, (const double*)ctx->ch_ebmf.p,
                                          (int32_t*)ctx->ch_f.p, (double*)ctx->ch_logz_cur.p,
                                          (double*)ctx->ch_w_cur.p, io->acc, io->dl, (int*)ctx->status.p, ctx->st,
                                          io->step));
     else
-        FKG_CUDA(ctx, launch_logz(dd, L.batch, L.max_n, (const double*)ws.w.p, (const double*)ws.beta.p,
+        FKG_CUDA(ctx, launch_logz(dd, L.batch, L.max_n, (double*)ws.w.p, (const double*)ws.beta.p,
                                   (double*)ws.logz.p, want_exp ? (double*)ws.exp_e.p : nullptr,
                                   want_exp ? (double*)ws.fermi.p : nullptr, (int*)ctx->status.p, ctx->st));
     stage_end(ctx, FKG_STAGE_LOGZ);
@@ -326,6 +331,56 @@ int check_status(fkg_ctx* ctx) {
     if (h & kStatusNoConverge) return set_err(ctx, FKG_ERR_NUMERIC, "an eigenvalue iteration did not converge");
     if (h & kStatusTimeout) return set_err(ctx, FKG_ERR_TIMEOUT, "a bounded device wait ran out");
     if (h & kStatusBadArg) return set_err(ctx, FKG_ERR_ARG, "a device-side argument check failed");
+    return FKG_OK;
+}
+
+// fkg_eigh_logz without eigenvectors; want_q: the reduction's reflectors are
+// kept, so that enqueue_vectors can follow (FP64 path).
+static int eigh_values(fkg_ctx* ctx, int batch, const int32_t* lattice_id, const double* diag, const double* beta,
+                       double* evals, double* exp_e, double* fermi, double* logz, bool want_q) {
+    if (!diag || !beta) return set_err(ctx, FKG_ERR_ARG, "diag/beta is NULL");
+    Layout& L = ctx->solve_layout;
+    int rc;
+    if ((rc = make_layout(ctx, batch, lattice_id, L))) return rc;
+    const bool want_exp = exp_e || fermi;
+    if ((rc = ensure_solve_ws(ctx, ctx->solve, L, want_exp))) return rc;
+    const size_t V = (size_t)L.v_total;
+    // pinned staging: diag (V) + beta (batch) in; evals, exp, fermi (3V) + logz (batch) out
+    if ((rc = ensure_pinned(ctx, sizeof(double) * (4 * V + 2 * batch)))) return rc;
+    double* hin = (double*)ctx->pin;
+    double* hb = hin + V;
+    double* hout = hb + batch;
+    long long src = 0;
+    for (int c = 0; c < batch; ++c) {
+        const ChainDesc& d = L.desc[c];
+        for (int i = 0; i < d.ld; ++i) hin[d.v_off + i] = i < d.n ? diag[src + i] : 0.0;
+        if (!(beta[c] > 0.0) || beta[c] - beta[c] != 0.0) return set_err(ctx, FKG_ERR_ARG, "beta must be finite and > 0");
+        hb[c] = beta[c];
+        src += d.n;
+    }
+    FKG_CUDA(ctx, cudaMemsetAsync(ctx->status.p, 0, sizeof(int), ctx->st));
+    if ((rc = upload_layout(ctx, ctx->solve, L))) return rc;
+    FKG_CUDA(ctx, cudaMemcpyAsync(ctx->solve.diag.p, hin, sizeof(double) * V, cudaMemcpyHostToDevice, ctx->st));
+    FKG_CUDA(ctx, cudaMemcpyAsync(ctx->solve.beta.p, hb, sizeof(double) * batch, cudaMemcpyHostToDevice, ctx->st));
+    if ((rc = enqueue_solve(ctx, ctx->solve, L, want_exp, nullptr, want_q))) return rc;
+    double* ow = hout;
+    double* oe = ow + V;
+    double* of = oe + V;
+    double* oz = of + V;
+    if (evals) FKG_CUDA(ctx, cudaMemcpyAsync(ow, ctx->solve.w.p, sizeof(double) * V, cudaMemcpyDeviceToHost, ctx->st));
+    if (exp_e) FKG_CUDA(ctx, cudaMemcpyAsync(oe, ctx->solve.exp_e.p, sizeof(double) * V, cudaMemcpyDeviceToHost, ctx->st));
+    if (fermi) FKG_CUDA(ctx, cudaMemcpyAsync(of, ctx->solve.fermi.p, sizeof(double) * V, cudaMemcpyDeviceToHost, ctx->st));
+    FKG_CUDA(ctx, cudaMemcpyAsync(oz, ctx->solve.logz.p, sizeof(double) * batch, cudaMemcpyDeviceToHost, ctx->st));
+    if ((rc = check_status(ctx))) return rc;
+    long long dst = 0;
+    for (int c = 0; c < batch; ++c) {
+        const ChainDesc& d = L.desc[c];
+        if (evals) std::memcpy(evals + dst, ow + d.v_off, sizeof(double) * d.n);
+        if (exp_e) std::memcpy(exp_e + dst, oe + d.v_off, sizeof(double) * d.n);
+        if (fermi) std::memcpy(fermi + dst, of + d.v_off, sizeof(double) * d.n);
+        if (logz) logz[c] = oz[c];
+        dst += d.n;
+    }
     return FKG_OK;
 }
 
@@ -521,49 +576,7 @@ int fkg_eigh_logz(fkg_ctx* ctx, int batch, const int32_t* lattice_id, const doub
     if (!ctx) return FKG_ERR_ARG;
     if (!diag || !beta) return set_err(ctx, FKG_ERR_ARG, "diag/beta is NULL");
     if (evecs) return eigh_vectors(ctx, batch, lattice_id, diag, beta, evals, exp_e, fermi, evecs, logz);
-    Layout& L = ctx->solve_layout;
-    int rc;
-    if ((rc = make_layout(ctx, batch, lattice_id, L))) return rc;
-    const bool want_exp = exp_e || fermi;
-    if ((rc = ensure_solve_ws(ctx, ctx->solve, L, want_exp))) return rc;
-    const size_t V = (size_t)L.v_total;
-    // pinned staging: diag (V) + beta (batch) in; evals, exp, fermi (3V) + logz (batch) out
-    if ((rc = ensure_pinned(ctx, sizeof(double) * (4 * V + 2 * batch)))) return rc;
-    double* hin = (double*)ctx->pin;
-    double* hb = hin + V;
-    double* hout = hb + batch;
-    long long src = 0;
-    for (int c = 0; c < batch; ++c) {
-        const ChainDesc& d = L.desc[c];
-        for (int i = 0; i < d.ld; ++i) hin[d.v_off + i] = i < d.n ? diag[src + i] : 0.0;
-        if (!(beta[c] > 0.0) || beta[c] - beta[c] != 0.0) return set_err(ctx, FKG_ERR_ARG, "beta must be finite and > 0");
-        hb[c] = beta[c];
-        src += d.n;
-    }
-    FKG_CUDA(ctx, cudaMemsetAsync(ctx->status.p, 0, sizeof(int), ctx->st));
-    if ((rc = upload_layout(ctx, ctx->solve, L))) return rc;
-    FKG_CUDA(ctx, cudaMemcpyAsync(ctx->solve.diag.p, hin, sizeof(double) * V, cudaMemcpyHostToDevice, ctx->st));
-    FKG_CUDA(ctx, cudaMemcpyAsync(ctx->solve.beta.p, hb, sizeof(double) * batch, cudaMemcpyHostToDevice, ctx->st));
-    if ((rc = enqueue_solve(ctx, ctx->solve, L, want_exp))) return rc;
-    double* ow = hout;
-    double* oe = ow + V;
-    double* of = oe + V;
-    double* oz = of + V;
-    if (evals) FKG_CUDA(ctx, cudaMemcpyAsync(ow, ctx->solve.w.p, sizeof(double) * V, cudaMemcpyDeviceToHost, ctx->st));
-    if (exp_e) FKG_CUDA(ctx, cudaMemcpyAsync(oe, ctx->solve.exp_e.p, sizeof(double) * V, cudaMemcpyDeviceToHost, ctx->st));
-    if (fermi) FKG_CUDA(ctx, cudaMemcpyAsync(of, ctx->solve.fermi.p, sizeof(double) * V, cudaMemcpyDeviceToHost, ctx->st));
-    FKG_CUDA(ctx, cudaMemcpyAsync(oz, ctx->solve.logz.p, sizeof(double) * batch, cudaMemcpyDeviceToHost, ctx->st));
-    if ((rc = check_status(ctx))) return rc;
-    long long dst = 0;
-    for (int c = 0; c < batch; ++c) {
-        const ChainDesc& d = L.desc[c];
-        if (evals) std::memcpy(evals + dst, ow + d.v_off, sizeof(double) * d.n);
-        if (exp_e) std::memcpy(exp_e + dst, oe + d.v_off, sizeof(double) * d.n);
-        if (fermi) std::memcpy(fermi + dst, of + d.v_off, sizeof(double) * d.n);
-        if (logz) logz[c] = oz[c];
-        dst += d.n;
-    }
-    return FKG_OK;
+    return eigh_values(ctx, batch, lattice_id, diag, beta, evals, exp_e, fermi, logz, false);
 }
 
 int fkg_chains_init(fkg_ctx* ctx, int batch, const int32_t* lattice_id, const int32_t* f, const double* U,
@@ -731,7 +744,7 @@ int fkg_free_energy_grad(fkg_ctx* ctx, int batch, const int32_t* lattice_id, con
     FKG_CUDA(ctx, cudaMemcpyAsync(ws.beta.p, hb, sizeof(double) * batch, cudaMemcpyHostToDevice, st));
     FKG_CUDA(ctx, cudaMemcpyAsync(ws.Ulist.p, hprm, sizeof(double) * 3 * batch, cudaMemcpyHostToDevice, st));
     FKG_CUDA(ctx, cudaMemcpyAsync(ws.fint.p, hf, sizeof(int32_t) * V, cudaMemcpyHostToDevice, st));
-    if ((rc = enqueue_solve(ctx, ws, L, false))) return rc;
+    if ((rc = enqueue_solve(ctx, ws, L, false, nullptr, true))) return rc;
     const bool f32 = ctx->precision == FKG_PREC_MIXED;
     if (!f32 && (rc = enqueue_vectors(ctx, ws, L))) return rc;
     const void* X = f32 ? ws.Z.p : ws.Z64.p;
@@ -808,7 +821,7 @@ int fkg_set_stiffness_ops(fkg_ctx* ctx, int lattice_id, int n, const int32_t* ro
 // each column's eigenvalue, the column order); used by the measures.
 static int solve_with_vectors(fkg_ctx* ctx, int batch, const int32_t* lattice_id, const double* diag,
                               const double* beta, const void** X, const double** eps, const int** perm) {
-    int rc = fkg_eigh_logz(ctx, batch, lattice_id, diag, beta, nullptr, nullptr, nullptr, nullptr, nullptr);
+    int rc = eigh_values(ctx, batch, lattice_id, diag, beta, nullptr, nullptr, nullptr, nullptr, true);
     if (rc) return rc;
     Workspace& ws = ctx->solve;
     const bool f32 = ctx->precision == FKG_PREC_MIXED;
@@ -1083,7 +1096,7 @@ static int fetch_vectors(fkg_ctx* ctx, Workspace& ws, const Layout& L, double* e
 int eigh_vectors(fkg_ctx* ctx, int batch, const int32_t* lattice_id, const double* diag, const double* beta,
                  double* evals, double* exp_e, double* fermi, double* evecs, double* logz) {
     // values, exp, fermi, logZ as fkg_eigh_logz without vectors, then the vectors
-    int rc = fkg_eigh_logz(ctx, batch, lattice_id, diag, beta, evals, exp_e, fermi, nullptr, logz);
+    int rc = eigh_values(ctx, batch, lattice_id, diag, beta, evals, exp_e, fermi, logz, true);
     if (rc) return rc;
     Layout& L = ctx->solve_layout;
     if (ctx->precision == FKG_PREC_F64 && (rc = enqueue_vectors(ctx, ctx->solve, L))) return rc;

@@ -224,10 +224,14 @@ int kpm_warps_per_cta(int bmax);
 // (may be null): kStatusBadArg when a CSR column lies outside [0, n)
 extern const int kSytrdF32Nb[3];
 extern const int kSytrdF64Nb[2];
-cudaError_t launch_sytrd_v3_f64(const ChainDesc* d_desc, int batch, int max_ld, const double* d_diag, double* d_A,
-                                double* d_d, double* d_e, double* d_tau, cudaStream_t st, int variant = 1,
-                                const int* d_order = nullptr, int* d_counter = nullptr, int num_sms = 0,
-                                int* d_status = nullptr);
+// FP64 path (sytrd_cluster.cu): h_desc host copy of the descriptors (read only
+// with a work list), d_A the reflectors (null: not stored, nor tau), d_spill
+// room for the tiles beyond shared memory (8 bytes per workspace entry, may be
+// d_A's own buffer when no reflectors are stored; null: must fit)
+cudaError_t launch_sytrd_f64(const ChainDesc* h_desc, const ChainDesc* d_desc, int batch, int max_ld,
+                             const double* d_diag, double* d_A, void* d_spill, double* d_d, double* d_e,
+                             double* d_tau, cudaStream_t st, int variant, const int* d_order, int* d_counter,
+                             int* d_status);
 cudaError_t launch_sytrd_v3_f32(const ChainDesc* d_desc, int batch, int max_ld, const double* d_diag, float* d_A,
                                 double* d_d, double* d_e, float* d_tau, cudaStream_t st, int variant = 1,
                                 const int* d_order = nullptr, int* d_counter = nullptr, int num_sms = 0,
@@ -298,12 +302,13 @@ cudaError_t launch_stiffness(const ChainDesc* d_desc, const StiffOps* d_ops, int
                              const void* d_X, const double* d_eps, const double* d_beta, void* d_JX, double2* d_ef,
                              double* d_scratch, double* d_out, int nw, const double* d_wgrid, double eta,
                              double* d_cond, cudaStream_t st);
-cudaError_t launch_logz(const ChainDesc* d_desc, int batch, int max_n, const double* d_w, const double* d_beta,
+// logZ of each chain; puts a chain's eigenvalues (d_w) in ascending order first where rounding left them out of it
+cudaError_t launch_logz(const ChainDesc* d_desc, int batch, int max_n, double* d_w, const double* d_beta,
                         double* d_logz, double* d_exp, double* d_fermi, int* d_status, cudaStream_t st);
 // logZ of each chain and, in the same launch, its Metropolis decision and
 // state update (the eigen-solve path's proposal step; equal to launch_logz
 // followed by launch_accept)
-cudaError_t launch_logz_accept(const ChainDesc* d_desc, int batch, const double* d_w, const double* d_beta,
+cudaError_t launch_logz_accept(const ChainDesc* d_desc, int batch, double* d_w, const double* d_beta,
                                double* d_logz, const int32_t* d_site, const double* d_u, const double* d_ebmf,
                                int32_t* d_f, double* d_logz_cur, double* d_w_cur, int32_t* d_accepted,
                                double* d_dlogz, int* d_status, cudaStream_t st, const int* d_step);

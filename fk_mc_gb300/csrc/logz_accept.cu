@@ -67,12 +67,28 @@ struct AcceptArgs {
 };
 
 __global__ void __launch_bounds__(kEigThreads)
-logz_kernel(const ChainDesc* __restrict__ descs, const double* __restrict__ ww, const double* __restrict__ beta,
+logz_kernel(const ChainDesc* __restrict__ descs, double* __restrict__ ww, const double* __restrict__ beta,
             double* __restrict__ logz, double* __restrict__ exp_out, double* __restrict__ fermi_out,
             int* __restrict__ status, AcceptArgs acc) {
     const ChainDesc D = descs[blockIdx.x];
     const int n = D.n;
     const double b = beta[blockIdx.x];
+    // Eigenvalues closer than their own rounding (exact degeneracies) come from
+    // independent searches and may be out of order by an ulp: put them in order.
+    bool down = false;
+    for (int i = threadIdx.x; i + 1 < n; i += blockDim.x) down = down || ww[D.v_off + i] > ww[D.v_off + i + 1];
+    if (__syncthreads_or(down)) {
+        if (threadIdx.x == 0) {
+            double* w = ww + D.v_off;
+            for (int i = 1; i < n; ++i) {
+                const double x = w[i];
+                int q = i - 1;
+                for (; q >= 0 && w[q] > x; --q) w[q + 1] = w[q];
+                w[q + 1] = x;
+            }
+        }
+        __syncthreads();
+    }
     double s = 0.0, c = 0.0;  // Neumaier running sum and compensation
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const double e = ww[D.v_off + i];
@@ -160,14 +176,14 @@ __global__ void accept_kernel(const ChainDesc* __restrict__ descs, const int32_t
 
 }  // namespace
 
-cudaError_t launch_logz(const ChainDesc* d_desc, int batch, int max_n, const double* d_w, const double* d_beta,
+cudaError_t launch_logz(const ChainDesc* d_desc, int batch, int max_n, double* d_w, const double* d_beta,
                         double* d_logz, double* d_exp, double* d_fermi, int* d_status, cudaStream_t st) {
     if (batch <= 0) return cudaSuccess;
     logz_kernel<<<batch, kEigThreads, 0, st>>>(d_desc, d_w, d_beta, d_logz, d_exp, d_fermi, d_status, AcceptArgs{});
     return cudaGetLastError();
 }
 
-cudaError_t launch_logz_accept(const ChainDesc* d_desc, int batch, const double* d_w, const double* d_beta,
+cudaError_t launch_logz_accept(const ChainDesc* d_desc, int batch, double* d_w, const double* d_beta,
                                double* d_logz, const int32_t* d_site, const double* d_u, const double* d_ebmf,
                                int32_t* d_f, double* d_logz_cur, double* d_w_cur, int32_t* d_accepted,
                                double* d_dlogz, int* d_status, cudaStream_t st, const int* d_step) {

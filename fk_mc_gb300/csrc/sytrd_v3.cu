@@ -531,16 +531,6 @@ cudaError_t launch_v3(const ChainDesc* d_desc, int batch, int max_ld, const doub
 
 // Panel widths compiled per precision; `variant` picks one (the autotuner's choice).
 const int kSytrdF32Nb[3] = {4, 8, 16};
-const int kSytrdF64Nb[2] = {2, 4};
-
-cudaError_t launch_sytrd_v3_f64(const ChainDesc* d_desc, int batch, int max_ld, const double* d_diag, double* d_A,
-                                double* d_d, double* d_e, double* d_tau, cudaStream_t st, int variant,
-                                const int* d_order, int* d_counter, int num_sms, int* d_status) {
-    if (variant == 0)
-        return launch_v3<double, 2>(d_desc, batch, max_ld, d_diag, d_A, d_d, d_e, d_tau, d_order, d_counter, num_sms, st, d_status);
-    return launch_v3<double, 4>(d_desc, batch, max_ld, d_diag, d_A, d_d, d_e, d_tau, d_order, d_counter, num_sms, st, d_status);
-}
-
 cudaError_t launch_sytrd_v3_f32(const ChainDesc* d_desc, int batch, int max_ld, const double* d_diag, float* d_A,
                                 double* d_d, double* d_e, float* d_tau, cudaStream_t st, int variant,
                                 const int* d_order, int* d_counter, int num_sms, int* d_status) {
