@@ -454,7 +454,8 @@ int fkg_set_tuning(fkg_ctx* ctx, int precision, int n_max, int variant) {
     // mixed: 0..2 the one-stage panel widths, 3 the two-stage reduction (band kBand)
     const int nvar = precision == FKG_PREC_MIXED ? kMixedVariants : 2;
     if (variant < -1 || variant >= nvar) return set_err(ctx, FKG_ERR_ARG, "variant out of range");
-    (precision == FKG_PREC_MIXED ? ctx->tune_f32 : ctx->tune_f64)[std::min(16, (n_max + 63) / 64)] = variant;
+    int* tune = precision == FKG_PREC_MIXED ? ctx->tune_f32 : ctx->tune_f64;
+    tune[std::min(16, (n_max + 63) / 64)] = variant;
     ctx->drop_graph();
     return FKG_OK;
 }
