@@ -10,7 +10,9 @@ batch of random configurations with CUDA events around the launches
 JSON. A variant's time is the sum of all stages of the solve (reduction,
 tridiagonal eigenproblem, back-transformation, refinement): the two-stage
 reduction moves work into the back-transformation (the band stage's
-reflectors). For the mixed path it then times the two back-transformation
+reflectors). On the mixed path it adds a values-only solve and one with
+eigenvectors (the panel widths matter only for the latter; the values-only
+one-stage reduction has one width). It then times the mixed path's two back-transformation
 kernels (mma.sync with the block of Z in shared memory, tcgen05 with
 tensor-memory accumulators; fkg_set_tuning_back) per size class under the
 chosen reduction. `Solver(..., tuning=path)` (default: the table shipped next
@@ -36,8 +38,8 @@ def tune(batch=None, reps=3, seed=1):
     table = {"device": None, "entries": []}
     import torch
     table["device"] = torch.cuda.get_device_name(0)
-    if batch is None:  # two chains per SM: the occupancy the kernels are used at
-        batch = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    if batch is None:  # one chain per SM: between the few chains and the many that one choice has to serve
+        batch = torch.cuda.get_device_properties(0).multi_processor_count
     rng = np.random.default_rng(seed)
     for prec, widths in VARIANTS.items():
         s = Solver(max_n=1024, max_batch=batch, precision=prec, tuning=None)
@@ -47,13 +49,17 @@ def tune(batch=None, reps=3, seed=1):
             f = rng.integers(0, 2, (batch, n))
             diag = (-1.0 + 2.0 * f).ravel()
             ids = np.zeros(batch, np.int32)
+            def solve():  # values only, and (mixed: another one-stage kernel) with eigenvectors
+                s.eigh_logz(ids, diag, 4.0)
+                if prec == "mixed":
+                    s.free_energy_grad(ids, f.ravel(), 2.0, 1.0, 1.0, 4.0)
             times = []
             for v in range(len(widths)):
                 s.set_tuning(prec, n, v)
-                s.eigh_logz(ids, diag, 4.0)  # warm
+                solve()  # warm
                 s.profile(True)
                 for _ in range(reps):
-                    s.eigh_logz(ids, diag, 4.0)
+                    solve()
                 times.append(sum(s.stage_time(st)[0] for st in STAGES) / reps)
                 s.profile(False)
             best = int(np.argmin(times))

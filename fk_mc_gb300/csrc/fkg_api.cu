@@ -248,10 +248,19 @@ int enqueue_solve(fkg_ctx* ctx, Workspace& ws, const Layout& L, bool want_exp, c
                                        (double*)ws.e.p, (float*)ws.Q2.p, L.a_total, ctx->st));
             ctx->launches += 2;
         } else {
-            FKG_CUDA(ctx, launch_sytrd_v3_f32(dd, L.batch, L.max_ld, (const double*)ws.diag.p, (float*)ws.A32.p,
-                                              (double*)ws.d.p, (double*)ws.e.p, (float*)ws.aux32.p, ctx->st,
-                                              pick_variant(ctx, L, true), (const int*)ws.order.p, (int*)ws.counter.p,
-                                              ctx->num_sms, (int*)ctx->status.p));
+            // FP32 eigenvectors that leave the library keep sytrd_v3's rounding; the order
+            // where that ends is where the two-stage reduction used to be the tuned choice
+            if (want_q && L.max_n <= 960)
+                FKG_CUDA(ctx, launch_sytrd_v3_f32(dd, L.batch, L.max_ld, (const double*)ws.diag.p, (float*)ws.A32.p,
+                                                  (double*)ws.d.p, (double*)ws.e.p, (float*)ws.aux32.p, ctx->st,
+                                                  pick_variant(ctx, L, true), (const int*)ws.order.p,
+                                                  (int*)ws.counter.p, ctx->num_sms, (int*)ctx->status.p));
+            else
+                FKG_CUDA(ctx, launch_sytrd_f32(L.desc.data(), dd, L.batch, L.max_ld, (const double*)ws.diag.p,
+                                               (float*)ws.A32.p, ws.VT.p /* written by larft later */,
+                                               (double*)ws.d.p, (double*)ws.e.p, (float*)ws.aux32.p, ctx->st,
+                                               (const int*)ws.order.p, (int*)ws.counter.p, ctx->num_sms,
+                                               (int*)ctx->status.p));
             ctx->launches++;
         }
         stage_end(ctx, FKG_STAGE_REDUCE);

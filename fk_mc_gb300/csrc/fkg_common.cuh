@@ -219,23 +219,26 @@ cudaError_t launch_kpm(const KpmDesc* d_kdesc, int batch, int max_n, int max_ld,
                        int kmax, const double* d_diag, const double* d_beta, KpmAB* d_ab, int* d_steps,
                        double* d_part, double* d_mu, double* d_logz, int* d_status, cudaStream_t st);
 int kpm_warps_per_cta(int bmax);
-// variant: index into kSytrdF64Nb / kSytrdF32Nb (panel width); d_order (may be
-// null): chain indices longest first for the persistent schedule; d_status
-// (may be null): kStatusBadArg when a CSR column lies outside [0, n)
-extern const int kSytrdF32Nb[3];
-extern const int kSytrdF64Nb[2];
-// FP64 path (sytrd_cluster.cu): h_desc host copy of the descriptors (read only
-// with a work list), d_A the reflectors (null: not stored, nor tau), d_spill
-// room for the tiles beyond shared memory (8 bytes per workspace entry, may be
-// d_A's own buffer when no reflectors are stored; null: must fit)
+// One-stage reductions (sytrd_cluster.cuh). h_desc: host copy of the descriptors
+// (read only with a work list); d_A: the reflectors (FP64: null, neither they
+// nor tau are stored); d_spill: room for the tiles beyond shared memory (8 or 4
+// bytes per workspace entry; FP64 without reflectors: d_A's buffer serves; null:
+// all must fit); d_order (may be null): chain indices longest first for the
+// persistent schedule; d_status (may be null): kStatusBadArg when a CSR column
+// lies outside [0, n), kStatusNaN for entries that are not finite (FP64).
+// variant (FP64): panel width, index into {2, 4}
 cudaError_t launch_sytrd_f64(const ChainDesc* h_desc, const ChainDesc* d_desc, int batch, int max_ld,
                              const double* d_diag, double* d_A, void* d_spill, double* d_d, double* d_e,
                              double* d_tau, cudaStream_t st, int variant, const int* d_order, int* d_counter,
                              int* d_status);
+cudaError_t launch_sytrd_f32(const ChainDesc* h_desc, const ChainDesc* d_desc, int batch, int max_ld,
+                             const double* d_diag, float* d_A, void* d_spill, double* d_d, double* d_e, float* d_tau,
+                             cudaStream_t st, const int* d_order, int* d_counter, int num_sms, int* d_status);
+// FP32 reduction of solves whose FP32 eigenvectors leave the library
+// (sytrd_v3.cu); variant: panel width, index into {4, 8, 16}
 cudaError_t launch_sytrd_v3_f32(const ChainDesc* d_desc, int batch, int max_ld, const double* d_diag, float* d_A,
-                                double* d_d, double* d_e, float* d_tau, cudaStream_t st, int variant = 1,
-                                const int* d_order = nullptr, int* d_counter = nullptr, int num_sms = 0,
-                                int* d_status = nullptr);
+                                double* d_d, double* d_e, float* d_tau, cudaStream_t st, int variant,
+                                const int* d_order, int* d_counter, int num_sms, int* d_status);
 // shift: reflector k has its unit at row k + shift (1: one-stage reduction,
 // kBand: the two-stage reduction's first stage)
 cudaError_t launch_larft_vt(const ChainDesc* d_desc, int batch, int max_n, const float* d_A32, const float* d_tau32,

@@ -14,7 +14,7 @@ namespace fkg {
 constexpr int kMaxLattices = 64;
 constexpr int kMaxN = 1024;  // largest matrix order the kernels are built for
 // reduction variants of the mixed path (fkg_set_tuning): 0..2 the one-stage
-// kernel's panel widths (kSytrdF32Nb), kTwoStageVariant the two-stage reduction
+// kernel's panel widths {4, 8, 16}, kTwoStageVariant the two-stage reduction
 constexpr int kTwoStageVariant = 3;
 constexpr int kMixedVariants = 4;
 
@@ -192,7 +192,8 @@ struct StepIO {
     double* dl;
     const int* step;
 };
-// want_q: the reduction's reflectors are kept for enqueue_vectors (FP64 path)
+// want_q: eigenvectors are used after the solve (FP64 path: the reduction's
+// reflectors are kept for enqueue_vectors)
 int enqueue_solve(fkg_ctx* ctx, Workspace& ws, const Layout& L, bool want_exp, const StepIO* io = nullptr,
                   bool want_q = false);
 int enqueue_steps(fkg_ctx* ctx, int nsteps, const int32_t* d_site, const double* d_u, int32_t* d_acc,

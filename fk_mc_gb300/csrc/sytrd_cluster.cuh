@@ -1,4 +1,4 @@
-// sytrd_cluster.cu — Householder tridiagonalisation by a thread-block cluster
+// sytrd_cluster.cuh — Householder tridiagonalisation by a thread-block cluster
 // per chain, the trailing matrix held in the cluster's shared memory.
 //
 // Replaces the first half of Eigen::SelfAdjointEigenSolver at
@@ -6,13 +6,13 @@
 // and the dense copy (:212) are fused into the tile fill.
 //
 // Algorithm (panel of NB reflectors, deferred symmetric rank-2k update), as in
-// sytrd_v3.cu: per column the pending updates of the panel on that column, the
+// LAPACK's dlatrd: per column the pending updates of the panel on that column, the
 // reflector, p = A22 v with the stale trailing matrix corrected by the panel's
 // V and W; after the panel A22 -= V W^T + W V^T.
 //
 // Arithmetic (template parameter P):
-//   F32  FP32 throughout (the mixed path's reduction);
-//   Fix  FP64-grade arithmetic on the integer pipe. GB300 issues one FP64
+//   F32  FP32 throughout (the mixed path's reduction; sytrd_f32.cu);
+//   Fix  FP64-grade arithmetic on the integer pipe (sytrd_f64.cu). GB300 issues one FP64
 //        multiply-add per warp every 64-76 cycles of a sub-partition, one
 //        32 x 32 + 64 bit integer multiply-add every 2 (measured). All matrix
 //        and vector entries are 64-bit fixed-point numbers with the quantum
@@ -43,6 +43,7 @@
 // Two cluster barriers per column: after the column and its norm have been
 // written to every CTA's shared memory, and after the partial products have;
 // the rest of a column is computed redundantly by every CTA.
+#pragma once
 #include <cooperative_groups.h>
 
 #include <cfloat>
@@ -72,7 +73,7 @@ __device__ __forceinline__ float add_mod(float a, float b) { return a + b; }
 __device__ __forceinline__ ll add_mod(ll a, ll b) { return (ll)((ull)a + (ull)b); }
 
 // Sums of VN values over the lanes that differ in the lane bits `HI`, `HI`/2,
-// ... (VN of them halve): see sytrd_v3.cu. After it the lane holds the total of
+// ... (VN of them halve), by recursive halving. After it the lane holds the total of
 // value `idx` over those lanes.
 template <int VN, int HI, typename T>
 __device__ __forceinline__ T reduce_scatter(T (&x)[VN], int lane, int& idx) {
@@ -92,8 +93,11 @@ __device__ __forceinline__ T reduce_scatter(T (&x)[VN], int lane, int& idx) {
     return x[0];
 }
 
+// W = 8: two CTAs share an SM (128 registers a thread); W = 16: one
+template <int W>
 struct F32 {
-    static constexpr int kWarps = 16;
+    static constexpr int kWarps = W, kOcc = W == 8 ? 2 : 1;
+    static constexpr double kBase = 6.0, kPerRow = 0.0035, kPerTile = 0.115;  // column time, see launch_cluster
     using V = float;  // matrix / vector entry
     using S = float;  // sum
     using G = float;  // reflectors in global memory
@@ -123,7 +127,8 @@ struct F32 {
 };
 
 struct Fix {
-    static constexpr int kWarps = 8;  // 236 registers a thread
+    static constexpr int kWarps = 8, kOcc = 1;  // 236 registers a thread
+    static constexpr double kBase = 8.8, kPerRow = 0.0034, kPerTile = 0.68;
     using V = int2;  // (hi, lo)
     using S = ll;
     using G = double;
@@ -264,7 +269,7 @@ __host__ __device__ inline Smem smem_layout(int max_ld, int C, int max_slots) {
 __host__ __device__ inline int slots_of(int nt, int C) { return (nt * (nt + 1) / 2 + C - 1) / C; }
 
 template <class P, int NB>
-__global__ void __launch_bounds__(P::kWarps * 32, 1)
+__global__ void __launch_bounds__(P::kWarps * 32, P::kOcc)
 sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restrict__ diag,
                      typename P::G* __restrict__ Aout, void* __restrict__ spill, double* __restrict__ dout,
                      double* __restrict__ eout, typename P::G* __restrict__ tauout, const int* __restrict__ order,
@@ -840,14 +845,16 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
 }  // namespace
 
 // Cluster size and grid of a launch. The time of one chain's column was fitted
-// on the GPU (N = 64 .. 1024, one chain per cluster): about 11 k cycles that do
-// not depend on C plus 0.68 k cycles per tile of the CTA's mean share (a third of
-// the chain's tiles), +0.8 k for the cluster barriers; `fit` clusters run at
-// once (152, 76, 36, 15 for C = 1, 2, 4, 8). Measured ms (FP64 path) behind the
-// choice: 256 chains of N = 576: 30.4 (C = 1), 34.2 (2), 46.6 (4); 16 chains:
-// 13.8, 8.6, 5.9, 9.5 (C = 8: two rounds); one chain of N = 343: 4.2, 3.0, 2.4, 2.1.
+// on the GPU (N = 64 .. 1024, one chain per cluster) as P::kBase + P::kPerRow n
+// + P::kPerTile times a CTA's mean share of tiles (a third of the chain's over
+// C), +0.8 for the cluster barriers, in k cycles; `fit` clusters run at once
+// (152, 76, 36, 15 for C = 1, 2, 4, 8). Measured ms behind the choice (C = 1, 2,
+// 4, 8), FP64 path: 256 chains of N = 576 30.4, 34.2, 46.6, 85; 16 chains 13.8, 8.6,
+// 5.9, 9.5 (two rounds); one chain of N = 343 4.2, 3.0, 2.4, 2.1. FP32: 256 chains
+// of N = 576 7.9, 12.8, 21.3, 47.6; 16 chains of N = 1024 15.3, 10.1, 7.4, 12.7.
+template <class P>
 static double cluster_cost(int n, int nt, int C) {
-    return n * (11.0 + (C > 1 ? 0.8 : 0.0) + 0.68 * (nt * (nt + 1) / 2) / (3.0 * C));
+    return n * (P::kBase + P::kPerRow * n + (C > 1 ? 0.8 : 0.0) + P::kPerTile * (nt * (nt + 1) / 2) / (3.0 * C));
 }
 
 template <class P, int NB>
@@ -857,7 +864,7 @@ static cudaError_t launch_cluster(const ChainDesc* h_desc, const ChainDesc* d_de
                                   cudaStream_t st) {
     if (batch <= 0) return cudaSuccess;
     auto* kern = sytrd_cluster_kernel<P, NB>;
-    const size_t tile_bytes = sizeof(typename P::V) * kTileElems, limit = 226 * 1024;
+    const size_t tile_bytes = sizeof(typename P::V) * kTileElems, limit = 226 * 1024 / P::kOcc;
     cudaError_t err;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at;
@@ -888,7 +895,7 @@ static cudaError_t launch_cluster(const ChainDesc* h_desc, const ChainDesc* d_de
             if (fit < 1) continue;
             double sum = 0.0, mx = 0.0, mn = 1e300;
             for (int c = 0; c < batch; ++c) {
-                const double t = cluster_cost(h_desc[c].n, h_desc[c].ld / kTile, C);
+                const double t = cluster_cost<P>(h_desc[c].n, h_desc[c].ld / kTile, C);
                 sum += t;
                 mx = max(mx, t);
                 mn = min(mn, t);
@@ -912,20 +919,6 @@ static cudaError_t launch_cluster(const ChainDesc* h_desc, const ChainDesc* d_de
     cfg.dynamicSmemBytes = best_smem;
     return cudaLaunchKernelEx(&cfg, kern, d_desc, d_diag, d_A, d_spill, d_d, d_e, d_tau, d_order, batch, d_counter,
                               d_status, max_ld, best_slots, best_cap);
-}
-
-// Panel widths compiled for the FP64 path; `variant` picks one (fkg_set_tuning).
-const int kSytrdF64Nb[2] = {2, 4};
-
-cudaError_t launch_sytrd_f64(const ChainDesc* h_desc, const ChainDesc* d_desc, int batch, int max_ld,
-                             const double* d_diag, double* d_A, void* d_spill, double* d_d, double* d_e,
-                             double* d_tau, cudaStream_t st, int variant, const int* d_order, int* d_counter,
-                             int* d_status) {
-    if (variant == 0)
-        return launch_cluster<Fix, 2>(h_desc, d_desc, batch, max_ld, d_diag, d_A, d_spill, d_d, d_e, d_tau, d_order,
-                                      d_counter, d_status, st);
-    return launch_cluster<Fix, 4>(h_desc, d_desc, batch, max_ld, d_diag, d_A, d_spill, d_d, d_e, d_tau, d_order,
-                                  d_counter, d_status, st);
 }
 
 }  // namespace fkg

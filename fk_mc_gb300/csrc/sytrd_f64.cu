@@ -1,0 +1,17 @@
+// sytrd_f64.cu — the FP64 path's Householder reduction (sytrd_cluster.cuh with
+// two-limb fixed-point arithmetic).
+#include "sytrd_cluster.cuh"
+
+namespace fkg {
+
+// variant: panel width 2 or 4 (fkg_set_tuning)
+cudaError_t launch_sytrd_f64(const ChainDesc* h_desc, const ChainDesc* d_desc, int batch, int max_ld,
+                             const double* d_diag, double* d_A, void* d_spill, double* d_d, double* d_e,
+                             double* d_tau, cudaStream_t st, int variant, const int* d_order, int* d_counter,
+                             int* d_status) {
+    auto* launch = variant == 0 ? launch_cluster<Fix, 2> : launch_cluster<Fix, 4>;
+    return launch(h_desc, d_desc, batch, max_ld, d_diag, d_A, d_spill, d_d, d_e, d_tau, d_order, d_counter, d_status,
+                  st);
+}
+
+}  // namespace fkg

@@ -1,5 +1,9 @@
-// sytrd_v3.cu — blocked Householder tridiagonalisation, one CTA per chain,
-// FP64 (plain path) or FP32 (mixed path).
+// sytrd_v3.cu — blocked Householder tridiagonalisation in FP32, one CTA per
+// chain: the mixed path's reduction where FP32 eigenvectors leave the library
+// (gradients, measures, eigenvectors). Values-only solves use the faster
+// sytrd_cluster.cuh; its other order of summation would change every output
+// that is computed from the FP32 vectors by the path's own error (1e-7 of
+// dF/dU), so those solves keep this kernel's rounding up to n = 960.
 //
 // Replaces the first half of Eigen::SelfAdjointEigenSolver at
 // src/configuration.cpp:213; the Hamiltonian build (src/configuration.cpp:79-91)
@@ -15,9 +19,9 @@
 // The trailing matrix is read once per column (the matrix-vector product) and
 // read+written once per panel (the rank-2k update).
 //
-// The design aims at a low instruction count per matrix element, which is
-// what bounds this kernel on GB300 (the FP32 version is issue bound, the FP64
-// version bound by the narrow FP64 pipe):
+// The design aims at a low instruction count per matrix element; the kernel is
+// bound by the latency of its L2 loads (N = 576, 256 chains: 9.9 ms; the cluster
+// kernel 7.9):
 //   * the padding rows/columns and the upper part of every 32x32 diagonal
 //     tile are zeroed once, so interior tiles load with no per-element masks
 //     (entries outside the active window multiply a zero of v);
@@ -26,7 +30,7 @@
 //     rank-2k update; W never touches global memory;
 //   * matrix-vector tiles issue their 32 column loads before using them;
 //     column sums go through a padded per-warp shared-memory transpose;
-//   * 8 warps per CTA; FP32 at N <= 576 fits two CTAs per SM.
+//   * 8 warps per CTA; at N <= 576 two CTAs fit on an SM.
 #include "fkg_common.cuh"
 
 namespace fkg {
@@ -65,13 +69,7 @@ __device__ __forceinline__ T warp_reduce_scatter(T (&x)[V], int lane, int& idx) 
     return t;
 }
 
-// c - a b - d e. FP64: as two fused multiply-adds (written out, `c -= a * b +
-// d * e` compiles to a multiply, a fused multiply-add and an add: three issues
-// of the narrow FP64 pipe for two multiply-adds of work). FP32 keeps the
-// written-out form and its rounding (that kernel is not bound by its pipe).
-__device__ __forceinline__ double fnma2(double a, double b, double d, double e, double c) {
-    return fma(-d, e, fma(-a, b, c));
-}
+// c - a b - d e
 __device__ __forceinline__ float fnma2(float a, float b, float d, float e, float c) { return c - (a * b + d * e); }
 
 // four contiguous values from 16-byte-aligned shared memory (vector loads)
@@ -79,17 +77,13 @@ __device__ __forceinline__ void load4(const float* p, float (&o)[4]) {
     const float4 x = *reinterpret_cast<const float4*>(p);
     o[0] = x.x; o[1] = x.y; o[2] = x.z; o[3] = x.w;
 }
-__device__ __forceinline__ void load4(const double* p, double (&o)[4]) {
-    const double2 x = *reinterpret_cast<const double2*>(p), y = *reinterpret_cast<const double2*>(p + 2);
-    o[0] = x.x; o[1] = x.y; o[2] = y.x; o[3] = y.y;
-}
 
 // One CTA reduces one chain at a time. Without a work list (order == null)
 // CTA b takes chain b; with one, the CTAs are persistent: each takes the next
 // entry of `order` (chains sorted by decreasing n, longest first) from the
 // counter until the list is used up, which balances uneven batches.
 template <typename T, int NB>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
+__global__ void __launch_bounds__(kThreads, 2)
 sytrd_v3_kernel(const ChainDesc* __restrict__ descs, const double* __restrict__ diag, T* __restrict__ Aws,
                 double* __restrict__ dout, double* __restrict__ eout, T* __restrict__ tauout,
                 const int* __restrict__ order, int norder, int* __restrict__ counter, int* __restrict__ status) {
@@ -234,7 +228,7 @@ sytrd_v3_kernel(const ChainDesc* __restrict__ descs, const double* __restrict__ 
             // ---- (3a) p = A22 v, stale trailing matrix, lower tiles, no masks ----
             // Warp w takes tiles w, w + kWarps, ... of the lower tiles (I, J),
             // I0 <= J <= I, in row order; the column sums go through a
-            // shared-memory transpose of the tile. FP32 keeps two tiles in
+            // shared-memory transpose of the tile. Two tiles are kept in
             // registers: the next tile's 32 loads are in flight while the
             // current one is used.
             {
@@ -284,33 +278,24 @@ sytrd_v3_kernel(const ChainDesc* __restrict__ descs, const double* __restrict__ 
                 };
                 int I = I0, J = I0;
                 advance(I, J, warp);
-                if constexpr (sizeof(T) == 4) {
-                    T a0[kTile], a1[kTile];
-                    int t = warp;
-                    if (t < total) load(I, J, a0);
-                    while (t < total) {
-                        int I1 = I, J1 = J;
-                        advance(I1, J1, kWarps);
-                        const bool h1 = t + kWarps < total;
-                        if (h1) load(I1, J1, a1);
-                        use(I, J, a0);
-                        if (!h1) break;
-                        int I2 = I1, J2 = J1;
-                        advance(I2, J2, kWarps);
-                        const bool h2 = t + 2 * kWarps < total;
-                        if (h2) load(I2, J2, a0);
-                        use(I1, J1, a1);
-                        t += 2 * kWarps;
-                        I = I2;
-                        J = J2;
-                    }
-                } else {
-                    T a[kTile];
-                    for (int t = warp; t < total; t += kWarps) {
-                        load(I, J, a);
-                        use(I, J, a);
-                        advance(I, J, kWarps);
-                    }
+                T a0[kTile], a1[kTile];
+                int t = warp;
+                if (t < total) load(I, J, a0);
+                while (t < total) {
+                    int I1 = I, J1 = J;
+                    advance(I1, J1, kWarps);
+                    const bool h1 = t + kWarps < total;
+                    if (h1) load(I1, J1, a1);
+                    use(I, J, a0);
+                    if (!h1) break;
+                    int I2 = I1, J2 = J1;
+                    advance(I2, J2, kWarps);
+                    const bool h2 = t + 2 * kWarps < total;
+                    if (h2) load(I2, J2, a0);
+                    use(I1, J1, a1);
+                    t += 2 * kWarps;
+                    I = I2;
+                    J = J2;
                 }
             }
             // ---- (3b) c1 = W^T v, c2 = V^T v over the panel's earlier reflectors ----
@@ -360,13 +345,11 @@ sytrd_v3_kernel(const ChainDesc* __restrict__ descs, const double* __restrict__ 
             __syncthreads();
         }
         // ---- (5) A(tb:, tb:) -= V W^T + W V^T (lower tiles) ----
-        // FP32: on the tensor cores. Per 32 x 32 tile, u = [V_I W_I] [W_J V_J]^T
+        // On the tensor cores. Per 32 x 32 tile, u = [V_I W_I] [W_J V_J]^T
         // (K = 2 NB) as mma.sync m16n8k8 3xTF32 from zero, then A -= u with
         // round-to-nearest FP32 (the tensor core's own accumulation truncates);
         // the tile (in accumulator layout) is loaded before u is formed.
-        // FP64 (bound by its FP64 pipe, not by latency): four columns at a
-        // time with fewer live registers.
-        if constexpr (sizeof(T) == 4) {
+        {
             const int tb = k0 + nbk;
             const int I0 = tb >> 5;
             const int ntr = nt - I0;
@@ -443,48 +426,6 @@ sytrd_v3_kernel(const ChainDesc* __restrict__ descs, const double* __restrict__ 
                         }
                 advance(I, J, kWarps);
             }
-        } else {
-        const int tb = k0 + nbk;
-        const int I0 = tb >> 5;
-        int cnt = 0;
-        for (int I = I0; I < nt; ++I) {
-            for (int J = I0; J <= I; ++J, ++cnt) {
-                if ((cnt & (kWarps - 1)) != warp) continue;
-                const int i = I * kTile + lane;
-                T VI[NB], WI[NB];
-#pragma unroll
-                for (int l = 0; l < NB; ++l) { VI[l] = VpT[(size_t)i * NB + l]; WI[l] = WpT[(size_t)i * NB + l]; }
-                T* At = A + (size_t)(J * kTile) * ld + i;
-                const bool edge = (J == I0) || (I == J);
-                if (!edge) {
-                    for (int c = 0; c < kTile; c += 4) {
-                        T acc[4];
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) acc[q] = At[(size_t)(c + q) * ld];
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            const T* vj = VpT + (size_t)(J * kTile + c + q) * NB;
-                            const T* wj = WpT + (size_t)(J * kTile + c + q) * NB;
-#pragma unroll
-                            for (int l = 0; l < NB; ++l) acc[q] = fnma2(VI[l], wj[l], WI[l], vj[l], acc[q]);
-                        }
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) At[(size_t)(c + q) * ld] = acc[q];
-                    }
-                } else {
-                    for (int c = 0; c < kTile; ++c) {
-                        const int jc = J * kTile + c;
-                        if (jc < tb || i < jc) continue;
-                        const T* vj = VpT + (size_t)jc * NB;
-                        const T* wj = WpT + (size_t)jc * NB;
-                        T a = At[(size_t)c * ld];
-#pragma unroll
-                        for (int l = 0; l < NB; ++l) a = fnma2(VI[l], wj[l], WI[l], vj[l], a);
-                        At[(size_t)c * ld] = a;
-                    }
-                }
-            }
-        }
         }
         __syncthreads();
         for (int t = tid; t < 2 * NB * ld; t += kThreads) VpT[t] = T(0);
@@ -529,8 +470,7 @@ cudaError_t launch_v3(const ChainDesc* d_desc, int batch, int max_ld, const doub
 
 }  // namespace
 
-// Panel widths compiled per precision; `variant` picks one (the autotuner's choice).
-const int kSytrdF32Nb[3] = {4, 8, 16};
+// variant: panel width 4, 8 or 16 (the autotuner's choice)
 cudaError_t launch_sytrd_v3_f32(const ChainDesc* d_desc, int batch, int max_ld, const double* d_diag, float* d_A,
                                 double* d_d, double* d_e, float* d_tau, cudaStream_t st, int variant,
                                 const int* d_order, int* d_counter, int num_sms, int* d_status) {

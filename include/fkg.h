@@ -226,7 +226,10 @@ int fkg_set_stream(fkg_ctx* ctx, void* cuda_stream);
 
 /* Panel width of the Householder reduction for matrices of order up to n_max
  * (size buckets of 64): variant indexes the compiled widths {4, 8, 16}
- * (FKG_PREC_MIXED) or {2, 4} (FKG_PREC_F64); -1 restores the default.
+ * (FKG_PREC_MIXED) or {2, 4} (FKG_PREC_F64); FKG_PREC_MIXED 3 selects the
+ * two-stage reduction; -1 restores the default. On the mixed path the widths
+ * apply to solves whose eigenvectors are used (gradients, measures,
+ * eigenvectors, n <= 960); values-only solves have one one-stage reduction.
  * Written by the autotuner (fk_mc_gb300/autotune.py) from measured times. */
 int fkg_set_tuning(fkg_ctx* ctx, int precision, int n_max, int variant);
 
