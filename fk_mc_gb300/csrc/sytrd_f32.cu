@@ -1,6 +1,6 @@
 // sytrd_f32.cu — the mixed path's one-stage Householder reduction
 // (sytrd_cluster.cuh in FP32).
-#include "sytrd_cluster.cuh"
+#include "sytrd_small.cuh"
 
 namespace fkg {
 
@@ -14,6 +14,14 @@ namespace fkg {
 cudaError_t launch_sytrd_f32(const ChainDesc* h_desc, const ChainDesc* d_desc, int batch, int max_ld,
                              const double* d_diag, float* d_A, void* d_spill, double* d_d, double* d_e, float* d_tau,
                              cudaStream_t st, const int* d_order, int* d_counter, int num_sms, int* d_status) {
+    if (batch <= 0) return cudaSuccess;
+    if (max_ld <= 128) {
+        auto* small = max_ld <= 32   ? launch_small<F32<8>, 32, 8>
+                      : max_ld <= 64 ? launch_small<F32<8>, 64, 8>
+                      : max_ld <= 96 ? launch_small<F32<8>, 96, 8>
+                                     : launch_small<F32<8>, 128, 4>;
+        return small(d_desc, batch, d_diag, d_A, d_d, d_e, d_tau, d_order, d_status, st);
+    }
     const bool narrow = max_ld <= 256 || (max_ld <= 480 && batch > num_sms);
     auto* launch = narrow                          ? launch_cluster<F32<8>, 4>
                    : max_ld > 768 && batch > 96 ? launch_cluster<F32<16>, 8>
