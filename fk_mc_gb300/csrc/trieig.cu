@@ -13,18 +13,15 @@
 //      within a few eps32 ||T|| of T, so widening by 16 eps32 ||T|| gives a
 //      bracket of the FP64 eigenvalue;
 //   2. where the widened brackets of the neighbouring indices j-1 and j+1
-//      stay clear of it, that bracket holds exactly lambda_j; elsewhere (block
-//      edges, eigenvalues closer than the FP32 resolution) two FP64 Sturm
-//      counts verify it (a failed check falls back to the Gershgorin
-//      interval);
-//   3. if the bracket holds exactly one eigenvalue, a safeguarded Newton
-//      iteration on the characteristic polynomial p_n(x) = det(T - x I)
-//      (three-term recurrence for p and p', rescaled by powers of two, no
-//      divisions) converges quadratically to full FP64 accuracy; the sign of
-//      p_n at the bracket ends is (-1)^count, so every iterate keeps a valid
-//      bracket and falls back to bisection when Newton leaves it;
-//   4. otherwise (eigenvalues closer than the FP32 resolution) FP64 bisection
-//      on Sturm counts finishes the job.
+//      stay clear of it, or FP32 counts further out say so (block edges), that
+//      bracket holds exactly lambda_j;
+//   3. if the bracket holds exactly one eigenvalue, Newton on the characteristic
+//      polynomial p_n(x) = det(T - x I) (three-term recurrence, rescaled by
+//      powers of two, no divisions) in double-float and one last step with
+//      p_n in FP64;
+//   4. otherwise (eigenvalues closer than the FP32 resolution) a warp per
+//      eigenvalue: FP64 Sturm counts at the ends, then safeguarded Newton in
+//      FP64 or 32-point multisection.
 // One thread per eigenvalue index; d and e of the chain sit in shared memory.
 #include <cfloat>
 
@@ -111,12 +108,14 @@ struct TriShared {
     float* d32;
     float* e232;  // e_i^2 in FP32, floored at FLT_MIN (i < n - 1)
     float2* de;   // (d_i, e_{i-1}^2) for the FP32 counts
+    float* e2l;   // e_i^2 - e232[i]
+    float* dl;    // d_i - d32[i] (null: T is FP32-exact)
 };
 
-// shared-memory layout of one chain's tridiagonal; `extra` floats follow
-__device__ __forceinline__ TriShared tri_shared(double* sm, int ld) {
+// shared-memory layout of one chain's tridiagonal (pairs: d as FP32 pairs too)
+__device__ __forceinline__ TriShared tri_shared(double* sm, int ld, bool pairs) {
     float* f = (float*)(sm + 2 * ld);
-    return TriShared{sm, sm + ld, f, f + ld, (float2*)(f + 2 * ld)};
+    return TriShared{sm, sm + ld, f, f + ld, (float2*)(f + 2 * ld), f + 4 * ld, pairs ? f + 5 * ld : nullptr};
 }
 
 // Loads d, e^2 (FP64 and FP32 copies) of chain D into shared memory and
@@ -134,6 +133,8 @@ __device__ void load_tridiag(const ChainDesc& D, const double* __restrict__ dd, 
         S.e2[i] = er * er;
         S.d32[i] = (float)di;
         S.e232[i] = i + 1 < n ? fmaxf((float)(er * er), FLT_MIN) : 0.f;
+        S.e2l[i] = (float)(er * er - (double)S.e232[i]);
+        if (S.dl) S.dl[i] = (float)(di - (double)S.d32[i]);
         S.de[i] = make_float2((float)di, i > 0 ? fmaxf((float)(el * el), FLT_MIN) : 0.f);
         gl = fmin(gl, di - el - er);
         gu = fmax(gu, di + el + er);
@@ -223,72 +224,76 @@ __device__ void block_brackets(const TriShared& S, int n, int j, bool active, co
 // within a few eps32 ||T|| of T.
 __device__ __forceinline__ double bracket_slack(const TriBounds& B) { return 16.0 * FLT_EPSILON * B.tnorm; }
 
-// Steps 2-4: FP64 eigenvalue j from its FP32 bracket. isolated: the widened
-// brackets of j-1 and j+1 stay clear of this one, so it holds exactly
-// lambda_j and the FP64 Sturm counts that would verify it are skipped.
-__device__ double refine64(TriShared S, int n, int j, const TriBounds& B, float lo, float hi, bool isolated,
-                           int* status) {
+// Safeguarded Newton on p_n in FP64 inside [a, b], which holds exactly one
+// eigenvalue, number ca; sign(p_n(x)) = (-1)^count(x). Converged when the step
+// falls below 4 eps max(|x|, ||T||), i.e. at the accuracy of the Sturm
+// recurrence itself; from the FP32 bracket that takes 3-5 evaluations, the cap
+// of 12 only stops rounding-level oscillation.
+// A Newton step s_k after s_{k-1} leaves an error of about |s_k|^2 |p''/2p'| ~
+// |s_k|^3 / s_{k-1}^2 (quadratic convergence); when that is 4x below the
+// tolerance the step is the last one, which from an FP32 bracket usually saves
+// the third evaluation.
+__device__ double newton64(const TriShared& S, int n, int ca, double tnorm, double a, double b) {
     const double eps = DBL_EPSILON;
-    const double tnorm = B.tnorm, pivmin = B.pivmin;
+    const double sa = (ca & 1) ? -1.0 : 1.0;  // sign of p_n at a
+    double x = 0.5 * (a + b), dxold = b - a, dx = dxold, prev = 0.0;
+    for (int it = 0; it < 12; ++it) {
+        double p, dp;
+        charpoly(S.d, S.e2, n, x, p, dp);
+        if (p == 0.0) { a = b = x; break; }
+        if ((p > 0.0) == (sa > 0.0)) a = x; else b = x;
+        const double step = p / dp;
+        const double tol = 4.0 * eps * fmax(fabs(x), tnorm);
+        // converged: the Newton correction is at the rounding level of p_n,
+        // or the one after it would be
+        if (dp != 0.0 && (fabs(step) <= tol || (prev > 0.0 && fabs(step) * step * step <= 0.25 * tol * prev * prev)) &&
+            x - step >= a && x - step <= b) {
+            x -= step;
+            break;
+        }
+        double xn = x - step;
+        if (!(dp != 0.0) || !(xn > a && xn < b) || fabs(2.0 * (xn - x)) > fabs(dxold)) {
+            dxold = dx;
+            xn = 0.5 * (a + b);
+            dx = xn - x;
+            prev = 0.0;
+        } else {
+            dxold = dx;
+            dx = xn - x;
+            prev = fabs(step);
+        }
+        x = xn;
+        if (fabs(dx) <= 4.0 * eps * fmax(fabs(x), tnorm) || b - a <= 4.0 * eps * fmax(fabs(x), tnorm)) break;
+    }
+    return fmin(fmax(x, a), b);
+}
+
+// FP64 eigenvalue j of a bracket that nothing confirms yet, by a whole warp (an
+// FP64 instruction costs the narrow pipe the same for one lane as for 32):
+// Sturm counts at both ends; if it holds exactly lambda_j Newton, else
+// multisection with 32 points a round (five bisections each).
+__device__ double refine64_warp(const TriShared& S, int n, int j, const TriBounds& B, float lo, float hi,
+                                int* status) {
+    const double eps = DBL_EPSILON;
+    const int lane = threadIdx.x & 31;
     const double delta = bracket_slack(B);
     double a = fmax((double)lo - delta, B.gl), b = fmin((double)hi + delta, B.gu);
-    int ca = j, cb = j + 1;
-    if (!isolated) {
-        ca = count64(S.d, S.e2, n, a, pivmin);
-        cb = count64(S.d, S.e2, n, b, pivmin);
-        if (!(ca <= j && j < cb)) {
-            a = B.gl; b = B.gu; ca = 0; cb = n;
-        }
+    const int c = count64(S.d, S.e2, n, lane == 0 ? a : b, B.pivmin);
+    int ca = __shfl_sync(0xffffffffu, c, 0), cb = __shfl_sync(0xffffffffu, c, 1);
+    if (!(ca <= j && j < cb)) {
+        a = B.gl; b = B.gu; ca = 0; cb = n;
     }
-    if (ca == j && cb == j + 1) {
-        // ---- 3. safeguarded Newton on p_n; sign(p_n(x)) = (-1)^count(x) ----
-        // Converged when the step falls below 4 eps max(|x|, ||T||), i.e. at
-        // the accuracy of the Sturm recurrence itself; from the FP32 bracket
-        // that takes 3-5 evaluations, the cap of 12 only stops rounding-level
-        // oscillation.
-        // A Newton step s_k after s_{k-1} leaves an error of about
-        // |s_k|^2 |p''/2p'| ~ |s_k|^3 / s_{k-1}^2 (quadratic convergence);
-        // when that is 4x below the tolerance the step is the last one, which
-        // from an FP32 bracket usually saves the third evaluation.
-        const double sa = (ca & 1) ? -1.0 : 1.0;  // sign of p_n at a
-        double x = 0.5 * (a + b), dxold = b - a, dx = dxold, prev = 0.0;
-        for (int it = 0; it < 12; ++it) {
-            double p, dp;
-            charpoly(S.d, S.e2, n, x, p, dp);
-            if (p == 0.0) { a = b = x; break; }
-            if ((p > 0.0) == (sa > 0.0)) a = x; else b = x;
-            const double step = p / dp;
-            const double tol = 4.0 * eps * fmax(fabs(x), tnorm);
-            // converged: the Newton correction is at the rounding level of p_n,
-            // or the one after it would be
-            if (dp != 0.0 && (fabs(step) <= tol || (prev > 0.0 && fabs(step) * step * step <= 0.25 * tol * prev * prev)) &&
-                x - step >= a && x - step <= b) {
-                x -= step;
-                break;
-            }
-            double xn = x - step;
-            if (!(dp != 0.0) || !(xn > a && xn < b) || fabs(2.0 * (xn - x)) > fabs(dxold)) {
-                dxold = dx;
-                xn = 0.5 * (a + b);
-                dx = xn - x;
-                prev = 0.0;
-            } else {
-                dxold = dx;
-                dx = xn - x;
-                prev = fabs(step);
-            }
-            x = xn;
-            if (fabs(dx) <= 4.0 * eps * fmax(fabs(x), tnorm) || b - a <= 4.0 * eps * fmax(fabs(x), tnorm)) break;
-        }
-        return fmin(fmax(x, a), b);
-    }
-    // ---- 4. FP64 bisection inside the bracket ----
-    for (int it = 0; it < 128; ++it) {
-        const double mid = 0.5 * (a + b);
-        if (b - a <= 2.0 * eps * fmax(fabs(a), fabs(b)) + 0.5 * eps * tnorm || mid <= a || mid >= b) break;
-        if (count64(S.d, S.e2, n, mid, pivmin) > j) b = mid;
-        else a = mid;
-        if (it == 127) atomicOr(status, kStatusNoConverge);
+    if (ca == j && cb == j + 1) return newton64(S, n, ca, B.tnorm, a, b);
+    for (int it = 0; it < 64; ++it) {
+        const double w = b - a, mid = 0.5 * (a + b);
+        if (w <= 2.0 * eps * fmax(fabs(a), fabs(b)) + 0.5 * eps * B.tnorm || mid <= a || mid >= b) break;
+        const double x = fmin(fmax(a + w * ((lane + 1) * (1.0 / 33.0)), a), b);
+        const unsigned up = __ballot_sync(0xffffffffu, count64(S.d, S.e2, n, x, B.pivmin) > j);
+        const int f = up ? __ffs(up) - 1 : 32;  // first point above lambda_j
+        const double nb = __shfl_sync(0xffffffffu, x, min(f, 31)), na = __shfl_sync(0xffffffffu, x, max(f - 1, 0));
+        if (f < 32) b = nb;
+        if (f > 0) a = na;
+        if (it == 63) { if (lane == 0) atomicOr(status, kStatusNoConverge); }
     }
     return 0.5 * (a + b);
 }
@@ -309,32 +314,6 @@ __device__ __forceinline__ void neighbour_gaps(float* br, int n, int j, bool act
     else if (t > 0) gl_gap = ((double)lo - delta) - ((double)br[2 * (t - 1) + 1] + delta);
     if (j == n - 1) gr_gap = DBL_MAX;
     else if (t + 1 < (int)blockDim.x) gr_gap = ((double)br[2 * (t + 1)] - delta) - ((double)hi + delta);
-}
-
-// One thread per eigenvalue index, FP64 result for every index.
-__global__ void __launch_bounds__(kEigThreads)
-trieig_values_kernel(const ChainDesc* __restrict__ descs, const double* __restrict__ dd,
-                     const double* __restrict__ ee, double* __restrict__ ww, int* __restrict__ status) {
-    extern __shared__ double sm[];
-    const ChainDesc D = descs[blockIdx.x];
-    const int n = D.n;
-    if ((int)(blockIdx.y * blockDim.x) >= n) return;
-    const TriShared S = tri_shared(sm, D.ld);
-    double gl, gu, emax2;
-    load_tridiag(D, dd, ee, S, gl, gu, emax2);
-    const TriBounds B = tri_bounds(n, gl, gu, emax2);
-    __shared__ float br[2 * kEigThreads];
-    const int j = blockIdx.y * blockDim.x + threadIdx.x;
-    const bool active = j < n;
-    float lo = 0.f, hi = 0.f;
-    block_brackets(S, n, j, active, B, lo, hi);
-    double lgap, rgap;
-    const double delta = bracket_slack(B);
-    neighbour_gaps(br, n, j, active, lo, hi, delta, lgap, rgap);
-    if (!active) return;
-    const double lam = refine64(S, n, j, B, lo, hi, lgap > 2.0 * delta && rgap > 2.0 * delta, status);
-    ww[D.v_off + j] = lam;
-    if (!isfinite(lam)) atomicOr(status, kStatusNaN);
 }
 
 // ---- mixed path: the eigenvalues of T only serve as shifts of the FP32
@@ -484,6 +463,158 @@ __device__ bool shift_df(const float* d, const float* e2h, const float* e2l, int
     return false;
 }
 
+// The listed eigenvalues in FP64, one warp each.
+__device__ void list64(const ChainDesc& D, const TriShared& S, int n, const TriBounds& B, int count, const int* list,
+                       const float* lbr, double* __restrict__ ww, int* __restrict__ status) {
+    for (int q = threadIdx.x >> 5; q < count; q += blockDim.x >> 5) {
+        const double lam = refine64_warp(S, n, list[q], B, lbr[2 * q], lbr[2 * q + 1], status);
+        if ((threadIdx.x & 31) == 0) {
+            ww[D.v_off + list[q]] = lam;
+            if (!isfinite(lam)) atomicOr(status, kStatusNaN);
+        }
+    }
+}
+
+// p_n and p_n' as charpoly_df with d and e^2 as pairs; `e`: the common scale is 2^e.
+__device__ void charpoly_df2(const TriShared& S, int n, float xh, float xl, float& p, float& dp, int& e) {
+    float p0h = 1.f, p0l = 0.f, dp0 = 0.f;
+    DfRow t = df_shift(S.d32[0], xh, xl - S.dl[0]);
+    float p1h, p1l;
+    fast_two_sum(t.th, t.tl, p1h, p1l);
+    float dp1 = -1.f;
+    e = 0;
+    for (int i = 1; i < n; ++i) {
+        t = df_shift(S.d32[i], xh, xl - S.dl[i]);
+        const float bh = S.e232[i - 1];
+        float p2h, p2l;
+        df_step(t, bh, S.e2l[i - 1], p1h, p1l, p0h, p0l, p2h, p2l);
+        const float dp2 = fmaf(t.th, dp1, -fmaf(bh, dp0, p1h));
+        p0h = p1h; p0l = p1l; dp0 = dp1;
+        p1h = p2h; p1l = p2l; dp1 = dp2;
+        if ((i & 3) == 0) {
+            const float m = fmaxf(fabsf(p1h), fabsf(dp1));
+            const float sc = df_scale(m);
+            e += m > 0x1p50f ? 50 : (m < 0x1p-50f && m > 0.f ? -50 : 0);
+            p0h *= sc; p0l *= sc; dp0 *= sc; p1h *= sc; p1l *= sc; dp1 *= sc;
+        }
+    }
+    p = p1h + p1l;
+    dp = dp1;
+}
+
+// Newton in double-float from the middle of an isolated FP32 bracket, until the
+// next step would be below 1e-13 ||T||; returns the point, and p_n' there (to FP32
+// accuracy, up to 2^edp). False when the iteration cannot be trusted.
+__device__ bool newton_df(const TriShared& S, int n, const TriBounds& B, float lo, float hi, double& x, double& dpx,
+                          int& edp) {
+    const double delta = bracket_slack(B), tol = 1e-13 * B.tnorm;
+    const double x0 = 0.5 * ((double)lo + (double)hi);
+    float xh = (float)x0, xl = (float)(x0 - (double)xh), prev = 0.f;
+    for (int it = 0; it < kDfIters; ++it) {
+        float p, dp;
+        charpoly_df2(S, n, xh, xl, p, dp, edp);
+        const float step = p / dp;
+        if (!(dp != 0.f) || !isfinite(step)) return false;
+        float sh, se, nh, nl;
+        two_sum(xh, -step, sh, se);
+        fast_two_sum(sh, se + xl, nh, nl);
+        x = (double)nh + (double)nl;
+        if (!(x >= (double)lo - delta && x <= (double)hi + delta)) return false;
+        const float as = fabsf(step);
+        if ((double)as <= tol || (prev > 0.f && (double)as * as * as <= 0.25 * tol * (double)prev * prev)) {
+            dpx = (double)dp;
+            return true;
+        }
+        prev = as;
+        xh = nh;
+        xl = nl;
+    }
+    return false;
+}
+
+// Does the widened bracket [lo - delta, hi + delta] hold exactly lambda_j? Decided
+// with FP32 counts a further 1.5 delta out: an FP32 count at y is the exact count at a
+// point within delta of y, so count32(lo - 2.5 delta) >= j puts lambda_{j-1}
+// below lo - delta, and likewise above.
+__device__ __forceinline__ bool isolated32(const TriShared& S, int n, int j, const TriBounds& B, float lo, float hi) {
+    const float d25 = (float)(2.5 * bracket_slack(B));
+    return (j == 0 || count32(S.de, n, lo - d25) >= j) && (j == n - 1 || count32(S.de, n, hi + d25) <= j + 1);
+}
+
+// p_n(x) in FP64 up to 2^e (no derivative: three FP64 operations a row).
+__device__ __forceinline__ double charpoly_value(const double* __restrict__ d, const double* __restrict__ e2, int n,
+                                                 double x, int& e) {
+    double p0 = 1.0, p1 = d[0] - x;
+    e = 0;
+    for (int i = 1; i < n; ++i) {
+        const double p2 = fma(d[i] - x, p1, -e2[i - 1] * p0);
+        p0 = p1;
+        p1 = p2;
+        if ((i & 7) == 0) {
+            // magnitude from the exponent fields: the FP64 pipe is the bound here
+            const int m = max(__double2hiint(p0) & 0x7ff00000, __double2hiint(p1) & 0x7ff00000);
+            if (m > (1023 + 400) << 20) { p0 *= 0x1p-400; p1 *= 0x1p-400; e += 400; }
+            else if (m < (1023 - 400) << 20 && m > 0) { p0 *= 0x1p400; p1 *= 0x1p400; e -= 400; }
+        }
+    }
+    return p1;
+}
+
+// One thread per eigenvalue index, FP64 result for every index: Newton in
+// double-float (FP32 pairs, T rounded to them: ~1e-14 ||T||) and one last step
+// with p_n in FP64 and the pairs' derivative, three FP64 operations a row
+// instead of five in two or three evaluations. What is not isolated, or does
+// not behave, goes to a list that the block's warps work off in FP64.
+__global__ void __launch_bounds__(kEigThreads)
+trieig_values_kernel(const ChainDesc* __restrict__ descs, const double* __restrict__ dd,
+                     const double* __restrict__ ee, double* __restrict__ ww, int* __restrict__ status) {
+    extern __shared__ double sm[];
+    const ChainDesc D = descs[blockIdx.x];
+    const int n = D.n;
+    if ((int)(blockIdx.y * blockDim.x) >= n) return;
+    const TriShared S = tri_shared(sm, D.ld, true);
+    double gl, gu, emax2;
+    load_tridiag(D, dd, ee, S, gl, gu, emax2);
+    const TriBounds B = tri_bounds(n, gl, gu, emax2);
+    __shared__ float br[2 * kEigThreads];
+    __shared__ int list[kEigThreads];
+    __shared__ float lbr[2 * kEigThreads];
+    __shared__ int cnt;
+    if (threadIdx.x == 0) cnt = 0;
+    const int j = blockIdx.y * blockDim.x + threadIdx.x;
+    const bool active = j < n;
+    float lo = 0.f, hi = 0.f;
+    block_brackets(S, n, j, active, B, lo, hi);
+    double lgap, rgap;
+    const double delta = bracket_slack(B);
+    neighbour_gaps(br, n, j, active, lo, hi, delta, lgap, rgap);
+    if (active) {
+        bool done = false;
+        if ((lgap > 2.0 * delta && rgap > 2.0 * delta) || isolated32(S, n, j, B, lo, hi)) {
+            double x, dp;
+            int edp;
+            if (newton_df(S, n, B, lo, hi, x, dp, edp)) {
+                int ep;
+                const double p = charpoly_value(S.d, S.e2, n, x, ep);
+                const double step = scalbn(p / dp, max(-2000, min(2000, ep - edp)));
+                const double lam = x - step;
+                if (fabs(step) <= 1e-11 * B.tnorm && lam >= (double)lo - delta && lam <= (double)hi + delta) {
+                    ww[D.v_off + j] = lam;
+                    done = true;
+                }
+            }
+        }
+        if (!done) {
+            const int q = atomicAdd(&cnt, 1);
+            list[q] = j;
+            lbr[2 * q] = lo;
+            lbr[2 * q + 1] = hi;
+        }
+    }
+    __syncthreads();
+    list64(D, S, n, B, cnt, list, lbr, ww, status);
+}
+
 __global__ void __launch_bounds__(kEigThreads)
 trieig_shift_kernel(const ChainDesc* __restrict__ descs, const double* __restrict__ dd,
                     const double* __restrict__ ee, double* __restrict__ ww, double* __restrict__ ctol,
@@ -492,15 +623,13 @@ trieig_shift_kernel(const ChainDesc* __restrict__ descs, const double* __restric
     const ChainDesc D = descs[blockIdx.x];
     const int n = D.n;
     if ((int)(blockIdx.y * blockDim.x) >= n) return;
-    const TriShared S = tri_shared(sm, D.ld);
-    float* e2l = (float*)(S.de + D.ld);
+    const TriShared S = tri_shared(sm, D.ld, false);
     __shared__ float br[2 * kEigThreads];
     __shared__ int list[kEigThreads];
     __shared__ float lbr[2 * kEigThreads];
     __shared__ int cnt;
     double gl, gu, emax2;
     load_tridiag(D, dd, ee, S, gl, gu, emax2);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) e2l[i] = (float)(S.e2[i] - (double)S.e232[i]);
     if (threadIdx.x == 0) cnt = 0;
     __syncthreads();
     const TriBounds B = tri_bounds(n, gl, gu, emax2);
@@ -516,7 +645,7 @@ trieig_shift_kernel(const ChainDesc* __restrict__ descs, const double* __restric
     neighbour_gaps(br, n, j, active, lo, hi, delta, lgap, rgap);
     if (active) {
         double x;
-        if (shift_df(S.d32, S.e232, e2l, n, j, B, lo, hi, lgap > 2.0 * delta && rgap > 2.0 * delta, x)) {
+        if (shift_df(S.d32, S.e232, S.e2l, n, j, B, lo, hi, lgap > 2.0 * delta && rgap > 2.0 * delta, x)) {
             ww[D.v_off + j] = x;
         } else {
             const int q = atomicAdd(&cnt, 1);
@@ -526,27 +655,20 @@ trieig_shift_kernel(const ChainDesc* __restrict__ descs, const double* __restric
         }
     }
     __syncthreads();
-    // the rest in FP64, packed onto the first threads
-    const int k = cnt;
-    if ((int)threadIdx.x < k) {
-        const int jj = list[threadIdx.x];
-        const double lam = refine64(S, n, jj, B, lbr[2 * threadIdx.x], lbr[2 * threadIdx.x + 1], false, status);
-        ww[D.v_off + jj] = lam;
-        if (!isfinite(lam)) atomicOr(status, kStatusNaN);
-    }
+    list64(D, S, n, B, cnt, list, lbr, ww, status);  // the rest in FP64
 }
 
 }  // namespace
 
 size_t trieig_smem_bytes(int max_ld) {
-    return (size_t)max_ld * (2 * sizeof(double) + 2 * sizeof(float) + sizeof(float2));
+    return (size_t)max_ld * (2 * sizeof(double) + 4 * sizeof(float) + sizeof(float2));
 }
 
 
 cudaError_t launch_trieig_shifts(const ChainDesc* d_desc, int batch, int max_n, int max_ld, const double* d_d,
                                  const double* d_e, double* d_w, double* d_ctol, int* d_status, cudaStream_t st) {
     if (batch <= 0) return cudaSuccess;
-    const size_t smem = trieig_smem_bytes(max_ld) + sizeof(float) * (size_t)max_ld;
+    const size_t smem = trieig_smem_bytes(max_ld);
     cudaError_t err = cudaFuncSetAttribute(trieig_shift_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
     dim3 grid(batch, (max_n + kEigThreads - 1) / kEigThreads);
