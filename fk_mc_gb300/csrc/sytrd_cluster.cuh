@@ -14,23 +14,24 @@
 //   F32  FP32 throughout (the mixed path's reduction; sytrd_f32.cu);
 //   Fix  FP64-grade arithmetic on the integer pipe (sytrd_f64.cu). GB300 issues one FP64
 //        multiply-add per warp every 64-76 cycles of a sub-partition, one
-//        32 x 32 + 64 bit integer multiply-add every 2 (measured). All matrix
-//        and vector entries are 64-bit fixed-point numbers with the quantum
-//        2^-56 S (matrix; S = the power of two above the largest row sum of
-//        |H|, so ||H||_2 <= S), 2^-56 (v), 2^-55 S (w), held as two limbs
-//        x = hi 2^26 + lo (hi 32 bits, |lo| <= 2^25). A product is three integer
-//        multiply-adds: hi hi into one 64-bit sum, hi lo + lo hi into another;
-//        lo lo (< 2^-62, signed) is dropped. Every sum is exact: the results
-//        are bounded by the norms (|A v| <= sqrt(2) S, |w| <= 2 S, the cross
-//        sums by sqrt(n) times the limbs' ranges, < 2^62 for n <= 1024), and
+//        32 x 32 -> 64 bit integer multiplication every 4 (measured). All matrix
+//        and vector entries are 64-bit fixed-point numbers relative to S, the
+//        power of two above the largest row sum of |H| (so ||H||_2 <= S), held as
+//        two limbs x = hi 2^LO + lo (hi 32 bits, |lo| <= 2^(LO - 1); formats at
+//        struct Fix). A product is three integer multiplications: hi hi into one
+//        64-bit sum, hi lo + lo hi into another; lo lo is dropped. Every sum is
+//        exact: the results are bounded by the norms (|A v| <= sqrt(2) S, |w| <=
+//        2 S, the cross sums by sqrt(n) times the limbs' ranges), and
 //        intermediate wrap-around modulo 2^64 is harmless. Orthogonal
 //        transformations keep ||A||_2, so no entry outgrows its format. The
-//        rounding is one quantum per entry and panel (2^-57 S) where FP64
-//        rounds every product; the norm of a column is an exact integer sum,
+//        rounding is half a quantum per entry and panel where FP64 rounds every
+//        product; the norm of a column is an exact integer sum,
 //        its inverse square root a Newton iteration from the FP32 estimate on
 //        64-bit integers (the FP64 square root and divisions cost ~1100 cycles
-//        each per column). Errors against 64-bit LAPACK: below the FP64
-//        kernel's at every size measured.
+//        each per column). Errors against 34-digit arithmetic
+//        (rms over the spectrum / ||H||; FP64 kernel before, this): N = 64 6.0e-17,
+//        2.6e-17; N = 64 with U = 20 2.1e-16, 4.2e-17; N = 125 5.1e-17, 2.5e-17; N = 144
+//        5.3e-17, 3.8e-17; N = 196 7.0e-17, 3.8e-17.
 //
 // Work split. A chain's lower 32 x 32 tiles are numbered by decreasing tile
 // column, so the tiles alive at a step are always a prefix; tile t belongs to
@@ -126,9 +127,14 @@ struct F32 {
     static __device__ __forceinline__ V upd(V a, const Acc& u) { return a - u.s; }  // a - u (rank-2k update)
 };
 
+// LO: bits of the low limb (quanta 2^-(30 + LO) S of a matrix, 2^-(30 + LO) of
+// v, 2^-(29 + LO) S of w). 27 keeps the cross sums below 2^63 for n <= 1024, 28 for
+// n <= 256.
+template <int LO>
 struct Fix {
-    static constexpr int kWarps = 8, kOcc = 1;  // 236 registers a thread
+    static constexpr int kWarps = 8, kOcc = 1;  // ~240 registers a thread
     static constexpr double kBase = 8.8, kPerRow = 0.0034, kPerTile = 0.68;
+    static constexpr int kLo = LO;
     using V = int2;  // (hi, lo)
     using S = ll;
     using G = double;
@@ -153,13 +159,21 @@ struct Fix {
         a.x += mw(p1.x, q1.y) + mw(p1.y, q1.x);
     }
     // the sum in units of the hi hi products
-    static __device__ __forceinline__ S sum(const Acc& a) { return (ll)(a.h + (ull)(((ll)a.x + (1 << 25)) >> 26)); }
+    static __device__ __forceinline__ S sum(const Acc& a) {
+        return (ll)(a.h + (ull)(((ll)a.x + (1 << (LO - 1))) >> LO));
+    }
     static __device__ __forceinline__ V vzero() { return make_int2(0, 0); }
     static __device__ __forceinline__ V split(ll a) {
-        const int lo = ((int)a << 6) >> 6;
-        return make_int2((int)((a - lo) >> 26), lo);
+        const int lo = ((int)a << (32 - LO)) >> (32 - LO);
+        return make_int2((int)((a - lo) >> LO), lo);
     }
-    static __device__ __forceinline__ ll join(V v) { return (ll)v.x * (1 << 26) + v.y; }
+    static __device__ __forceinline__ ll join(V v) { return (ll)v.x * (1 << LO) + v.y; }
+    // x rounded from units 2^-XB to units 2^-YB
+    template <int XB, int YB>
+    static __device__ __forceinline__ ll round_to(ll x) {
+        if constexpr (XB > YB) return (x + (1ll << (XB - YB - 1))) >> (XB - YB);
+        else return x << (YB - XB);
+    }
     static __device__ __forceinline__ void ld4(const void* t, int q, int lane, V (&a)[4]) {
         const int4 h = ((const int4*)t)[q * 32 + lane], l = ((const int4*)t)[256 + q * 32 + lane];
         a[0] = make_int2(h.x, l.x); a[1] = make_int2(h.y, l.y);
@@ -180,9 +194,25 @@ struct Fix {
         ((int*)t)[off] = v.x;
         ((int*)t)[kTileElems + off] = v.y;
     }
-    // a - u: u = sum of v w products in units 2^-59 S, a in 2^-56 S
-    static __device__ __forceinline__ ll upd_ll(V a, const Acc& u) { return join(a) - ((sum(u) + 4) >> 3); }
+    // a - u: u = sum of v w products in units 2^-59 S, a in 2^-(30 + LO) S. Rounded
+    // with all the bits of the cross products: from the sum in whole units every
+    // second to eighth rounding would be a tie, whose common direction adds up over
+    // the entries and columns.
+    static __device__ __forceinline__ ll upd_ll(V a, const Acc& u) {
+        constexpr int sh = 29 - LO;
+        const ll low = ((ll)((unsigned)u.h & ((1u << sh) - 1)) << LO) + (ll)u.x + (1 << 28);
+        return join(a) - (((ll)u.h >> sh) + (low >> 29));
+    }
     static __device__ __forceinline__ V upd(V a, const Acc& u) { return split(upd_ll(a, u)); }
+    // w = tau p - K v: p in units 2^-60 S, K v (kv) in 2^-59 S
+    static __device__ __forceinline__ V w_entry(ll p, ll tau, const Acc& kv) {
+        const ll k60 = (ll)(2 * kv.h) + (((ll)kv.x + (1 << (LO - 2))) >> (LO - 1));
+        return split(round_to<60, 29 + LO>(__mul64hi(p * 4, tau) - k60));
+    }
+    // K = tau^2 p.v / 2 (p.v in units 2^-60 S)
+    static __device__ __forceinline__ V k_value(ll pv, ll tau) {
+        return split(round_to<60, 29 + LO>(__mul64hi(__mul64hi(pv * 2, tau) * 4, tau)));
+    }
 };
 
 // offset of entry (r, c) of a tile (lane-owned 16-byte units)
@@ -394,8 +424,8 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                 continue;
             }
             eS = m > 0x1p-900 ? ilogb(m * (1.0 + 0x1p-30)) + 1 : -899;
-            quant = scalbn(1.0, eS - 56);
-            inv = scalbn(1.0, 56 - eS);
+            quant = scalbn(1.0, eS - 30 - P::kLo);
+            inv = scalbn(1.0, 30 + P::kLo - eS);
         }
         __syncthreads();
         auto owner_slot = [&](int I, int J) {  // slot of tile (I, J) if this CTA owns it, else -1
@@ -490,8 +520,8 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                         hh = warp_sum_ll(hh);
                         hl = warp_sum_ll(hl);
                         l2 = warp_sum_ll(l2);
-                        const unsigned __int128 s2 = ((unsigned __int128)(ull)hh << 52) +
-                                                     (unsigned __int128)((__int128)hl << 27) + (ull)l2;
+                        const unsigned __int128 s2 = ((unsigned __int128)(ull)hh << (2 * P::kLo)) +
+                                                     (unsigned __int128)((__int128)hl << (P::kLo + 1)) + (ull)l2;
                         R = fix_reflector(s2, alpha);
                         if (lane == 0) s_refl = R;
                     }
@@ -512,9 +542,9 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                 if (rank == 0 && tid == 0) {  // raw; converted after the last column (FP64 pipe)
                     if constexpr (kFix) {
                         // 2^-62 S: sqrt(s2) has at most 62 bits there
-                        const int sh = R.z / 2 - 8;
+                        const int sh = R.z / 2 - 34 + P::kLo;
                         const ll xn = (ll)(sh >= 0 ? R.xn >> sh : R.xn << -sh);
-                        *(ll*)(eout + D.v_off + k) = flat ? alpha * 64 : (alpha >= 0 ? -xn : xn);
+                        *(ll*)(eout + D.v_off + k) = flat ? alpha << (32 - P::kLo) : (alpha >= 0 ? -xn : xn);
                         if (Aout) *(ull*)(tauout + D.v_off + k) = R.tau;
                     } else {
                         *(float*)(eout + D.v_off + k) = beta;
@@ -526,12 +556,12 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                     V vi = P::vzero();
                     if (!flat && i >= s && i < n) {
                         if constexpr (kFix) {
-                            ll v56 = 1ll << 56;
+                            ll v = 1ll << (30 + P::kLo);
                             if (i > s) {
-                                v56 = (__mul64hi(xb[i] << (R.z / 2 - 1), (ll)R.r) + 16) >> 5;
-                                if (alpha < 0) v56 = -v56;
+                                v = P::template round_to<61, 30 + P::kLo>(__mul64hi(xb[i] << (R.z / 2 - 1), (ll)R.r));
+                                if (alpha < 0) v = -v;
                             }
-                            vi = P::split(v56);
+                            vi = P::split(v);
                         } else {
                             vi = i == s ? 1.f : xb[i] * scale;
                         }
@@ -541,7 +571,7 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                     if (flat) Wp[i * NB + j] = P::vzero();
                     if (i > s && i < n && ((i >> 5) & cm) == rank) {
                         if constexpr (kFix) {
-                            if (Aout) A[(size_t)k * ld + i] = (double)P::join(vi) * 0x1p-56;
+                            if (Aout) A[(size_t)k * ld + i] = (double)P::join(vi) * (1.0 / (1ll << (30 + P::kLo)));
                         } else {
                             A[(size_t)k * ld + i] = vi;
                         }
@@ -663,7 +693,7 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                             const int a0 = pwi[3 * i], a1 = pwi[3 * i + 1], a2 = pwi[3 * i + 2];
                             pwi[3 * i] = pwi[3 * i + 1] = pwi[3 * i + 2] = 0;
                             p = (ll)((ull)(ll)a0 + ((ull)(ll)a1 << 21) + ((ull)(ll)a2 << 42));  // units 2^-60 S
-                            P::mac(pv, P::split((p + 8) >> 4), vv[i]);
+                            P::mac(pv, P::split(P::template round_to<60, 30 + P::kLo>(p)), vv[i]);
                         } else {
                             p = 0.f;
 #pragma unroll
@@ -710,9 +740,8 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                         for (int l = 0; l < NB; ++l) {
                             const S a = __shfl_sync(0xffffffffu, c, l), b = __shfl_sync(0xffffffffu, c, NB + l);
                             if constexpr (kFix) {
-                                // c1: 2^-59 S -> 2^-54 S, c2: 2^-60 -> 2^-55
-                                c1[l] = P::split((a + 16) >> 5);
-                                c2[l] = P::split((b + 16) >> 5);
+                                c1[l] = P::split(P::template round_to<59, 28 + P::kLo>(a));
+                                c2[l] = P::split(P::template round_to<60, 29 + P::kLo>(b));
                             } else {
                                 c1[l] = a;
                                 c2[l] = b;
@@ -727,9 +756,7 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                     float K = 0.f;
                     V Kv;
                     if constexpr (kFix) {
-                        const ll t1 = __mul64hi(pv, (ll)R.tau);        // 2^-58 S: tau p.v
-                        const ll kk = __mul64hi(t1, (ll)R.tau);        // 2^-57 S: tau^2 p.v / 2
-                        Kv = P::split((kk + 2) >> 2);                  // 2^-55 S
+                        Kv = P::k_value(pv, (ll)R.tau);
                     } else {
                         K = 0.5f * tau * (tau * pv);
                         Kv = K;
@@ -753,7 +780,7 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                                 Acc kv;
                                 P::zero(kv);
                                 P::mac(kv, Kv, vv[i]);  // 2^-59 S
-                                w = P::split((2 * __mul64hi(q, (ll)R.tau) - P::sum(kv) + 8) >> 4);
+                                w = P::w_entry(q, (ll)R.tau, kv);
                             } else {
                                 w = tau * (q - u.s) - K * vv[i];
                             }
@@ -817,7 +844,7 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                 if (slot < 0) continue;
                 const V a = P::get(tile(slot), elem_off(jj & 31, i & 31));
                 S* o = (S*)((e == 1 ? eout : dout) + D.v_off + i);
-                if constexpr (kFix) *o = P::join(a) * (e == 1 ? 64 : 1);
+                if constexpr (kFix) *o = P::join(a) << (e == 1 ? 32 - P::kLo : 0);
                 else *o = a;
             }
         }
@@ -829,7 +856,7 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                 double* e = eout + D.v_off + i;
                 if constexpr (kFix) {
                     *d = (double)__ldcg((ll*)d) * quant;
-                    if (i < n - 1) *e = (double)__ldcg((ll*)e) * (quant * 0x1p-6);
+                    if (i < n - 1) *e = (double)__ldcg((ll*)e) * (quant / (1ll << (32 - P::kLo)));
                     double* t = tauout + D.v_off + i;
                     if (Aout && i < n - 2) *t = (double)__ldcg((ull*)t) * 0x1p-62;
                 } else {

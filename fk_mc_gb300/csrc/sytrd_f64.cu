@@ -11,13 +11,13 @@ cudaError_t launch_sytrd_f64(const ChainDesc* h_desc, const ChainDesc* d_desc, i
                              int* d_status) {
     if (batch <= 0) return cudaSuccess;
     if (max_ld <= 128) {
-        auto* small = max_ld <= 32   ? launch_small<Fix, 32, 8>
-                      : max_ld <= 64 ? launch_small<Fix, 64, 8>
-                      : max_ld <= 96 ? launch_small<Fix, 96, 8>
-                                     : launch_small<Fix, 128, 4>;
+        auto* small = max_ld <= 32   ? launch_small<Fix<28>, 32, 8>
+                      : max_ld <= 64 ? launch_small<Fix<28>, 64, 8>
+                      : max_ld <= 96 ? launch_small<Fix<28>, 96, 8>
+                                     : launch_small<Fix<28>, 128, 4>;
         return small(d_desc, batch, d_diag, d_A, d_d, d_e, d_tau, d_order, d_status, st);
     }
-    auto* launch = variant == 0 ? launch_cluster<Fix, 2> : launch_cluster<Fix, 4>;
+    auto* launch = variant == 0 ? launch_cluster<Fix<27>, 2> : launch_cluster<Fix<27>, 4>;
     return launch(h_desc, d_desc, batch, max_ld, d_diag, d_A, d_spill, d_d, d_e, d_tau, d_order, d_counter, d_status,
                   st);
 }

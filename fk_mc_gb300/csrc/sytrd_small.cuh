@@ -87,8 +87,8 @@ sytrd_small_kernel(const ChainDesc* __restrict__ descs, const double* __restrict
             return;
         }
         const int eS = m > 0x1p-900 ? ilogb(m * (1.0 + 0x1p-30)) + 1 : -899;
-        quant = scalbn(1.0, eS - 56);
-        inv = scalbn(1.0, 56 - eS);
+        quant = scalbn(1.0, eS - 30 - P::kLo);
+        inv = scalbn(1.0, 30 + P::kLo - eS);
     }
     __syncthreads();
     auto add_elem = [&](int i, int j, double a) {
@@ -151,15 +151,15 @@ sytrd_small_kernel(const ChainDesc* __restrict__ descs, const double* __restrict
                 hh = warp_sum_ll(hh);
                 hl = warp_sum_ll(hl);
                 l2 = warp_sum_ll(l2);
-                const unsigned __int128 s2 = ((unsigned __int128)(ull)hh << 52) +
-                                             (unsigned __int128)((__int128)hl << 27) + (ull)l2;
+                const unsigned __int128 s2 = ((unsigned __int128)(ull)hh << (2 * P::kLo)) +
+                                             (unsigned __int128)((__int128)hl << (P::kLo + 1)) + (ull)l2;
                 Rf = fix_reflector(s2, alpha);
                 flat = Rf.zero;
                 if (lane == 0) {
                     M.refl = Rf;
-                    const int sh = Rf.z / 2 - 8;  // 2^-62 S: sqrt(s2) has at most 62 bits there
+                    const int sh = Rf.z / 2 - 34 + P::kLo;  // 2^-62 S: sqrt(s2) has at most 62 bits there
                     const ll xn = (ll)(sh >= 0 ? Rf.xn >> sh : Rf.xn << -sh);
-                    M.er[k] = flat ? alpha * 64 : (alpha >= 0 ? -xn : xn);
+                    M.er[k] = flat ? alpha << (32 - P::kLo) : (alpha >= 0 ? -xn : xn);
                     M.dr[k] = M.x[k];
                     M.tr[k] = Rf.tau;
                 }
@@ -190,12 +190,12 @@ sytrd_small_kernel(const ChainDesc* __restrict__ descs, const double* __restrict
                 V vi = P::vzero();
                 if (!flat && i >= s && i < n) {
                     if constexpr (kFix) {
-                        ll v56 = 1ll << 56;
+                        ll v = 1ll << (30 + P::kLo);
                         if (i > s) {
-                            v56 = (__mul64hi(xi[m] << (Rf.z / 2 - 1), (ll)Rf.r) + 16) >> 5;
-                            if (alpha < 0) v56 = -v56;
+                            v = P::template round_to<61, 30 + P::kLo>(__mul64hi(xi[m] << (Rf.z / 2 - 1), (ll)Rf.r));
+                            if (alpha < 0) v = -v;
                         }
-                        vi = P::split(v56);
+                        vi = P::split(v);
                     } else {
                         vi = i == s ? 1.f : xi[m] * scale;
                     }
@@ -203,7 +203,7 @@ sytrd_small_kernel(const ChainDesc* __restrict__ descs, const double* __restrict
                 M.vq[(i % G) * kStride + i / G] = vi;
                 if (i > s && i < n) {
                     if constexpr (kFix) {
-                        if (Aout) A[(size_t)k * ld + i] = (double)P::join(vi) * 0x1p-56;
+                        if (Aout) A[(size_t)k * ld + i] = (double)P::join(vi) * (1.0 / (1ll << (30 + P::kLo)));
                     } else {
                         A[(size_t)k * ld + i] = vi;
                     }
@@ -237,7 +237,7 @@ sytrd_small_kernel(const ChainDesc* __restrict__ descs, const double* __restrict
             Acc pv;
             P::zero(pv);
             if (q == 0) {
-                if constexpr (kFix) P::mac(pv, P::split((p + 8) >> 4), vr);
+                if constexpr (kFix) P::mac(pv, P::split(P::template round_to<60, 30 + P::kLo>(p)), vr);
                 else P::mac(pv, p, vr);
             }
             S pvs = P::sum(pv);
@@ -255,11 +255,10 @@ sytrd_small_kernel(const ChainDesc* __restrict__ descs, const double* __restrict
             if constexpr (kFix) {
                 pv = warp_sum_ll(pv);
                 const ll tau = (ll)M.refl.tau;
-                const ll kk = __mul64hi(__mul64hi(pv, tau), tau);  // 2^-57 S: tau^2 p.v / 2
                 Acc kv;
                 P::zero(kv);
-                P::mac(kv, P::split((kk + 2) >> 2), vr);           // 2^-59 S
-                wr = P::split((2 * __mul64hi(p, tau) - P::sum(kv) + 8) >> 4);
+                P::mac(kv, P::k_value(pv, tau), vr);
+                wr = P::w_entry(p, tau, kv);
             } else {
                 pv = warp_sum(pv);
                 const float tau = M.tau;
@@ -298,7 +297,7 @@ sytrd_small_kernel(const ChainDesc* __restrict__ descs, const double* __restrict
         if constexpr (kFix) x = P::join(a[e]);
         else x = a[e];
         if (c == r) M.dr[r] = x;
-        else if constexpr (kFix) M.er[c] = x * 64;
+        else if constexpr (kFix) M.er[c] = x << (32 - P::kLo);
         else M.er[c] = x;
     }
     __syncthreads();
@@ -307,7 +306,7 @@ sytrd_small_kernel(const ChainDesc* __restrict__ descs, const double* __restrict
         double* e = eout + D.v_off + i;
         if constexpr (kFix) {
             *d = (double)M.dr[i] * quant;
-            if (i < n - 1) *e = (double)M.er[i] * (quant * 0x1p-6);
+            if (i < n - 1) *e = (double)M.er[i] * (quant / (1ll << (32 - P::kLo)));
             if (Aout && i < n - 2) tauout[D.v_off + i] = (double)M.tr[i] * 0x1p-62;
         } else {
             *d = (double)M.dr[i];
