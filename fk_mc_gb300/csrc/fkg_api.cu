@@ -228,7 +228,8 @@ int enqueue_solve(fkg_ctx* ctx, Workspace& ws, const Layout& L, bool want_exp, c
         FKG_CUDA(ctx, launch_sytrd_f64(L.desc.data(), dd, L.batch, L.max_ld, (const double*)ws.diag.p,
                                        want_q ? A : nullptr, want_q ? ws.tiles.p : ws.A.p, (double*)ws.d.p,
                                        (double*)ws.e.p, (double*)ws.tau.p, ctx->st, pick_variant(ctx, L, false),
-                                       (const int*)ws.order.p, (int*)ws.counter.p, (int*)ctx->status.p));
+                                       (const int*)ws.order.p, (int*)ws.counter.p, ctx->num_sms,
+                                       (int*)ctx->status.p));
         stage_end(ctx, FKG_STAGE_REDUCE);
         ctx->launches++;
     } else {

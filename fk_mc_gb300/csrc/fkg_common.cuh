@@ -230,7 +230,7 @@ int kpm_warps_per_cta(int bmax);
 cudaError_t launch_sytrd_f64(const ChainDesc* h_desc, const ChainDesc* d_desc, int batch, int max_ld,
                              const double* d_diag, double* d_A, void* d_spill, double* d_d, double* d_e,
                              double* d_tau, cudaStream_t st, int variant, const int* d_order, int* d_counter,
-                             int* d_status);
+                             int num_sms, int* d_status);
 cudaError_t launch_sytrd_f32(const ChainDesc* h_desc, const ChainDesc* d_desc, int batch, int max_ld,
                              const double* d_diag, float* d_A, void* d_spill, double* d_d, double* d_e, float* d_tau,
                              cudaStream_t st, const int* d_order, int* d_counter, int num_sms, int* d_status);

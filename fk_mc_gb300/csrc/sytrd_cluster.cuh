@@ -94,10 +94,10 @@ __device__ __forceinline__ T reduce_scatter(T (&x)[VN], int lane, int& idx) {
     return x[0];
 }
 
-// W = 8: two CTAs share an SM (128 registers a thread); W = 16: one
+// W warps a CTA; four CTAs of 4 warps, two of 8 or one of 16 share an SM
 template <int W>
 struct F32 {
-    static constexpr int kWarps = W, kOcc = W == 8 ? 2 : 1;
+    static constexpr int kWarps = W, kOcc = 16 / W;
     static constexpr double kBase = 6.0, kPerRow = 0.0035, kPerTile = 0.115;  // column time, see launch_cluster
     using V = float;  // matrix / vector entry
     using S = float;  // sum
@@ -129,10 +129,11 @@ struct F32 {
 
 // LO: bits of the low limb (quanta 2^-(30 + LO) S of a matrix, 2^-(30 + LO) of
 // v, 2^-(29 + LO) S of w). 27 keeps the cross sums below 2^63 for n <= 1024, 28 for
-// n <= 256.
-template <int LO>
+// n <= 256. W warps a CTA; two CTAs of 4 warps or one of 8 (~240 registers a
+// thread) share an SM.
+template <int LO, int W>
 struct Fix {
-    static constexpr int kWarps = 8, kOcc = 1;  // ~240 registers a thread
+    static constexpr int kWarps = W, kOcc = 8 / W;
     static constexpr double kBase = 8.8, kPerRow = 0.0034, kPerTile = 0.68;
     static constexpr int kLo = LO;
     using V = int2;  // (hi, lo)

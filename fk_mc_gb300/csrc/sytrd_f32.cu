@@ -4,11 +4,11 @@
 
 namespace fkg {
 
-// Two CTAs of 8 warps on an SM overlap each other's barriers but halve the
-// shared memory that a chain's tiles get; measured ms (NB = 4; 8 | 16 warps): 512
-// chains of N = 64 0.34 | 0.68, 304 of N = 256 1.10 | 1.82, 304 of N = 400 3.12 |
-// 3.98, 128 of N = 400 2.28 | 2.00, 256 of N = 576 8.5 | 7.9, one of N = 1024 7.2 |
-// 6.4. Panels of 8 halve the updates' passes over tiles in global memory, which
+// Several CTAs on an SM overlap each other's barriers but share its shared
+// memory among their tiles; measured ms (NB = 4; 4 | 8 | 16 warps): 512 chains of
+// N = 144 0.62 | 0.96, 304 of N = 144 0.51 | 0.49, 512 of N = 256 1.62 | 2.18, 304 of
+// N = 256 1.30 | 1.10 | 1.82, 304 of N = 400 3.71 | 3.12 | 3.98, 128 of N = 400 - | 2.28 |
+// 2.00, 256 of N = 576 - | 8.5 | 7.9, one of N = 1024 - | 7.2 | 6.4. Panels of 8 halve the updates' passes over tiles in global memory, which
 // pays where most tiles lie there: 128 chains of N = 1024 26.6 (4), 24.6 (8); 152 of
 // N = 784 12.7, 12.3; 32 of N = 1024 7.4, 8.2; 256 of N = 576 7.9, 8.8.
 cudaError_t launch_sytrd_f32(const ChainDesc* h_desc, const ChainDesc* d_desc, int batch, int max_ld,
@@ -23,7 +23,8 @@ cudaError_t launch_sytrd_f32(const ChainDesc* h_desc, const ChainDesc* d_desc, i
         return small(d_desc, batch, d_diag, d_A, d_d, d_e, d_tau, d_order, d_status, st);
     }
     const bool narrow = max_ld <= 256 || (max_ld <= 480 && batch > num_sms);
-    auto* launch = narrow                          ? launch_cluster<F32<8>, 4>
+    auto* launch = max_ld <= 256 && batch > 2 * num_sms ? launch_cluster<F32<4>, 4>
+                   : narrow                     ? launch_cluster<F32<8>, 4>
                    : max_ld > 768 && batch > 96 ? launch_cluster<F32<16>, 8>
                                                    : launch_cluster<F32<16>, 4>;
     return launch(h_desc, d_desc, batch, max_ld, d_diag, d_A, d_spill, d_d, d_e, d_tau, d_order, d_counter, d_status,

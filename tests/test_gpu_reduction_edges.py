@@ -43,7 +43,7 @@ def _check(s, H, diags):
 @pytest.fixture()
 def solver(cuda_ok, fkg_lib):
     import fk_mc_gb300
-    s = fk_mc_gb300.Solver(max_n=1024, max_batch=160, precision="f64")
+    s = fk_mc_gb300.Solver(max_n=1024, max_batch=170, precision="f64")
     yield s
     s.close()
 
@@ -56,7 +56,7 @@ def test_orders_around_tiles(solver, n):
     _check(solver, H, [rng.uniform(-2, 2, n) for _ in range(3)])
 
 
-@pytest.mark.parametrize("n,B", [(353, 1), (353, 20), (353, 60), (353, 160), (700, 1), (700, 40), (1000, 2), (1024, 17)])
+@pytest.mark.parametrize("n,B", [(353, 1), (353, 20), (353, 60), (353, 160), (200, 170), (384, 170), (385, 153), (700, 1), (700, 40), (1000, 2), (1024, 17)])
 def test_cluster_sizes_and_spilled_tiles(solver, n, B):
     rng = np.random.default_rng(n + B)
     H = _random_csr(n, rng)

@@ -51,7 +51,7 @@ def test_orders_around_tiles(solver, n):
     _run(solver, n, 3, n)
 
 
-@pytest.mark.parametrize("n,B", [(200, 310), (256, 153), (350, 1), (350, 160), (480, 160), (481, 160), (600, 20),
+@pytest.mark.parametrize("n,B", [(200, 310), (256, 305), (130, 306), (256, 153), (350, 1), (350, 160), (480, 160), (481, 160), (600, 20),
                                  (700, 60), (1000, 2), (1024, 17), (800, 100)])
 def test_cluster_sizes_and_warp_counts(solver, n, B):
     _run(solver, n, B, n + B)
