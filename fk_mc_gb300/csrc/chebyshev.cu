@@ -97,27 +97,38 @@ __device__ double ritz_extreme(const dfl* al, const dfl* b2, int k, double glo, 
     return warp_extreme(al, b2, k, glo, ghi, largest);
 }
 
-// Block-wide double-float sum, returned as FP64 to every thread; the
-// cross-warp step is done once (thread 0). `red` needs blockDim/32 + 1 slots.
-__device__ __forceinline__ double block_sum_df(dfl x, float2* red) {
+// Block-wide double-float sum, to every thread: each warp's sum through shared
+// memory, the cross-warp sum by every thread itself (fixed order), one barrier.
+// `red` alternates between two sets of blockDim/32 slots (phase), so that the
+// next call may write while a slow warp still reads this one's.
+__device__ __forceinline__ dfl block_sum_df(dfl x, float2 (*red)[kKpmThreads / 32], int& phase) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    float2* r = red[phase];
+    phase ^= 1;
     x = warp_sum_df(x);
-    if (lane == 0) red[wid] = make_float2(x.hi, x.lo);
+    if (lane == 0) r[wid] = make_float2(x.hi, x.lo);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        dfl s = {red[0].x, red[0].y};
-        for (int i = 1; i < nw; ++i) s = df_add(s, {red[i].x, red[i].y});
-        red[nw] = make_float2(s.hi, s.lo);
-    }
-    __syncthreads();
-    const double r = (double)red[nw].x + (double)red[nw].y;
-    __syncthreads();  // red is reused by the next call
-    return r;
+    dfl t = {0.0f, 0.0f};
+    if (lane < nw) t = {r[lane].x, r[lane].y};
+    return warp_sum_df(t);
+}
+
+// sqrt(x), x > 0: the FP32 root corrected by one Newton step carried in
+// double-float (s + (x - s^2) / (2 s), the residual formed exactly by fma)
+__device__ __forceinline__ dfl df_sqrt(dfl x) {
+    if (!(x.hi > 0.0f)) return {0.0f, 0.0f};
+    const float s = sqrtf(x.hi);
+    const float r = fmaf(-s, s, x.hi) + x.lo;
+    const float c = 0.5f * r / s, h = s + c;
+    return {h, c - (h - s)};
 }
 
 // Lanczos on H = hopping + diag(d) from a fixed start vector, no
 // re-orthogonalisation (the extreme Ritz values converge regardless), in
-// double-float with the three Lanczos vectors in shared memory. Every 16
+// double-float with the three Lanczos vectors in shared memory. The scalars of a
+// step (alpha, beta, 1/beta) stay in double-float too: as FP64 numbers their square
+// root, division and conversions, done by every warp, kept the narrow FP64 pipe busy
+// for half of the kernel. Every 16
 // steps warp 0 and warp 1 compute the smallest and largest eigenvalue of the
 // Lanczos tridiagonal; the run stops when both moved less than 1e-13 of the
 // spectral width in two consecutive checks, when the Krylov space is
@@ -135,7 +146,8 @@ kpm_bounds_kernel(const KpmDesc* __restrict__ descs, const double* __restrict__ 
     dfl* V1 = V0 + D.ld;
     dfl* V2 = V1 + D.ld;
     dfl* dgd = V2 + D.ld;
-    __shared__ float2 red[kKpmThreads / 32 + 1];
+    __shared__ float2 red[2][kKpmThreads / 32];
+    int phase = 0;
     __shared__ double redd[kKpmThreads / 32];
     __shared__ double ext[2];
     const double* dg = diag + D.v_off;
@@ -148,14 +160,16 @@ kpm_bounds_kernel(const KpmDesc* __restrict__ descs, const double* __restrict__ 
         dgd[i] = df_of(dg[i]);
         s2 = df_add(s2, df_mul(v, v));
     }
-    const dfl inv = df_of(1.0 / sqrt(block_sum_df(s2, red)));
+    const dfl inv = df_rcp(df_sqrt(block_sum_df(s2, red, phase)));
     for (int i = tid; i < n; i += blockDim.x) V1[i] = df_mul(V1[i], inv);
     __syncthreads();
-    double bprev = 0.0, hnorm = 0.0, tmin = 0.0, tmax = 0.0, dmin = 0.0, dmax = 0.0;
+    dfl bprev = {0.0f, 0.0f};
+    float hnorm = 0.0f;
+    double tmin = 0.0, tmax = 0.0, dmin = 0.0, dmax = 0.0;
     int stable = 0, kdim = 0;
     bool have_prev = false, done = false;
     for (int k = 0; k < kmax && !done; ++k) {
-        const dfl nb = df_of(-bprev);
+        const dfl nb = {-bprev.hi, -bprev.lo};
         dfl dot = {0.0f, 0.0f};
         for (int i = tid; i < n; i += blockDim.x) {
             dfl sacc = df_mul(dgd[i], V1[i]);
@@ -167,24 +181,24 @@ kpm_bounds_kernel(const KpmDesc* __restrict__ descs, const double* __restrict__ 
             V2[i] = w;
             dot = df_add(dot, df_mul(w, V1[i]));
         }
-        const double alpha = block_sum_df(dot, red);
-        const dfl na = df_of(-alpha);
+        const dfl alpha = block_sum_df(dot, red, phase);
+        const dfl na = {-alpha.hi, -alpha.lo};
         dfl nn = {0.0f, 0.0f};
         for (int i = tid; i < n; i += blockDim.x) {
             const dfl w = df_add(V2[i], df_mul(na, V1[i]));
             V2[i] = w;
             nn = df_add(nn, df_mul(w, w));
         }
-        const double beta = sqrt(block_sum_df(nn, red));
+        const dfl beta2 = block_sum_df(nn, red, phase), beta = df_sqrt(beta2);
         if (tid == 0) {
-            al[k] = df_of(alpha);
-            b2[k] = df_of(beta * beta);
+            al[k] = alpha;
+            b2[k] = beta2;
         }
-        hnorm = fmax(hnorm, fabs(alpha) + beta + bprev);
+        hnorm = fmaxf(hnorm, fabsf(alpha.hi) + beta.hi + bprev.hi);
         kdim = k + 1;
-        const bool exhausted = !(beta > 1e-11 * hnorm);
+        const bool exhausted = !(beta.hi > 1e-11f * hnorm);
         if (!exhausted) {
-            const dfl ib = df_of(1.0 / beta);
+            const dfl ib = df_rcp(beta);
             for (int i = tid; i < n; i += blockDim.x) V2[i] = df_mul(V2[i], ib);
         }
         __syncthreads();  // al/b2 and the new vector visible to all
@@ -332,21 +346,35 @@ __global__ void kpm_moments_kernel(const KpmDesc* __restrict__ descs, const doub
 // logZ. M moments (even), G grid points.
 __global__ void __launch_bounds__(kKpmThreads)
 kpm_final_kernel(const KpmDesc* __restrict__ descs, const double* __restrict__ part, const KpmAB* __restrict__ ab,
-                 const double* __restrict__ beta_c, int M, int G, double* __restrict__ mu_out,
+                 const double* __restrict__ beta_c, int M, int G, int mblk, double* __restrict__ mu_out,
                  double* __restrict__ logz, int* __restrict__ status) {
     extern __shared__ __align__(16) double ksm[];
-    __shared__ double red[kKpmThreads / 32];
+    __shared__ double psum[kKpmThreads];
     const KpmDesc D = descs[blockIdx.x];
     const int R = D.R, nq = 3 * R, n = D.n, tid = threadIdx.x;
     double* sums = ksm;          // nq
     double* mu = sums + nq;      // M
     double* fg = mu + M;         // G: logz_f on the grid
     double* cm = fg + G;         // M: coefficients
-    for (int q = 0; q < nq; ++q) {
+    double* ac = cm + M;         // G: angles of the grid
+    double* tab = ac + G;        // mblk x G: T_m on the grid
+    // column sums: thread (g, q) adds every ng-th column (coalesced rows of nq), then
+    // the ng partial sums in order
+    const int ng = max(1, (int)blockDim.x / nq);
+    for (int t = tid; t < nq * ng; t += blockDim.x) {
+        const int q = t % nq;
         double s = 0.0;
-        for (int j = tid; j < n; j += blockDim.x) s += part[(size_t)(D.v_off + j) * nq + q];
-        s = block_sum(s, red);
-        if (tid == 0) sums[q] = s;
+        for (int j = t / nq; j < n; j += ng) s += part[(size_t)(D.v_off + j) * nq + q];
+        if (ng == 1) sums[q] = s;
+        else psum[t] = s;
+    }
+    if (ng > 1) {
+        __syncthreads();
+        if (tid < nq) {
+            double s = psum[tid];
+            for (int g = 1; g < ng; ++g) s += psum[g * nq + tid];
+            sums[tid] = s;
+        }
     }
     const KpmAB st = ab[blockIdx.x];
     const double a = st.a, b = st.b, beta = beta_c[blockIdx.x], N = (double)n;
@@ -376,15 +404,23 @@ kpm_final_kernel(const KpmDesc* __restrict__ descs, const double* __restrict__ p
             }
         }
     }
-    // c_m = moment_f(logz_f, m): trapezoid in the angle (include/fk_mc/chebyshev.hpp:38-56)
-    for (int m = tid; m < M; m += blockDim.x) {
-        double s = 0.0;
-        for (int i = 0; i + 1 < G; ++i) {
-            const double xi = -cos(M_PI * ((double)i * step)), xi1 = -cos(M_PI * ((double)(i + 1) * step));
-            const double ti = cos((double)m * acos(xi)), ti1 = cos((double)m * acos(xi1));
-            s += (fg[i + 1] * ti1 + fg[i] * ti) * ((double)(i + 1) * step - (double)i * step);
+    // c_m = moment_f(logz_f, m): trapezoid in the angle (include/fk_mc/chebyshev.hpp:38-56).
+    // T_m(x_i) = cos(m acos(x_i)) of the grid in parallel, then the sums (a thread
+    // per moment evaluated six FP64 functions per grid interval before). acos(x_i)
+    // once per point; the table goes in blocks of moments that fit its space.
+    for (int i = tid; i < G; i += blockDim.x) ac[i] = acos(-cos(M_PI * ((double)i * step)));
+    for (int m0 = 0; m0 < M; m0 += mblk) {
+        const int mb = min(mblk, M - m0);
+        __syncthreads();
+        for (int q = tid; q < mb * G; q += blockDim.x) tab[q] = cos((double)(m0 + q / G) * ac[q % G]);
+        __syncthreads();
+        for (int m = tid; m < mb; m += blockDim.x) {
+            const double* t = tab + (size_t)m * G;
+            double s = 0.0;
+            for (int i = 0; i + 1 < G; ++i)
+                s += (fg[i + 1] * t[i + 1] + fg[i] * t[i]) * ((double)(i + 1) * step - (double)i * step);
+            cm[m0 + m] = s * 0.5;
         }
-        cm[m] = s * 0.5;
     }
     __syncthreads();
     if (tid == 0) {
@@ -423,9 +459,12 @@ cudaError_t launch_kpm(const KpmDesc* d_kdesc, int batch, int max_n, int max_ld,
     kpm_moments_kernel<<<dim3((max_n + wpc - 1) / wpc, batch), 32 * wpc, sm_m, st>>>(d_kdesc, d_diag, d_ab, d_part,
                                                                                       wpc);
     if ((err = cudaGetLastError())) return err;
-    const size_t sm_f = sizeof(double) * (3 * (size_t)R + 2 * (size_t)M + (size_t)G);
+    // moments per block of the T_m table: as many as fit in 64 KB
+    const int mblk = max(1, min(M, (int)(8192 / G)));
+    const size_t sm_f = sizeof(double) * (3 * (size_t)R + 2 * (size_t)M + (2 + (size_t)mblk) * (size_t)G);
     if ((err = cudaFuncSetAttribute(kpm_final_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_f))) return err;
-    kpm_final_kernel<<<batch, kKpmThreads, sm_f, st>>>(d_kdesc, d_part, d_ab, d_beta, M, G, d_mu, d_logz, d_status);
+    kpm_final_kernel<<<batch, kKpmThreads, sm_f, st>>>(d_kdesc, d_part, d_ab, d_beta, M, G, mblk, d_mu, d_logz,
+                                                     d_status);
     return cudaGetLastError();
 }
 
