@@ -36,7 +36,7 @@
 namespace fkg {
 namespace {
 
-constexpr int kR1Threads = 256;
+constexpr int kR1MaxThreads = 640;
 
 __device__ __forceinline__ void neumaier(double& s, double& c, double term) {
     const double t = s + term;
@@ -44,10 +44,21 @@ __device__ __forceinline__ void neumaier(double& s, double& c, double term) {
     s = t;
 }
 
+// 1/a to the pair's accuracy: FP32 estimate, residual 1 - a q formed exactly by
+// fma, second-order correction (the IEEE FP32 division of df_rcp costs as much
+// as the rest of a term)
+__device__ __forceinline__ dfl df_rcp2(dfl a) {
+    const float q = __fdividef(1.0f, a.hi);
+    const float p = a.hi * q, pe = fmaf(a.hi, q, -p);
+    const float e = ((1.0f - p) - pe) - a.lo * q;
+    const float rl = q * fmaf(e, e, e), h = q + rl;
+    return {h, rl - (h - q)};
+}
+
 // n eigenvalues per proposal (ascending), z: n weights (row `site` of the
 // eigenvector matrix), rho: the diagonal change, beta. Outputs logz and,
 // when ev_out is not null, the new eigenvalues ascending.
-__global__ void __launch_bounds__(kR1Threads)
+__global__ void __launch_bounds__(kR1MaxThreads)
 rank1_kernel(int n, const double* __restrict__ evals, const double* __restrict__ zrow, const double* __restrict__ rho_c,
              const double* __restrict__ beta_c, double* __restrict__ logz, double* __restrict__ ev_out,
              int* __restrict__ status) {
@@ -59,9 +70,9 @@ rank1_kernel(int n, const double* __restrict__ evals, const double* __restrict__
     float2* dhl = (float2*)(root + n);  // poles as FP32 pairs hi + lo
     float2* whl = dhl + n;              // weights as FP32 pairs hi + lo
     __shared__ int sh_m, sh_nf;
-    __shared__ double sh_tol;
-    __shared__ double ps[kR1Threads], pc[kR1Threads];
-    const int c = blockIdx.x, tid = threadIdx.x;
+    __shared__ double ps[kR1MaxThreads / 32], pc[kR1MaxThreads / 32];
+    __shared__ int pm[kR1MaxThreads / 32];
+    const int c = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
     const double* lam = evals + (size_t)c * n;
     const double* z = zrow + (size_t)c * n;
     const double rho_s = rho_c[c], beta = beta_c[c];
@@ -73,15 +84,55 @@ rank1_kernel(int n, const double* __restrict__ evals, const double* __restrict__
         w[k] = z[src];  // z for now; squared below
     }
     __syncthreads();
-    if (tid == 0) {
-        // deflation, in pole order: merge (nearly) equal poles by a Givens
-        // rotation of their z components, drop negligible weights
-        double dmax = 0.0, zz = 0.0;
-        for (int k = 0; k < n; ++k) {
-            dmax = fmax(dmax, fabs(d[k]));
-            zz += w[k] * w[k];
+    // deflation tolerance from max |d| and the total weight
+    double dmax = 0.0, zz = 0.0;
+    for (int k = tid; k < n; k += blockDim.x) {
+        dmax = fmax(dmax, fabs(d[k]));
+        zz += w[k] * w[k];
+    }
+    dmax = warp_max(dmax);
+    zz = warp_sum(zz);
+    if (lane == 0) { ps[warp] = dmax; pc[warp] = zz; }
+    __syncthreads();
+    dmax = warp_max(lane < nwarp ? ps[lane] : 0.0);
+    zz = warp_sum(lane < nwarp ? pc[lane] : 0.0);
+    const double tol = 8.0 * DBL_EPSILON * fmax(dmax, rho * zz);
+    bool close = false;
+    for (int k = tid; k + 1 < n; k += blockDim.x) close = close || d[k + 1] - d[k] <= tol;
+    if (!__syncthreads_or(close)) {
+        // no equal poles: only negligible weights leave. Compaction in pole order,
+        // in place (chunks of blockDim poles: the kept ones move down, behind the
+        // chunks already read).
+        int m = 0;
+        for (int k0 = 0; k0 < n; k0 += blockDim.x) {
+            const int k = k0 + tid;
+            const double dk = k < n ? d[k] : 0.0, zk = k < n ? w[k] : 0.0;
+            const bool keep = k < n && !(rho * zk * zk <= tol);
+            const unsigned mask = __ballot_sync(0xffffffffu, keep);
+            if (lane == 0) pm[warp] = __popc(mask);
+            __syncthreads();
+            int before = 0, total = 0;
+            for (int q = 0; q < nwarp; ++q) {
+                if (q < warp) before += pm[q];
+                total += pm[q];
+            }
+            const int pos = m + before + __popc(mask & ((1u << lane) - 1));
+            if (keep) {
+                d[pos] = dk;
+                w[pos] = zk * zk;
+            } else if (k < n) {
+                fixed[k - pos] = dk;  // the poles dropped before k
+            }
+            m += total;
+            __syncthreads();
         }
-        const double tol = 8.0 * DBL_EPSILON * fmax(dmax, rho * zz);
+        if (tid == 0) {
+            sh_m = m;
+            sh_nf = n - m;
+        }
+    } else if (tid == 0) {
+        // in pole order: merge (nearly) equal poles by a Givens rotation of their z
+        // components, drop negligible weights
         int m = 0, nf = 0;
         double cd = d[0], cz = w[0];
         for (int k = 1; k <= n; ++k) {
@@ -119,11 +170,9 @@ rank1_kernel(int n, const double* __restrict__ evals, const double* __restrict__
         }
         sh_m = m;
         sh_nf = nf;
-        sh_tol = tol;
     }
     __syncthreads();
     const int m = sh_m, nf = sh_nf;
-    const double tol = sh_tol;
     double wsum_l = 0.0;
     for (int k = tid; k < m; k += blockDim.x) {
         const float hi = (float)d[k];
@@ -132,17 +181,11 @@ rank1_kernel(int n, const double* __restrict__ evals, const double* __restrict__
         whl[k] = make_float2(wh, (float)(w[k] - (double)wh));
         wsum_l += w[k];
     }
-    // total weight (for the last root's bracket): a fixed-order block sum
-    ps[tid] = wsum_l;
+    // total weight, for the last root's bracket
+    wsum_l = warp_sum(wsum_l);
+    if (lane == 0) ps[warp] = wsum_l;
     __syncthreads();
-    if (tid == 0) {
-        double s = 0.0;
-        for (int q = 0; q < (int)blockDim.x; ++q) s += ps[q];
-        pc[0] = s;
-    }
-    __syncthreads();
-    const double wsum = pc[0];
-    __syncthreads();
+    const double wsum = warp_sum(lane < nwarp ? ps[lane] : 0.0);
     const float rhof = (float)rho;
     int bad = 0;
     for (int i = tid; i < m; i += blockDim.x) {
@@ -199,7 +242,7 @@ rank1_kernel(int n, const double* __restrict__ evals, const double* __restrict__
             for (int k = 0; k < m; ++k) {
                 const float2 q = dhl[k], wq = whl[k];
                 const dfl den = df_add(df_add({q.x, q.y}, {-og.x, -og.y}), nt);
-                const dfl r = df_rcp(den);
+                const dfl r = df_rcp2(den);
                 const dfl wr = df_mul({wq.x, wq.y}, r);
                 F = df_add(F, wr);
                 FP = df_add(FP, df_mul(wr, r));
@@ -234,7 +277,8 @@ rank1_kernel(int n, const double* __restrict__ evals, const double* __restrict__
         // a gap of a few deflation tolerances places the root to within the gap
         // whether or not the iteration settled
         if (!conv && gap > 1024.0 * tol) bad = 1;
-        root[i] = dorg + t;
+        // inside its gap to the last bit: the merge below relies on ascending roots
+        root[i] = last ? fmax(dorg + t, d[i]) : fmin(fmax(dorg + t, d[i]), d[i + 1]);
     }
     if (bad) atomicOr(status, kStatusNoConverge);
     __syncthreads();
@@ -245,28 +289,43 @@ rank1_kernel(int n, const double* __restrict__ evals, const double* __restrict__
         const double x = -beta * e;
         neumaier(s, cc, fmax(x, 0.0) + log1p(exp(-fabs(x))));
     }
-    ps[tid] = s;
-    pc[tid] = cc;
+    // the threads' (sum, compensation) pairs merged with TwoSum, as in logz_kernel
+    auto merge = [&](double os, double oc) {
+        double t, err;
+        two_sum(s, os, t, err);
+        s = t;
+        cc += oc + err;
+    };
+#pragma unroll 1
+    for (int o = 16; o > 0; o >>= 1)
+        merge(__shfl_xor_sync(0xffffffffu, s, o), __shfl_xor_sync(0xffffffffu, cc, o));
+    if (lane == 0) { ps[warp] = s; pc[warp] = cc; }
     __syncthreads();
     if (tid == 0) {
-        double S = 0.0, C = 0.0;
-        for (int q = 0; q < (int)blockDim.x; ++q) {
-            C += pc[q];
-            neumaier(S, C, ps[q]);
-        }
-        const double r = S + C;
+        for (int q = 1; q < nwarp; ++q) merge(ps[q], pc[q]);
+        const double r = s + cc;
         logz[c] = r;
         if (!isfinite(r)) atomicOr(status, kStatusNaN);
-        if (ev_out) {  // merge roots and fixed values, back to the original sign, ascending
-            double* out = ev_out + (size_t)c * n;
-            int a = 0, b = 0;
-            for (int k = 0; k < n; ++k) {
-                double v;
-                if (b >= nf || (a < m && root[a] <= fixed[b])) v = root[a++];
-                else v = fixed[b++];
-                if (sg > 0) out[k] = v; else out[n - 1 - k] = -v;
-            }
+    }
+    if (!ev_out) return;
+    // roots and fixed values merged, back to the original sign, ascending. Both lists
+    // ascend (each root stays in its gap), so a value's place is its own index plus
+    // the number of the other list's values before it (a root goes before an equal
+    // fixed value).
+    double* out = ev_out + (size_t)c * n;
+    for (int k = tid; k < m + nf; k += blockDim.x) {
+        const bool is_root = k < m;
+        const double v = is_root ? root[k] : fixed[k - m];
+        const double* other = is_root ? fixed : root;
+        int a = 0, b = is_root ? nf : m;
+        while (a < b) {
+            const int h = (a + b) >> 1;
+            if (is_root ? other[h] < v : other[h] <= v) a = h + 1;
+            else b = h;
         }
+        const int pos = (is_root ? k : k - m) + a;
+        if (sg > 0) out[pos] = v;
+        else out[n - 1 - pos] = -v;
     }
 }
 
@@ -280,7 +339,9 @@ cudaError_t launch_rank1(int batch, int n, const double* d_evals, const double* 
     const size_t sm = rank1_smem_bytes(n);
     cudaError_t e = cudaFuncSetAttribute(rank1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    rank1_kernel<<<batch, kR1Threads, sm, st>>>(n, d_evals, d_z, d_rho, d_beta, d_logz, d_ev_out, d_status);
+    // one root per thread and pass, with whole passes where n exceeds a block
+    const int passes = (n + kR1MaxThreads - 1) / kR1MaxThreads, threads = ((n + passes - 1) / passes + 31) / 32 * 32;
+    rank1_kernel<<<batch, threads, sm, st>>>(n, d_evals, d_z, d_rho, d_beta, d_logz, d_ev_out, d_status);
     return cudaGetLastError();
 }
 

@@ -117,3 +117,28 @@ def test_host_adapter_rank1_chain(oracle, kind, L, U, beta):
         assert np.allclose(g["weight"], r["weight"], rtol=1e-9, atol=0)
         assert np.array_equal(g["f_final"], r["f_final"])
         assert np.allclose(g["energy"], r["energy"], rtol=1e-10, atol=0)
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 640, 641, 1024])
+@pytest.mark.parametrize("weights", ["all", "some", "none"])
+def test_rank1_block_edges(cuda_ok, fkg_lib, n, weights):
+    """Orders around the block size, with all, half or none of the weights deflated: eigenvalues ascending and equal
+    to numpy's of diag(l) + rho z z^T (both within n eps ||H||)."""
+    import fk_mc_gb300
+    rng = np.random.default_rng(n)
+    lam = np.sort(rng.uniform(-4, 4, n))
+    z = rng.standard_normal(n)
+    if weights != "all":
+        z[rng.permutation(n)[:n if weights == "none" else n // 2]] = 0.0
+    z /= max(np.linalg.norm(z), 1e-300)
+    rho = np.array([1.5, -1.5])
+    s = fk_mc_gb300.Solver(max_n=n, max_batch=2)
+    try:
+        logz, ev = s.rank1_logz(np.stack([lam, lam]), np.stack([z, z]), rho, 2.0, evals_new=True)
+    finally:
+        s.close()
+    for c in range(2):
+        ref = np.linalg.eigvalsh(np.diag(lam) + rho[c] * np.outer(z, z))
+        assert np.all(np.diff(ev[c]) >= 0)
+        assert np.abs(ev[c] - ref).max() <= 4 * max(n, 8) * np.finfo(float).eps * 5.5
+        assert abs(logz[c] - np.logaddexp(0, -2.0 * ref).sum()) <= 1e-12 * n
