@@ -1066,7 +1066,7 @@ int enqueue_vectors(fkg_ctx* ctx, Workspace& ws, const Layout& L) {
                                    (const double*)ws.w.p, (double*)ws.Z64.p, (double*)ws.stein.p, ctx->st));
     stage_end(ctx, FKG_STAGE_TRIEIG);
     stage_begin(ctx, FKG_STAGE_BACK);
-    FKG_CUDA(ctx, launch_backtransform_f64(dd, L.batch, L.max_n, L.max_ld, (const double*)ws.A.p,
+    FKG_CUDA(ctx, launch_backtransform_f64(dd, L.batch, L.max_n, (const double*)ws.A.p,
                                            (const double*)ws.tau.p, (double*)ws.Tf64.p, (double*)ws.Z64.p, ctx->st));
     stage_end(ctx, FKG_STAGE_BACK);
     ctx->launches += 3;

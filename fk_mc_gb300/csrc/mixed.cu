@@ -29,7 +29,6 @@ namespace {
 
 constexpr int kNb = 32;        // reflectors per panel
 constexpr int kChunk = 128;    // rows of V staged per pass
-constexpr int kBtThreads = 256;
 constexpr int kTwBatch = 16;   // twisted factorisation: stored values read per batch
 
 template <typename T>
@@ -256,153 +255,6 @@ twisted_kernel(const ChainDesc* __restrict__ descs, const double* __restrict__ d
     zscale[D.v_off + j] = rsqrtf(nrm);  // applied when the back-transformation loads Z
 }
 
-// ---- 3. back-transformation X = Q Z, one CTA per (chain, 32-column block) ----
-// The 32-column block of Z stays in shared memory for all panels. Per panel:
-//   W = V^T Zb (32 x 32): every warp takes a slice of the rows, each lane one
-//       column c with 32 register accumulators; the V row (32 values) is read
-//       with 128-bit broadcast loads from a staged chunk; the 8 partial W are
-//       summed through shared memory;
-//   W2 = T W, kept per lane as one column (32 registers);
-//   Zb -= V W2 with the same row split and broadcast loads.
-constexpr int kVs = kNb + 4;  // staged V row stride (elements): 16-byte aligned rows
-constexpr int kBtChunk = 64;   // rows of V staged per step of the back-transformation
-constexpr int kStageRegs = kBtChunk * kNb / kBtThreads;  // V values staged per thread per chunk
-
-// V(i0 + ii, k0 + kk) for this thread's share of a chunk (lane-contiguous rows:
-// coalesced global reads), into registers, so the next chunk's loads overlap
-// the current chunk's arithmetic.
-template <typename T>
-__device__ __forceinline__ void load_v(const T* __restrict__ A, int ld, int n, int k0, int kb, int i0,
-                                       T (&r)[kStageRegs]) {
-#pragma unroll
-    for (int q = 0; q < kStageRegs; ++q) {
-        const int idx = threadIdx.x + kBtThreads * q, kk = idx / kBtChunk, ii = idx % kBtChunk;
-        r[q] = (kk < kb) ? vref(A, ld, n, k0 + kk, i0 + ii) : T(0);
-    }
-}
-template <typename T>
-__device__ __forceinline__ void store_v(const T (&r)[kStageRegs], T* __restrict__ Vs) {
-#pragma unroll
-    for (int q = 0; q < kStageRegs; ++q) {
-        const int idx = threadIdx.x + kBtThreads * q, kk = idx / kBtChunk, ii = idx % kBtChunk;
-        Vs[ii * kVs + kk] = r[q];
-    }
-}
-
-// The column block lives in shared memory for FP32 (ZB_SMEM) and stays in
-// global memory for FP64 (a 32-column FP64 block of a 1024-row matrix would
-// not fit); its row stride is zs.
-// four contiguous values from 16-byte-aligned shared memory
-__device__ __forceinline__ void load4(const double* p, double (&o)[4]) {
-    const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
-    o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
-}
-
-template <typename T, bool ZB_SMEM>
-__global__ void __launch_bounds__(kBtThreads, 2)
-backtransform_kernel(const ChainDesc* __restrict__ descs, const T* __restrict__ A32, const T* __restrict__ Tf,
-                     T* __restrict__ Zws) {
-    extern __shared__ __align__(16) unsigned char smb_raw[];
-    T* smb = reinterpret_cast<T*>(smb_raw);
-    // one chain's column blocks are adjacent in launch order (blockIdx.x), so
-    // its reflector panels are read from DRAM once and from L2 afterwards
-    const ChainDesc D = descs[blockIdx.y];
-    const int n = D.n, ld = D.ld, j0 = blockIdx.x * 32;
-    if (j0 >= n) return;
-    const T* A = A32 + D.a_off;
-    T* Z = Zws + D.a_off;
-    const int zs = ZB_SMEM ? 32 : ld;
-    T* Zb = ZB_SMEM ? smb : Z + j0;                           // row i, column c at Zb[i * zs + c]
-    T* Vs = ZB_SMEM ? smb + (size_t)ld * 32 : smb;          // [kBtChunk][kVs]
-    T* Ws = Vs + kBtChunk * kVs;                              // [4][32 kk][32 c] partial sums
-    T* Ts = Ws + 4 * kNb * 32;                                // [32][33]
-    const int t = threadIdx.x, c = t & 31, g = t >> 5;
-    if (ZB_SMEM)
-        for (int i = g; i < n; i += kBtThreads / 32) Zb[i * 32 + c] = Z[(size_t)i * ld + j0 + c];
-    const int nrefl = n - 2;
-    const int npanel = nrefl > 0 ? (nrefl + kNb - 1) / kNb : 0;
-    const T* Tbase = Tf + (D.v_off / kNb) * (size_t)(kNb * kNb);
-    T stage[kStageRegs];
-    for (int p = npanel - 1; p >= 0; --p) {
-        const int k0 = p * kNb, kb = min(kNb, nrefl - k0), r0 = k0 + 1;
-        for (int q = t; q < kNb * kNb; q += kBtThreads) Ts[(q / kNb) * (kNb + 1) + q % kNb] = Tbase[(size_t)p * kNb * kNb + q];
-        T acc[kNb];
-#pragma unroll
-        for (int kk = 0; kk < kNb; ++kk) acc[kk] = T(0);
-        load_v(A, ld, n, k0, kb, r0, stage);
-        for (int i0 = r0; i0 < n; i0 += kBtChunk) {
-            __syncthreads();
-            store_v(stage, Vs);
-            __syncthreads();
-            if (i0 + kBtChunk < n) load_v(A, ld, n, k0, kb, i0 + kBtChunk, stage);
-            const int rows = min(kBtChunk, n - i0);
-            for (int ii = g; ii < rows; ii += kBtThreads / 32) {
-                const T z = (j0 + c < ld) ? Zb[(size_t)(i0 + ii) * zs + c] : T(0);
-                const T* vr = Vs + ii * kVs;
-#pragma unroll
-                for (int q = 0; q < kNb; q += 4) {
-                    T v4[4];
-                    load4(vr + q, v4);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) acc[q + u] = fma(v4[u], z, acc[q + u]);
-                }
-            }
-        }
-        // W(kk, c) = sum of the 8 warps' partial sums, in a fixed order (a
-        // three-level tree through Ws), so the result is bit-reproducible
-#pragma unroll
-        for (int half = 4; half >= 1; half >>= 1) {
-            if (g >= half && g < 2 * half)
-#pragma unroll
-                for (int kk = 0; kk < kNb; ++kk) Ws[((g - half) * kNb + kk) * 32 + c] = acc[kk];
-            __syncthreads();
-            if (g < half)
-#pragma unroll
-                for (int kk = 0; kk < kNb; ++kk) acc[kk] += Ws[(g * kNb + kk) * 32 + c];
-            __syncthreads();
-        }
-        if (g == 0)
-#pragma unroll
-            for (int kk = 0; kk < kNb; ++kk) Ws[kk * 32 + c] = acc[kk];
-        __syncthreads();
-        T w2[kNb];
-#pragma unroll
-        for (int kk = 0; kk < kNb; ++kk) {
-            T s = T(0);
-#pragma unroll
-            for (int l = 0; l < kNb; ++l) s = fma(Ts[kk * (kNb + 1) + l], Ws[l * 32 + c], s);  // T upper triangular
-            w2[kk] = s;
-        }
-        // Zb(i, c) -= sum_kk V(i, kk) W2(kk, c), rows i in [r0, n)
-        load_v(A, ld, n, k0, kb, r0, stage);
-        for (int i0 = r0; i0 < n; i0 += kBtChunk) {
-            __syncthreads();
-            store_v(stage, Vs);
-            __syncthreads();
-            if (i0 + kBtChunk < n) load_v(A, ld, n, k0, kb, i0 + kBtChunk, stage);
-            const int rows = min(kBtChunk, n - i0);
-            for (int ii = g; ii < rows; ii += kBtThreads / 32) {
-                if (!ZB_SMEM && j0 + c >= n) continue;
-                T z0 = Zb[(size_t)(i0 + ii) * zs + c], z1 = T(0);
-                const T* vr = Vs + ii * kVs;
-#pragma unroll
-                for (int q = 0; q < kNb; q += 4) {
-                    T v4[4];
-                    load4(vr + q, v4);
-                    z0 = fma(-v4[0], w2[q], z0);
-                    z1 = fma(-v4[1], w2[q + 1], z1);
-                    z0 = fma(-v4[2], w2[q + 2], z0);
-                    z1 = fma(-v4[3], w2[q + 3], z1);
-                }
-                Zb[(size_t)(i0 + ii) * zs + c] = z0 + z1;
-            }
-        }
-        __syncthreads();
-    }
-    if (ZB_SMEM && j0 + c < n)
-        for (int i = g; i < n; i += kBtThreads / 32) Z[(size_t)i * ld + j0 + c] = Zb[i * 32 + c];
-}
-
 // ---- 4. Rayleigh quotients with the exact sparse H ----
 // theta_k = x_k^T H x_k / x_k^T x_k for the FP32 vector x_k, summed in
 // double-float (unevaluated FP32 pairs, ~48 significant bits): the diagonal
@@ -511,11 +363,6 @@ __global__ void sort_kernel(const ChainDesc* __restrict__ descs, const double* _
 
 }  // namespace
 
-template <typename T, bool ZB_SMEM>
-size_t backtransform_smem_bytes(int max_ld) {
-    return sizeof(T) * ((ZB_SMEM ? (size_t)max_ld * 32 : 0) + kBtChunk * kVs + 4 * kNb * 32 + kNb * (kNb + 1));
-}
-
 // larft (+ V T): needs only the reduction; enqueued on its own stream right
 // after it, so that it overlaps the shift and eigenvector kernels.
 cudaError_t launch_larft_vt(const ChainDesc* d_desc, int batch, int max_n, const float* d_A32, const float* d_tau32,
@@ -577,18 +424,14 @@ cudaError_t launch_mixed_refine(const ChainDesc* d_desc, int batch, int max_n, i
 
 // FP64 compact-WY factors and back-transformation (X = Q Z with Z row-major in
 // global memory) for the plain path's eigenvectors.
-cudaError_t launch_backtransform_f64(const ChainDesc* d_desc, int batch, int max_n, int max_ld, const double* d_A,
+cudaError_t launch_backtransform_f64(const ChainDesc* d_desc, int batch, int max_n, const double* d_A,
                                      const double* d_tau, double* d_Tf, double* d_Z, cudaStream_t st) {
     if (batch <= 0) return cudaSuccess;
-    cudaError_t err;
     const int npanel = (max_n + kNb - 1) / kNb;
     larft_kernel<double><<<dim3(batch, npanel), 256, 0, st>>>(d_desc, d_A, d_tau, d_Tf, nullptr, 0, 1);
-    if ((err = cudaGetLastError()) != cudaSuccess) return err;
-    const size_t sm_bt = backtransform_smem_bytes<double, false>(max_ld);
-    if ((err = cudaFuncSetAttribute(backtransform_kernel<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_bt))) return err;
-    if (batch > 65535) return cudaErrorInvalidValue;  // grid y limit
-    backtransform_kernel<double, false><<<dim3((max_n + 31) / 32, batch), kBtThreads, sm_bt, st>>>(d_desc, d_A, d_Tf, d_Z);
-    return cudaGetLastError();
+    const cudaError_t err = cudaGetLastError();
+    if (err != cudaSuccess) return err;
+    return launch_backtransform_fix(d_desc, batch, max_n, d_A, d_Tf, d_Z, st);
 }
 
 }  // namespace fkg
