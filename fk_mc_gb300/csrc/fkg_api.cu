@@ -1059,15 +1059,15 @@ int enqueue_vectors(fkg_ctx* ctx, Workspace& ws, const Layout& L) {
     const size_t V = (size_t)L.v_total;
     if ((rc = ensure_dev(ctx, ws.Z64, sizeof(double) * (size_t)L.a_total))) return rc;
     if ((rc = ensure_dev(ctx, ws.stein, sizeof(double) * stein_scratch_elems(L.a_total)))) return rc;
-    if ((rc = ensure_dev(ctx, ws.Tf64, sizeof(double) * 32 * V))) return rc;
+    if ((rc = ensure_dev(ctx, ws.Tf64, sizeof(long long) * 4 * V))) return rc;
     const ChainDesc* dd = (const ChainDesc*)ws.desc.p;
     stage_begin(ctx, FKG_STAGE_TRIEIG);
     FKG_CUDA(ctx, launch_stein_f64(dd, L.batch, L.max_n, L.max_ld, (const double*)ws.d.p, (const double*)ws.e.p,
                                    (const double*)ws.w.p, (double*)ws.Z64.p, (double*)ws.stein.p, ctx->st));
     stage_end(ctx, FKG_STAGE_TRIEIG);
     stage_begin(ctx, FKG_STAGE_BACK);
-    FKG_CUDA(ctx, launch_backtransform_f64(dd, L.batch, L.max_n, (const double*)ws.A.p,
-                                           (const double*)ws.tau.p, (double*)ws.Tf64.p, (double*)ws.Z64.p, ctx->st));
+    FKG_CUDA(ctx, launch_backtransform_f64(dd, L.batch, L.max_n, (double*)ws.A.p, (const double*)ws.tau.p,
+                                           (long long*)ws.Tf64.p, (double*)ws.Z64.p, ctx->st));
     stage_end(ctx, FKG_STAGE_BACK);
     ctx->launches += 3;
     return FKG_OK;

@@ -268,10 +268,8 @@ cudaError_t launch_mixed_refine(const ChainDesc* d_desc, int batch, int max_n, i
                                 cudaEvent_t ev_fork, cudaEvent_t ev_join, cudaEvent_t ev_larft, int bt_variant,
                                 long long wait_iters, int shift, const float* d_Q2, long long q2t_off,
                                 void (*stage)(void*, int, int), void* sctx);
-cudaError_t launch_backtransform_f64(const ChainDesc* d_desc, int batch, int max_n, const double* d_A,
-                                     const double* d_tau, double* d_Tf, double* d_Z, cudaStream_t st);
-cudaError_t launch_backtransform_fix(const ChainDesc* d_desc, int batch, int max_n, const double* d_A,
-                                     const double* d_Tf, double* d_Z, cudaStream_t st);
+cudaError_t launch_backtransform_f64(const ChainDesc* d_desc, int batch, int max_n, double* d_A, const double* d_tau,
+                                     long long* d_Tf, double* d_Z, cudaStream_t st);
 size_t stein_scratch_elems(long long a_total);
 cudaError_t launch_cluster_fix_f32(const ChainDesc* d_desc, int batch, int max_ld, const double* d_d,
                                    const double* d_e, const double* d_w, const double* d_ctol, float* d_Z,

@@ -31,13 +31,12 @@ constexpr int kNb = 32;        // reflectors per panel
 constexpr int kChunk = 128;    // rows of V staged per pass
 constexpr int kTwBatch = 16;   // twisted factorisation: stored values read per batch
 
-template <typename T>
-__device__ __forceinline__ T vref(const T* __restrict__ A, int ld, int n, int k, int i, int shift = 1) {
+__device__ __forceinline__ float vref(const float* __restrict__ A, int ld, int n, int k, int i, int shift = 1) {
     // element i of Householder vector k (v_k(k+shift) = 1, zero above; shift 1
     // for the one-stage reduction, the band width for the two-stage one)
-    if (i == k + shift) return T(1);
+    if (i == k + shift) return 1.f;
     if (i > k + shift && i < n) return A[(size_t)k * ld + i];
-    return T(0);
+    return 0.f;
 }
 
 // ---- 1. compact-WY factors, one CTA per (chain, panel) ----
@@ -50,31 +49,30 @@ __device__ __forceinline__ T vref(const T* __restrict__ A, int ld, int n, int k,
 // itself (every column block of a chain would otherwise split the same V).
 // FP32: 64 registers (no spills) so that four CTAs share an SM and hide the
 // latency of the V loads
-template <typename T>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
-larft_kernel(const ChainDesc* __restrict__ descs, const T* __restrict__ A32, const T* __restrict__ tau,
-             T* __restrict__ Tf, T* __restrict__ VT, long long plane, int shift) {
+__global__ void __launch_bounds__(256, 4)
+larft_kernel(const ChainDesc* __restrict__ descs, const float* __restrict__ A32, const float* __restrict__ tau,
+             float* __restrict__ Tf, float* __restrict__ VT, long long plane, int shift) {
     const ChainDesc D = descs[blockIdx.x];
     const int n = D.n, ld = D.ld, p = blockIdx.y;
     const int nrefl = n - 1 - shift;  // reflector k has its unit at row k + shift
     const int npanel = (nrefl + kNb - 1) / kNb;
     if (nrefl <= 0 || p >= npanel) return;
     const int k0 = p * kNb, kb = min(kNb, nrefl - k0), r0 = k0 + shift;
-    const T* A = A32 + D.a_off;
-    __shared__ T Vc[kChunk][kNb + 1];
-    __shared__ T G[kNb][kNb + 1];
-    __shared__ T Ts[kNb][kNb + 1];
+    const float* A = A32 + D.a_off;
+    __shared__ float Vc[kChunk][kNb + 1];
+    __shared__ float G[kNb][kNb + 1];
+    __shared__ float Ts[kNb][kNb + 1];
     const int t = threadIdx.x, c = t & 31, g = t >> 5;
-    T acc[4] = {T(0), T(0), T(0), T(0)};  // G[g + 8q][c]
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};  // G[g + 8q][c]
     for (int i0 = r0; i0 < n; i0 += kChunk) {
         for (int q = 0; q < kChunk * kNb / 256; ++q) {
             const int idx = t + 256 * q, kk = idx / kChunk, ii = idx % kChunk;
-            Vc[ii][kk] = (kk < kb) ? vref(A, ld, n, k0 + kk, i0 + ii, shift) : T(0);
+            Vc[ii][kk] = (kk < kb) ? vref(A, ld, n, k0 + kk, i0 + ii, shift) : 0.f;
         }
         __syncthreads();
         const int rows = min(kChunk, n - i0);
         for (int ii = 0; ii < rows; ++ii) {
-            const T vc = Vc[ii][c];
+            const float vc = Vc[ii][c];
 #pragma unroll
             for (int q = 0; q < 4; ++q) acc[q] = fma(Vc[ii][g + 8 * q], vc, acc[q]);
         }
@@ -82,7 +80,7 @@ larft_kernel(const ChainDesc* __restrict__ descs, const T* __restrict__ A32, con
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) G[g + 8 * q][c] = acc[q];
-    for (int q = 0; q < 4; ++q) Ts[g + 8 * q][c] = T(0);
+    for (int q = 0; q < 4; ++q) Ts[g + 8 * q][c] = 0.f;
     __syncthreads();
     // T from its inverse, T^-1 = diag(1/tau) + triu(G, 1) (Puglisi 1992;
     // Joffrain, Low, Quintana-Orti, van de Geijn, Van Zee 2006): lane j of warp
@@ -92,55 +90,53 @@ larft_kernel(const ChainDesc* __restrict__ descs, const T* __restrict__ A32, con
     // The 32 columns are independent: one pass of 528 FMAs per lane instead
     // of 32 dependent triangular products.
     if (g == 0) {
-        const T* tp = tau + D.v_off + k0;
+        const float* tp = tau + D.v_off + k0;
         const int j = c;
-        T t[kNb];
+        float t[kNb];
 #pragma unroll
         for (int r = kNb - 1; r >= 0; --r) {
-            const T tr = r < kb ? tp[r] : T(0);
-            T s0 = T(0), s1 = T(0), s2 = T(0), s3 = T(0);
+            const float tr = r < kb ? tp[r] : 0.f;
+            float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll
             for (int q = r + 1; q < kNb; ++q) {
-                const T gq = G[r][q] * t[q];  // t_q = 0 for q > j
+                const float gq = G[r][q] * t[q];  // t_q = 0 for q > j
                 if ((q & 3) == 0) s0 += gq;
                 else if ((q & 3) == 1) s1 += gq;
                 else if ((q & 3) == 2) s2 += gq;
                 else s3 += gq;
             }
-            t[r] = r > j ? T(0) : (r == j ? tr : -tr * ((s0 + s1) + (s2 + s3)));
+            t[r] = r > j ? 0.f : (r == j ? tr : -tr * ((s0 + s1) + (s2 + s3)));
         }
 #pragma unroll
         for (int r = 0; r < kNb; ++r) Ts[r][j] = t[r];
     }
     __syncthreads();
-    T* out = Tf + (D.v_off / kNb + p) * (size_t)(kNb * kNb);
+    float* out = Tf + (D.v_off / kNb + p) * (size_t)(kNb * kNb);
     for (int q = 0; q < 4; ++q) out[(g + 8 * q) * kNb + c] = Ts[g + 8 * q][c];
-    if constexpr (sizeof(T) == 4) {
-        if (VT == nullptr) return;
-        // VT(i, kk) = sum_l V(i, l) T(l, kk), T upper triangular: l <= kk
-        T* vth = VT + D.a_off;
-        T* vtl = vth + plane;
-        T* vh = vtl + plane;
-        T* vl = vh + plane;
-        for (int i = k0 + t; i < ld; i += blockDim.x) {
-            T vrow[kNb];
+    if (VT == nullptr) return;
+    // VT(i, kk) = sum_l V(i, l) T(l, kk), T upper triangular: l <= kk
+    float* vth = VT + D.a_off;
+    float* vtl = vth + plane;
+    float* vh = vtl + plane;
+    float* vl = vh + plane;
+    for (int i = k0 + t; i < ld; i += blockDim.x) {
+        float vrow[kNb];
 #pragma unroll
-            for (int l = 0; l < kNb; ++l) vrow[l] = (l < kb) ? vref(A, ld, n, k0 + l, i, shift) : T(0);
+        for (int l = 0; l < kNb; ++l) vrow[l] = (l < kb) ? vref(A, ld, n, k0 + l, i, shift) : 0.f;
 #pragma unroll 4
-            for (int kk = 0; kk < kNb; ++kk) {
-                T s = T(0);
+        for (int kk = 0; kk < kNb; ++kk) {
+            float s = 0.f;
 #pragma unroll
-                for (int l = 0; l < kNb; ++l)
-                    if (l <= kk) s = fma(vrow[l], Ts[l][kk], s);
-                unsigned hi, lo;
-                split_tf32(s, hi, lo);
-                const size_t o = (size_t)(k0 + kk) * ld + i;
-                vth[o] = __uint_as_float(hi);
-                vtl[o] = __uint_as_float(lo);
-                split_tf32(vrow[kk], hi, lo);
-                vh[o] = __uint_as_float(hi);
-                vl[o] = __uint_as_float(lo);
-            }
+            for (int l = 0; l < kNb; ++l)
+                if (l <= kk) s = fma(vrow[l], Ts[l][kk], s);
+            unsigned hi, lo;
+            split_tf32(s, hi, lo);
+            const size_t o = (size_t)(k0 + kk) * ld + i;
+            vth[o] = __uint_as_float(hi);
+            vtl[o] = __uint_as_float(lo);
+            split_tf32(vrow[kk], hi, lo);
+            vh[o] = __uint_as_float(hi);
+            vl[o] = __uint_as_float(lo);
         }
     }
 }
@@ -369,7 +365,7 @@ cudaError_t launch_larft_vt(const ChainDesc* d_desc, int batch, int max_n, const
                             float* d_Tf, float* d_VT, long long plane, int shift, cudaStream_t st) {
     if (batch <= 0) return cudaSuccess;
     const int npanel = (max_n + kNb - 1) / kNb;
-    larft_kernel<float><<<dim3(batch, npanel), 256, 0, st>>>(d_desc, d_A32, d_tau32, d_Tf, d_VT, plane, shift);
+    larft_kernel<<<dim3(batch, npanel), 256, 0, st>>>(d_desc, d_A32, d_tau32, d_Tf, d_VT, plane, shift);
     return cudaGetLastError();
 }
 
@@ -420,18 +416,6 @@ cudaError_t launch_mixed_refine(const ChainDesc* d_desc, int batch, int max_n, i
     if ((err = cudaGetLastError()) != cudaSuccess) return err;
     stage(sctx, 3, 1);
     return cudaSuccess;
-}
-
-// FP64 compact-WY factors and back-transformation (X = Q Z with Z row-major in
-// global memory) for the plain path's eigenvectors.
-cudaError_t launch_backtransform_f64(const ChainDesc* d_desc, int batch, int max_n, const double* d_A,
-                                     const double* d_tau, double* d_Tf, double* d_Z, cudaStream_t st) {
-    if (batch <= 0) return cudaSuccess;
-    const int npanel = (max_n + kNb - 1) / kNb;
-    larft_kernel<double><<<dim3(batch, npanel), 256, 0, st>>>(d_desc, d_A, d_tau, d_Tf, nullptr, 0, 1);
-    const cudaError_t err = cudaGetLastError();
-    if (err != cudaSuccess) return err;
-    return launch_backtransform_fix(d_desc, batch, max_n, d_A, d_Tf, d_Z, st);
 }
 
 }  // namespace fkg
