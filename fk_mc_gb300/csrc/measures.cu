@@ -95,6 +95,15 @@ stiff_columns_kernel(const ChainDesc* __restrict__ descs, const StiffOps* __rest
     if (threadIdx.x == 0) tpart[(size_t)blockIdx.x * gridDim.y + blockIdx.y] = (red[0] + red[1]) + (red[2] + red[3]);
 }
 
+// 1 / x to the last bit or two: the hardware's approximation (2^-20) and one
+// third-order Householder step, r (1 + e + e^2) with e = 1 - x r
+__device__ __forceinline__ double recip(double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
 // One 32 x 32 tile (ja <= ib) of S = X^T JX, S(a, b) = x_a . (Jm x_b), and its
 // pairs a < b: V += 2 pi (f_a - f_b) (-S(a,b)^2) / (e_b - e_a) where the
 // reference's conditions hold. 256 threads, 4 outputs each. With a frequency
@@ -181,36 +190,32 @@ stiff_pairs_kernel(const ChainDesc* __restrict__ descs, const TX* __restrict__ X
         // compact the tile's terms in a fixed (row-major) order; entries that
         // are no pair of the tile were zeroed above
         __syncthreads();
-        if constexpr (sizeof(TX) == 4) {
-            // FP32 copies, in parallel: thread t takes entries 4t .. 4t+3, its
-            // output offset is the block's exclusive prefix sum of the counts
-            int cnt = 0;
+        // thread t takes entries 4t .. 4t+3, its output offset is the block's
+        // exclusive prefix sum of the counts
+        double2 x[4];
+        int cnt = 0;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) cnt += terms[4 * t + u].y != 0.0;
-            int incl = cnt;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if ((t & 31) >= o) incl += y;
-            }
-            if ((t & 31) == 31) wcnt[t >> 5] = incl;
-            __syncthreads();
-            int off = incl - cnt;
-            for (int w = 0; w < (t >> 5); ++w) off += wcnt[w];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const double2 x = terms[4 * t + u];
-                if (x.y != 0.0) termf[off++] = make_float2((float)x.x, (float)x.y);
-            }
-            if (t == blockDim.x - 1) nterm = off;
-        } else if (t == 0) {
-            int m = 0;
-            for (int e = 0; e < kMt * kMt; ++e) {
-                const double2 x = terms[e];
-                if (x.y != 0.0) terms[m++] = x;
-            }
-            nterm = m;
+        for (int u = 0; u < 4; ++u) {
+            x[u] = terms[4 * t + u];
+            cnt += x[u].y != 0.0;
         }
+        int incl = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if ((t & 31) >= o) incl += y;
+        }
+        if ((t & 31) == 31) wcnt[t >> 5] = incl;
+        __syncthreads();  // counts there; every entry is read
+        int off = incl - cnt;
+        for (int w = 0; w < (t >> 5); ++w) off += wcnt[w];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (x[u].y != 0.0) {
+                if constexpr (sizeof(TX) == 4) termf[off++] = make_float2((float)x[u].x, (float)x[u].y);
+                else terms[off++] = make_double2(x[u].x, x[u].y * x[u].x);
+            }
+        if (t == blockDim.x - 1) nterm = off;
     }
     __syncthreads();
     if (t == 0) {
@@ -247,11 +252,26 @@ stiff_pairs_kernel(const ChainDesc* __restrict__ descs, const TX* __restrict__ X
                         c += (double)cb;
                     }
                 } else {
-                    const double w = wgrid[q];
-                    for (int k = s; k < m; k += S) {
-                        const double de = terms[k].x;  // e_i - e_j > 0
-                        const double a = w - de, b = w + de;
-                        c += terms[k].y * (w * de) / (fma(a, a, eta2) * fma(b, b, eta2));
+                    // FP64 pipe (a warp's instruction every 64-76 cycles): eight operations a term and
+                    // frequency instead of about twenty with a division. Odd in w, so |w| and
+                    // (|w| + d)^2 + eta^2 = (|w| - d)^2 + eta^2 + 4 |w| d without a cancellation; the
+                    // factor w is the sum's. 32 x N = 225 with 64
+                    // frequencies: 2.70 -> 1.73 ms, with the terms packed by all threads
+                    const double w = wgrid[q], wa = fabs(w), w4 = 4.0 * wa;
+                    // terms: e_i - e_j > 0, sigma (e_i - e_j)
+                    if (wa < 1e70 && eta2 > 1e-140 && eta2 < 1e140) {  // the product is in FP64's normal range
+                        for (int k = s; k < m; k += S) {
+                            const double2 x = terms[k];
+                            const double a = wa - x.x, p = fma(a, a, eta2);
+                            c = fma(x.y, recip(p * fma(w4, x.x, p)), c);
+                        }
+                        c *= w;
+                    } else {
+                        for (int k = s; k < m; k += S) {
+                            const double2 x = terms[k];
+                            const double a = wa - x.x, b = wa + x.x;
+                            c += w * x.y / (fma(a, a, eta2) * fma(b, b, eta2));
+                        }
                     }
                 }
             }
