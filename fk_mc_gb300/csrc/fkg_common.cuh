@@ -83,6 +83,15 @@ enum : int {
 // kernels' main loops (fkg_set_wait_limit changes it per context).
 constexpr long long kDefaultWaitIters = 1ll << 24;
 
+// 1 / x to the last bit or two: the hardware's approximation (2^-20) and one
+// third-order Householder step, r (1 + e + e^2) with e = 1 - x r; |x| and 1 / |x| in the normal range
+__device__ __forceinline__ double recip64(double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
 __device__ __forceinline__ double warp_sum(double x) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);

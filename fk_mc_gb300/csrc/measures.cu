@@ -95,15 +95,6 @@ stiff_columns_kernel(const ChainDesc* __restrict__ descs, const StiffOps* __rest
     if (threadIdx.x == 0) tpart[(size_t)blockIdx.x * gridDim.y + blockIdx.y] = (red[0] + red[1]) + (red[2] + red[3]);
 }
 
-// 1 / x to the last bit or two: the hardware's approximation (2^-20) and one
-// third-order Householder step, r (1 + e + e^2) with e = 1 - x r
-__device__ __forceinline__ double recip(double x) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    const double e = fma(-x, r, 1.0);
-    return fma(r, fma(e, e, e), r);
-}
-
 // One 32 x 32 tile (ja <= ib) of S = X^T JX, S(a, b) = x_a . (Jm x_b), and its
 // pairs a < b: V += 2 pi (f_a - f_b) (-S(a,b)^2) / (e_b - e_a) where the
 // reference's conditions hold. 256 threads, 4 outputs each. With a frequency
@@ -263,7 +254,7 @@ stiff_pairs_kernel(const ChainDesc* __restrict__ descs, const TX* __restrict__ X
                         for (int k = s; k < m; k += S) {
                             const double2 x = terms[k];
                             const double a = wa - x.x, p = fma(a, a, eta2);
-                            c = fma(x.y, recip(p * fma(w4, x.x, p)), c);
+                            c = fma(x.y, recip64(p * fma(w4, x.x, p)), c);
                         }
                         c *= w;
                     } else {

@@ -19,8 +19,6 @@
 namespace fkg {
 namespace {
 
-constexpr int kThreads = 128;
-
 struct LU {
     double* r0;   // reciprocals of the diagonal of U
     double* u1;   // first superdiagonal of U
@@ -65,67 +63,194 @@ __device__ void solve(LU f, int n, double* x) {
     for (int i = n - 3; i >= 0; --i) x[i] = (x[i] - f.u1[i] * x[i + 1] - f.u2[i] * x[i + 2]) * f.r0[i];
 }
 
-__global__ void __launch_bounds__(kThreads)
+// |x| as an integer: comparisons of FP64 numbers off the FP64 pipe
+__device__ __forceinline__ long long abs_bits(double x) { return __double_as_longlong(x) & 0x7fffffffffffffffll; }
+
+// x 2^-k by its exponent field; subnormal numbers, before or after, become 0
+__device__ __forceinline__ double scale_down(double x, int k) {
+    const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
+    return e == 0 || e <= k ? 0.0 : __hiloint2double(hi - k * (1 << 20), __double2loint(x));
+}
+
+// One thread per vector, a warp per CTA: the recurrences are serial, and a warp's FP64 instruction takes 64-76
+// cycles of its scheduler whatever its latency, so what counts is their number: 29 a row for the factorisation and
+// the three solves. The start vector comes from 32 sines by angle addition, the first forward elimination runs
+// inside the factorisation, reciprocals take the hardware's approximation and one third-order step, comparisons and
+// the scaling between solves (by powers of two) are integer work. Rows are stored [i][vector] (coalesced) and read
+// four ahead.
+// Measured (one thread's rows apart, branches, divisions and sines before): 32 chains of N = 225 1.41 -> 0.45 ms,
+// 256 of N = 576 27.5 -> 8.3 ms, one of N = 64 0.31 -> 0.11 ms.
+__global__ void __launch_bounds__(32)
 stein_kernel(const ChainDesc* __restrict__ descs, const double* __restrict__ dd, const double* __restrict__ ee,
              const double* __restrict__ ww, double* __restrict__ Zws, double* __restrict__ scratch) {
-    extern __shared__ double sme[];
+    extern __shared__ double2 de[];  // d_i, e_i
+    __shared__ double2 rot[32];      // sin, cos of 0.7 i
     const ChainDesc D = descs[blockIdx.x];
-    const int n = D.n, ld = D.ld;
-    if ((int)(blockIdx.y * blockDim.x) >= n) return;
-    double* d = sme;
-    double* e = sme + ld;
-    __shared__ double red[2][kThreads / 32];
+    const int n = D.n, ld = D.ld, lane = threadIdx.x, j = blockIdx.y * 32 + lane;
+    if ((int)blockIdx.y * 32 >= n) return;
+    for (int i = lane; i < n; i += 32) de[i] = make_double2(dd[D.v_off + i], i + 1 < n ? ee[D.v_off + i] : 0.0);
+    sincos(0.7 * lane, &rot[lane].x, &rot[lane].y);
+    __syncwarp();
     double gl = DBL_MAX, gu = -DBL_MAX;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        d[i] = dd[D.v_off + i];
-        e[i] = i + 1 < n ? ee[D.v_off + i] : 0.0;
+    for (int i = lane; i < n; i += 32) {
+        const double r = (i > 0 ? fabs(de[i - 1].y) : 0.0) + fabs(de[i].y);
+        gl = fmin(gl, de[i].x - r);
+        gu = fmax(gu, de[i].x + r);
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double r = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i + 1 < n ? fabs(e[i]) : 0.0);
-        gl = fmin(gl, d[i] - r);
-        gu = fmax(gu, d[i] + r);
-    }
-    gl = warp_min(gl);
-    gu = warp_max(gu);
-    if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = gl; red[1][threadIdx.x >> 5] = gu; }
-    __syncthreads();
-    for (int q = 0; q < kThreads / 32; ++q) { gl = fmin(gl, red[0][q]); gu = fmax(gu, red[1][q]); }
-    const double tnorm = fmax(fabs(gl), fabs(gu));
+    const double tnorm = fmax(fabs(warp_min(gl)), fabs(warp_max(gu)));
     const double ortol = 1e-5 * tnorm, pivmin = DBL_EPSILON * tnorm + DBL_MIN;
-    const int j = blockIdx.y * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const double* w = ww + D.v_off;
     if (j > 0 && w[j] - w[j - 1] <= ortol) return;  // not a cluster leader
     double* Z = Zws + D.a_off;
-    // per-thread scratch: 5 ld doubles (r0, u1, u2, m, piv) + the work vector;
-    // chain c owns [6 a_off_c, 6 a_off_c + 6 ld_c^2)
-    double* base = scratch + 6 * (size_t)D.a_off + (size_t)j * 6 * ld;
-    LU f{base, base + ld, base + 2 * ld, base + 3 * ld, reinterpret_cast<int*>(base + 4 * ld)};
-    double* x = base + 5 * ld;
+    // chain c owns [6 a_off_c, 6 a_off_c + 6 ld_c^2): planes of ld x ld, this thread's column j
+    const size_t plane = (size_t)ld * ld;
+    double* const r0 = scratch + 6 * (size_t)D.a_off + j;  // reciprocals of the diagonal of U
+    double* const u1 = r0 + plane;                         // its superdiagonals
+    double* const u2 = u1 + plane;
+    double* const ml = u2 + plane;                         // multipliers of L
+    double* const yy = ml + plane;                         // forward solution
+    unsigned* const pv = reinterpret_cast<unsigned*>(yy + plane - j) + j;  // row interchanges, 32 rows a word
+    const long long pivbits = abs_bits(pivmin);
+    auto guard = [&](double x) { return abs_bits(x) < pivbits ? copysign(pivmin, x) : x; };
+    const double rs = sin(0.7 * 32), rc = cos(0.7 * 32);
     for (int jj = j; jj < n && (jj == j || w[jj] - w[jj - 1] <= ortol); ++jj) {
         // a perturbation of 2 eps ||T|| keeps identical eigenvalues of a cluster apart
         const double lam = w[jj] + (jj - j) * 2.0 * DBL_EPSILON * tnorm;
-        factor(d, e, n, lam, pivmin, f);
-        for (int i = 0; i < n; ++i) x[i] = 1.0 + 0.25 * sin(0.7 * i + 1.3 * jj);  // fixed start vector
-        for (int it = 0; it < 3; ++it) {
-            solve(f, n, x);
-            for (int q = j; q < jj; ++q) {  // orthogonalise against the cluster's earlier vectors
-                double dot = 0.0;
-                for (int i = 0; i < n; ++i) dot += Z[(size_t)i * ld + q] * x[i];
-                for (int i = 0; i < n; ++i) x[i] -= dot * Z[(size_t)i * ld + q];
+        double* const z = Z + jj;
+        // fixed start vector 1 + sin(0.7 i + 1.3 jj) / 4: ps, pc the sine and cosine at the last multiple of 32
+        double ps, pc;
+        sincos(1.3 * jj, &ps, &pc);
+        ps *= 0.25;
+        pc *= 0.25;
+        auto start = [&](int i) {
+            if ((i & 31) == 0 && i > 0) {
+                const double t = fma(ps, rc, pc * rs);
+                pc = fma(pc, rc, -ps * rs);
+                ps = t;
             }
-            double nrm = 0.0;
-            for (int i = 0; i < n; ++i) nrm += x[i] * x[i];
-            const double sc = 1.0 / sqrt(nrm);
-            for (int i = 0; i < n; ++i) x[i] *= sc;
+            const double2 q = rot[i & 31];
+            return fma(pc, q.x, fma(ps, q.y, 1.0));
+        };
+        // factorisation, with the first forward elimination
+        double cd = de[0].x - lam, cs = de[0].y, cur = start(0);  // active row: diagonal, superdiagonal, right side
+        unsigned bits = 0;
+        for (int i = 0; i + 1 < n; ++i) {
+            const double sub = de[i].y, an = de[i + 1].x - lam, en = de[i + 1].y, nx = start(i + 1);
+            const bool swap = abs_bits(cd) < abs_bits(sub);
+            const double r = recip64(guard(swap ? sub : cd)), mu = (swap ? cd : sub) * r;
+            const double a1 = swap ? an : cs, a2 = swap ? en : 0.0, y = swap ? nx : cur;
+            const size_t o = (size_t)i * ld;
+            r0[o] = r;
+            u1[o] = a1;
+            u2[o] = a2;
+            ml[o] = mu;
+            yy[o] = y;
+            bits |= (unsigned)swap << (i & 31);
+            if ((i & 31) == 31) {
+                pv[(size_t)(i >> 5) * ld] = bits;
+                bits = 0;
+            }
+            cur = fma(-mu, y, swap ? cur : nx);
+            cd = fma(-mu, a1, swap ? cs : an);
+            cs = fma(-mu, a2, swap ? 0.0 : en);
+        }
+        if ((n - 1) & 31) pv[(size_t)((n - 1) >> 5) * ld] = bits;
+        const double rl = recip64(guard(cd));
+        double nrm, sg;  // squared norm, a component with the vector's sign
+        for (int it = 0;; ++it) {
+            // back substitution
+            double x1 = cur * rl, x2 = 0.0;
+            long long best = abs_bits(x1);  // the largest component (the first of equal ones) and its sign
+            sg = x1;
+            double sq[4] = {x1 * x1, 0.0, 0.0, 0.0};  // four sums round less than one
+            z[(size_t)(n - 1) * ld] = x1;
+            double cy[4], c1[4], c2[4], cr[4];
+            auto fetch = [&](int i0) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const size_t o = (size_t)max(i0 - u, 0) * ld;
+                    cy[u] = yy[o]; c1[u] = u1[o]; c2[u] = u2[o]; cr[u] = r0[o];
+                }
+            };
+            if (n > 1) fetch(n - 2);
+            for (int i0 = n - 2; i0 >= 0; i0 -= 4) {
+                double ty[4], t1[4], t2[4], tr[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) { ty[u] = cy[u]; t1[u] = c1[u]; t2[u] = c2[u]; tr[u] = cr[u]; }
+                if (i0 >= 4) fetch(i0 - 4);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (i0 >= u) {
+                        const double x = fma(-t1[u], x1, fma(-t2[u], x2, ty[u])) * tr[u];
+                        x2 = x1;
+                        x1 = x;
+                        z[(size_t)(i0 - u) * ld] = x;
+                        const long long ab = abs_bits(x);
+                        if (ab >= best) { best = ab; sg = x; }
+                        if (it == 2) sq[u] = fma(x, x, sq[u]);
+                    }
+            }
+            nrm = (sq[0] + sq[1]) + (sq[2] + sq[3]);
+            if (jj > j) {  // orthogonalise against the cluster's earlier vectors
+                for (int q = j; q < jj; ++q) {
+                    double dot = 0.0;
+                    for (int i = 0; i < n; ++i) dot += Z[(size_t)i * ld + q] * z[(size_t)i * ld];
+                    for (int i = 0; i < n; ++i) z[(size_t)i * ld] -= dot * Z[(size_t)i * ld + q];
+                }
+                best = -1;
+                nrm = 0.0;
+                for (int i = 0; i < n; ++i) {
+                    const double x = z[(size_t)i * ld];
+                    if (abs_bits(x) > best) { best = abs_bits(x); sg = x; }
+                    nrm = fma(x, x, nrm);
+                }
+            }
+            const int k = (int)(best >> 52) - 1023;  // 1024: not a number, which stays so
+            if (it == 2) {
+                if (!(nrm > 1e-280 && nrm < 1e280) && k < 1024) {  // squares out of range: the scaled vector
+                    nrm = 0.0;
+                    for (int i = 0; i < n; ++i) {
+                        const double x = scale_down(z[(size_t)i * ld], k);
+                        z[(size_t)i * ld] = x;
+                        nrm = fma(x, x, nrm);
+                    }
+                }
+                break;
+            }
+            // scaled forward elimination
+            const double nan = k == 1024 ? (double)NAN : 0.0;
+            cur = scale_down(z[0], k) + nan;
+            double cz[4], cm[4];
+            auto fetch2 = [&](int i0) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const size_t o = (size_t)min(i0 + u, n - 2) * ld;
+                    cm[u] = ml[o];
+                    cz[u] = z[o + ld];
+                }
+            };
+            if (n > 1) fetch2(0);
+            for (int i0 = 0; i0 + 1 < n; i0 += 4) {
+                double tm[4], tz[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) { tm[u] = cm[u]; tz[u] = cz[u]; }
+                if (i0 + 5 < n) fetch2(i0 + 4);
+                if ((i0 & 31) == 0) bits = pv[(size_t)(i0 >> 5) * ld];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (i0 + u + 1 < n) {
+                        const bool swap = bits >> ((i0 + u) & 31) & 1;
+                        const double nx = scale_down(tz[u], k), y = swap ? nx : cur;
+                        yy[(size_t)(i0 + u) * ld] = y;
+                        cur = fma(-tm[u], y, swap ? cur : nx);
+                    }
+            }
         }
         // sign: largest component positive (deterministic output)
-        int imax = 0;
-        for (int i = 1; i < n; ++i)
-            if (fabs(x[i]) > fabs(x[imax])) imax = i;
-        const double sg = x[imax] < 0.0 ? -1.0 : 1.0;
-        for (int i = 0; i < n; ++i) Z[(size_t)i * ld + jj] = sg * x[i];
+        const double sc = copysign(1.0 / sqrt(nrm), sg);
+#pragma unroll 4
+        for (int i = 0; i < n; ++i) z[(size_t)i * ld] *= sc;
     }
 }
 
@@ -280,11 +405,8 @@ size_t stein_scratch_elems(long long a_total) { return (size_t)6 * a_total; }
 cudaError_t launch_stein_f64(const ChainDesc* d_desc, int batch, int max_n, int max_ld, const double* d_d,
                              const double* d_e, const double* d_w, double* d_Z, double* d_scratch, cudaStream_t st) {
     if (batch <= 0) return cudaSuccess;
-    const size_t smem = sizeof(double) * 2 * max_ld;
-    cudaError_t err = cudaFuncSetAttribute(stein_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return err;
-    stein_kernel<<<dim3(batch, (max_n + kThreads - 1) / kThreads), kThreads, smem, st>>>(d_desc, d_d, d_e, d_w, d_Z,
-                                                                                          d_scratch);
+    stein_kernel<<<dim3(batch, (max_n + 31) / 32), 32, sizeof(double2) * max_ld, st>>>(d_desc, d_d, d_e, d_w, d_Z,
+                                                                                        d_scratch);
     return cudaGetLastError();
 }
 
