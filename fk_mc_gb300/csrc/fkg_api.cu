@@ -831,7 +831,7 @@ int fkg_set_stiffness_ops(fkg_ctx* ctx, int lattice_id, int n, const int32_t* ro
 // calc_ed(true) of a batch, eigenvectors left in the solve workspace (X,
 // each column's eigenvalue, the column order); used by the measures.
 static int solve_with_vectors(fkg_ctx* ctx, int batch, const int32_t* lattice_id, const double* diag,
-                              const double* beta, const void** X, const double** eps, const int** perm) {
+                              const double* beta, void** X, const double** eps, const int** perm) {
     int rc = eigh_values(ctx, batch, lattice_id, diag, beta, nullptr, nullptr, nullptr, nullptr, true);
     if (rc) return rc;
     Workspace& ws = ctx->solve;
@@ -847,7 +847,7 @@ int fkg_measure_ipr(fkg_ctx* ctx, int batch, const int32_t* lattice_id, const do
                     double* ipr) {
     if (!ctx) return FKG_ERR_ARG;
     if (!ipr) return set_err(ctx, FKG_ERR_ARG, "ipr is NULL");
-    const void* X;
+    void* X;
     const double* eps;
     const int* perm;
     int rc = solve_with_vectors(ctx, batch, lattice_id, diag, beta, &X, &eps, &perm);
@@ -883,7 +883,7 @@ int fkg_measure_stiffness(fkg_ctx* ctx, int batch, const int32_t* lattice_id, co
         if (id < 0 || id >= kMaxLattices || ctx->lat[id].snnz < 0)
             return set_err(ctx, FKG_ERR_STATE, "stiffness operators not set for lattice " + std::to_string(id));
     }
-    const void* X;
+    void* X;
     const double* eps;
     const int* perm;
     int rc = solve_with_vectors(ctx, batch, lattice_id, diag, beta, &X, &eps, &perm);

@@ -310,8 +310,9 @@ cudaError_t launch_backtransform_tc5(const ChainDesc* d_desc, int batch, int max
 cudaError_t launch_ipr(const ChainDesc* d_desc, int batch, int max_n, bool f32, const void* d_X, const int* d_perm,
                        double* d_out, cudaStream_t st);
 size_t stiffness_scratch_bytes(int batch, int max_n, int nw);
+// the plain path's eigenvectors are overwritten (fixed-point numbers)
 cudaError_t launch_stiffness(const ChainDesc* d_desc, const StiffOps* d_ops, int batch, int max_n, bool f32,
-                             const void* d_X, const double* d_eps, const double* d_beta, void* d_JX, double2* d_ef,
+                             void* d_X, const double* d_eps, const double* d_beta, void* d_JX, double2* d_ef,
                              double* d_scratch, double* d_out, int nw, const double* d_wgrid, double eta,
                              double* d_cond, cudaStream_t st);
 // logZ of each chain; puts a chain's eigenvalues (d_w) in ascending order first where rounding left them out of it

@@ -24,13 +24,20 @@
 // forms the tile and sums its pairs' terms; per-tile partial sums are added
 // in a fixed order, so the result is reproducible.
 #include <cfloat>
+#include <type_traits>
 
-#include "fkg_common.cuh"
+#include "sytrd_cluster.cuh"
 
 namespace fkg {
 namespace {
 
 constexpr int kMt = 32;  // tile of mJ
+
+// The plain path's mJ = X^T JX on the integer pipe: two-limb fixed-point numbers
+// (sytrd_cluster.cuh, struct Fix), X in quanta 2^-57, a column of JX in quanta
+// 2^-57 of a power of two above its norm; sums are exact, in units 2^-60 of it. The
+// FP64 pipe would take 64-76 cycles for a warp's multiply-add.
+using FX = Fix<27, 8>;
 
 // ipr of the k-th eigenvector in ascending eigenvalue order (perm: storage
 // column of the k-th, or null when the columns are already sorted)
@@ -55,26 +62,30 @@ ipr_kernel(const ChainDesc* __restrict__ descs, const TX* __restrict__ Xws, cons
 }
 
 // Per storage column b: eigenvalue and Fermi factor, the kinetic expectation
-// t_b = x_b^T Tm x_b, and the column b of JX = Jm X. Per CTA: sum_b f_b t_b.
+// t_b = x_b^T Tm x_b, and the column b of JX = Jm X. Per CTA: sum_b f_b t_b over 32
+// columns, a quarter of the rows per warp (32 chains of N = 225 are 64 warps of
+// whole columns otherwise). On the plain path JX and then X, in place, become
+// fixed-point numbers.
 template <typename TX>
 __global__ void __launch_bounds__(128)
-stiff_columns_kernel(const ChainDesc* __restrict__ descs, const StiffOps* __restrict__ ops,
-                     const TX* __restrict__ Xws, const double* __restrict__ eps, const double* __restrict__ beta,
-                     TX* __restrict__ JXws, double2* __restrict__ ef, double* __restrict__ tpart) {
-    __shared__ double red[4];
+stiff_columns_kernel(const ChainDesc* __restrict__ descs, const StiffOps* __restrict__ ops, TX* __restrict__ Xws,
+                     const double* __restrict__ eps, const double* __restrict__ beta, TX* __restrict__ JXws,
+                     double2* __restrict__ ef, double* __restrict__ tpart, double* __restrict__ jscale) {
+    __shared__ double red[4][32];
+    __shared__ double red2[sizeof(TX) == 8 ? 4 : 1][32];
     const ChainDesc D = descs[blockIdx.x];
     const int* __restrict__ srow = ops[blockIdx.x].rowptr;
     const int* __restrict__ scol = ops[blockIdx.x].col;
     const double* __restrict__ tval = ops[blockIdx.x].tval;
     const double* __restrict__ jval = ops[blockIdx.x].jval;
-    const int n = D.n, ld = D.ld;
-    const int b = blockIdx.y * blockDim.x + threadIdx.x;
-    double ft = 0.0;
-    if (b < n) {
-        const TX* X = Xws + D.a_off;
-        TX* JX = JXws + D.a_off;
-        double tb = 0.0;
-        for (int i = 0; i < n; ++i) {
+    const int n = D.n, ld = D.ld, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int b = blockIdx.y * 32 + lane, i0 = n * warp / 4, i1 = n * (warp + 1) / 4;
+    TX* X = Xws + D.a_off;
+    TX* JX = JXws + D.a_off;
+    double tb = 0.0;
+    [[maybe_unused]] double n2 = 0.0;  // squared norm of the column of JX
+    if (b < n)
+        for (int i = i0; i < i1; ++i) {
             double tx = 0.0, jx = 0.0;
             for (int p = srow[i]; p < srow[i + 1]; ++p) {
                 const double xc = (double)X[(size_t)scol[p] * ld + b];
@@ -83,16 +94,36 @@ stiff_columns_kernel(const ChainDesc* __restrict__ descs, const StiffOps* __rest
             }
             tb = fma((double)X[(size_t)i * ld + b], tx, tb);
             JX[(size_t)i * ld + b] = (TX)jx;
+            if constexpr (sizeof(TX) == 8) n2 = fma(jx, jx, n2);
         }
+    red[warp][lane] = tb;
+    if constexpr (sizeof(TX) == 8) red2[warp][lane] = n2;
+    __syncthreads();  // and every row of X is read
+    if constexpr (sizeof(TX) == 8)
+        if (b < n) {
+            n2 = (red2[0][lane] + red2[1][lane]) + (red2[2][lane] + red2[3][lane]);
+            int ex = 0;
+            if (n2 > 0.0 && n2 <= DBL_MAX) frexp(sqrt(n2), &ex);  // the norm is below 2^ex
+            if (warp == 0)
+                jscale[(size_t)blockIdx.x * gridDim.y * 32 + b] = n2 <= DBL_MAX ? ldexp(1.0, ex - 60) : (double)NAN;
+            const double qj = ldexp(1.0, 57 - ex);
+#pragma unroll 4
+            for (int i = i0; i < i1; ++i) {
+                const size_t o = (size_t)i * ld + b;
+                ((int2*)X)[o] = FX::split(__double2ll_rn(X[o] * 0x1p57));
+                ((int2*)JX)[o] = FX::split(__double2ll_rn(JX[o] * qj));
+            }
+        }
+    if (warp > 0) return;
+    double ft = 0.0;
+    if (b < n) {
         const double e = eps[D.v_off + b];
         const double f = 1.0 / (1.0 + exp(beta[blockIdx.x] * e));
         ef[D.v_off + b] = make_double2(e, f);
-        ft = f * tb;
+        ft = f * ((red[0][lane] + red[1][lane]) + (red[2][lane] + red[3][lane]));
     }
     ft = warp_sum(ft);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ft;
-    __syncthreads();
-    if (threadIdx.x == 0) tpart[(size_t)blockIdx.x * gridDim.y + blockIdx.y] = (red[0] + red[1]) + (red[2] + red[3]);
+    if (lane == 0) tpart[(size_t)blockIdx.x * gridDim.y + blockIdx.y] = ft;
 }
 
 // One 32 x 32 tile (ja <= ib) of S = X^T JX, S(a, b) = x_a . (Jm x_b), and its
@@ -104,10 +135,11 @@ stiff_columns_kernel(const ChainDesc* __restrict__ descs, const StiffOps* __rest
 template <typename TX>
 __global__ void __launch_bounds__(256)
 stiff_pairs_kernel(const ChainDesc* __restrict__ descs, const TX* __restrict__ Xws, const TX* __restrict__ JXws,
-                   const double2* __restrict__ ef, int ntile, double* __restrict__ vpart, int nw,
+                   const double* __restrict__ jscale, int jstride, const double2* __restrict__ ef, int ntile, double* __restrict__ vpart, int nw,
                    const double* __restrict__ wgrid, double eta, double* __restrict__ cpart) {
-    __shared__ TX Xa[kMt][kMt + 1];
-    __shared__ TX Jb[kMt][kMt + 1];
+    using E = std::conditional_t<sizeof(TX) == 8, int2, float>;
+    __shared__ E Xa[kMt][kMt + 1];
+    __shared__ E Jb[kMt][kMt + 1];
     __shared__ double red[8];
     __shared__ double2 terms[kMt * kMt];  // (e_i - e_j, sigma) of the tile's pairs, e_i > e_j
     __shared__ double cbuf[256];          // per-slice conductivity sums (S * nw <= 256)
@@ -132,22 +164,31 @@ stiff_pairs_kernel(const ChainDesc* __restrict__ descs, const TX* __restrict__ X
         return;
     }
     if (threadIdx.x == 0) nterm = 0;
-    const TX* X = Xws + D.a_off;
-    const TX* JX = JXws + D.a_off;
+    const E* X = (const E*)(Xws + D.a_off);
+    const E* JX = (const E*)(JXws + D.a_off);
     const int t = threadIdx.x, tc = t & 31, tr = t >> 5;  // this thread: column b = ib*32 + tc, rows a = ja*32 + tr + 8u
-    TX acc[4] = {TX(0), TX(0), TX(0), TX(0)};
+    std::conditional_t<sizeof(TX) == 8, FX::Acc, float> acc[4] = {};
     for (int r0 = 0; r0 < n; r0 += kMt) {
         for (int u = tr; u < kMt; u += 8) {
             const int r = r0 + u;
-            Xa[u][tc] = (r < n && ja * kMt + tc < n) ? X[(size_t)r * ld + ja * kMt + tc] : TX(0);
-            Jb[u][tc] = (r < n && ib * kMt + tc < n) ? JX[(size_t)r * ld + ib * kMt + tc] : TX(0);
+            Xa[u][tc] = (r < n && ja * kMt + tc < n) ? X[(size_t)r * ld + ja * kMt + tc] : E{};
+            Jb[u][tc] = (r < n && ib * kMt + tc < n) ? JX[(size_t)r * ld + ib * kMt + tc] : E{};
         }
         __syncthreads();
-#pragma unroll 8
-        for (int u = 0; u < kMt; ++u) {
-            const TX jb = Jb[u][tc];
+        if constexpr (sizeof(TX) == 8) {
+#pragma unroll 4
+            for (int u = 0; u < kMt; u += 2) {
+                const int2 jb0 = Jb[u][tc], jb1 = Jb[u + 1][tc];
 #pragma unroll
-            for (int v = 0; v < 4; ++v) acc[v] = fma(Xa[u][tr + 8 * v], jb, acc[v]);
+                for (int v = 0; v < 4; ++v) FX::mac2(acc[v], Xa[u][tr + 8 * v], jb0, Xa[u + 1][tr + 8 * v], jb1);
+            }
+        } else {
+#pragma unroll 8
+            for (int u = 0; u < kMt; ++u) {
+                const float jb = Jb[u][tc];
+#pragma unroll
+                for (int v = 0; v < 4; ++v) acc[v] = fma(Xa[u][tr + 8 * v], jb, acc[v]);
+            }
         }
         __syncthreads();
     }
@@ -158,6 +199,7 @@ stiff_pairs_kernel(const ChainDesc* __restrict__ descs, const TX* __restrict__ X
         for (int v = 0; v < 4; ++v) terms[(tr + 8 * v) * kMt + tc] = make_double2(0.0, 0.0);
     if (bcol < n) {
         const double2 efb = ef[D.v_off + bcol];
+        [[maybe_unused]] const double js = sizeof(TX) == 8 ? jscale[(size_t)blockIdx.y * jstride + bcol] : 1.0;
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
             const int a = ja * kMt + tr + 8 * v;
@@ -165,7 +207,9 @@ stiff_pairs_kernel(const ChainDesc* __restrict__ descs, const TX* __restrict__ X
             if (a >= n || (ja == ib && a >= bcol)) continue;
             const double2 efa = ef[D.v_off + a];
             if (!(fabs(efb.x - efa.x) > 1e-12)) continue;
-            const double s = (double)acc[v];
+            double s;
+            if constexpr (sizeof(TX) == 8) s = (double)FX::sum(acc[v]) * js;
+            else s = (double)acc[v];
             const double sigma = M_PI * (efa.y - efb.y) * (-s * s);
             if (fabs(sigma) > 1e-13) {
                 vsum += 2.0 * sigma / (efb.x - efa.x);
@@ -248,6 +292,7 @@ stiff_pairs_kernel(const ChainDesc* __restrict__ descs, const TX* __restrict__ X
                     // (|w| + d)^2 + eta^2 = (|w| - d)^2 + eta^2 + 4 |w| d without a cancellation; the
                     // factor w is the sum's. 32 x N = 225 with 64
                     // frequencies: 2.70 -> 1.73 ms, with the terms packed by all threads
+                    // (1.01 with the fixed-point mJ)
                     const double w = wgrid[q], wa = fabs(w), w4 = 4.0 * wa;
                     // terms: e_i - e_j > 0, sigma (e_i - e_j)
                     if (wa < 1e70 && eta2 > 1e-140 && eta2 < 1e140) {  // the product is in FP64's normal range
@@ -316,31 +361,33 @@ cudaError_t launch_ipr(const ChainDesc* d_desc, int batch, int max_n, bool f32, 
 }
 
 size_t stiffness_scratch_bytes(int batch, int max_n, int nw) {
-    const int ntb = (max_n + 127) / 128, nb = (max_n + kMt - 1) / kMt, ntile = nb * (nb + 1) / 2;
-    return sizeof(double) * (size_t)batch * (ntb + (size_t)ntile * (1 + nw));
+    const int nb = (max_n + kMt - 1) / kMt, ntile = nb * (nb + 1) / 2;
+    return sizeof(double) * (size_t)batch * (33 * nb + (size_t)ntile * (1 + nw));
 }
 
 cudaError_t launch_stiffness(const ChainDesc* d_desc, const StiffOps* d_ops, int batch, int max_n, bool f32,
-                             const void* d_X, const double* d_eps, const double* d_beta, void* d_JX, double2* d_ef,
+                             void* d_X, const double* d_eps, const double* d_beta, void* d_JX, double2* d_ef,
                              double* d_scratch, double* d_out, int nw, const double* d_wgrid, double eta,
                              double* d_cond, cudaStream_t st) {
     if (batch <= 0) return cudaSuccess;
     if (batch > 65535) return cudaErrorInvalidValue;  // grid y limit of the pair kernel
-    const int ntb = (max_n + 127) / 128, nb = (max_n + kMt - 1) / kMt, ntile = nb * (nb + 1) / 2;
-    double* tpart = d_scratch;
-    double* vpart = d_scratch + (size_t)batch * ntb;
+    const int nb = (max_n + kMt - 1) / kMt, ntb = nb, ntile = nb * (nb + 1) / 2;
+    double* jscale = d_scratch;
+    double* tpart = jscale + (size_t)batch * 32 * nb;
+    double* vpart = tpart + (size_t)batch * ntb;
     double* cpart = nw > 0 ? vpart + (size_t)batch * ntile : nullptr;
     if (f32) {
-        stiff_columns_kernel<float><<<dim3(batch, ntb), 128, 0, st>>>(d_desc, d_ops, (const float*)d_X, d_eps, d_beta,
-                                                                      (float*)d_JX, d_ef, tpart);
+        stiff_columns_kernel<float><<<dim3(batch, ntb), 128, 0, st>>>(d_desc, d_ops, (float*)d_X, d_eps, d_beta,
+                                                                      (float*)d_JX, d_ef, tpart, jscale);
         stiff_pairs_kernel<float><<<dim3(ntile, batch), 256, 0, st>>>(d_desc, (const float*)d_X, (const float*)d_JX,
-                                                                      d_ef, ntile, vpart, nw, d_wgrid, eta, cpart);
+                                                                      jscale, 32 * nb, d_ef, ntile, vpart, nw, d_wgrid,
+                                                                      eta, cpart);
     } else {
-        stiff_columns_kernel<double><<<dim3(batch, ntb), 128, 0, st>>>(d_desc, d_ops, (const double*)d_X, d_eps,
-                                                                       d_beta, (double*)d_JX, d_ef, tpart);
+        stiff_columns_kernel<double><<<dim3(batch, ntb), 128, 0, st>>>(d_desc, d_ops, (double*)d_X, d_eps, d_beta,
+                                                                       (double*)d_JX, d_ef, tpart, jscale);
         stiff_pairs_kernel<double><<<dim3(ntile, batch), 256, 0, st>>>(d_desc, (const double*)d_X,
-                                                                       (const double*)d_JX, d_ef, ntile, vpart, nw,
-                                                                       d_wgrid, eta, cpart);
+                                                                       (const double*)d_JX, jscale, 32 * nb, d_ef, ntile,
+                                                                       vpart, nw, d_wgrid, eta, cpart);
     }
     stiff_final_kernel<<<(batch + 127) / 128, 128, 0, st>>>(d_desc, batch, tpart, ntb, vpart, ntile, d_out);
     if (nw > 0) cond_final_kernel<<<(batch * nw + 127) / 128, 128, 0, st>>>(batch, ntile, nw, cpart, d_cond);
