@@ -216,6 +216,18 @@ struct Fix {
     }
 };
 
+// the NB entries of one row of Vp or Wp, in 16-byte loads
+template <int NB, typename V>
+__device__ __forceinline__ void ld_row(const V* p, V (&r)[NB]) {
+    constexpr int kPer = 16 / sizeof(V);
+    static_assert(NB % kPer == 0, "rows of whole 16-byte units");
+#pragma unroll
+    for (int q = 0; q < NB / kPer; ++q) {
+        const int4 x = ((const int4*)p)[q];
+        memcpy(&r[q * kPer], &x, 16);
+    }
+}
+
 // offset of entry (r, c) of a tile (lane-owned 16-byte units)
 __device__ __forceinline__ int elem_off(int r, int c) {
     const int q = ((r >> 4) & 1) * 4 + (c >> 3), lane = (r & 7) * 4 + ((c & 7) >> 1);
@@ -470,19 +482,22 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                     const int id0 = (nt - 1 - J) * (nt - J) / 2;
                     const int o = (rank - id0) & cm;
                     V vk[NB], wk[NB];
-#pragma unroll
-                    for (int l = 0; l < NB; ++l) { vk[l] = Vp[k * NB + l]; wk[l] = Wp[k * NB + l]; }
+                    ld_row<NB>(Vp + k * NB, vk);
+                    ld_row<NB>(Wp + k * NB, wk);
 #pragma unroll 1
                     for (int I = J + o + C * warp; I < nt; I += C * kWarps) {
                         const unsigned char* t = tile((id0 + I - J) >> lc);
                         const int i = I * kTile + lane;
                         Acc u;
                         P::zero(u);
+                        if (j > 0) {
+                            V vr[NB], wr[NB];
+                            ld_row<NB>(Vp + i * NB, vr);
+                            ld_row<NB>(Wp + i * NB, wr);
 #pragma unroll
-                        for (int l = 0; l < NB; ++l)
-                            if (l < j) {
-                                P::mac2(u, Vp[i * NB + l], wk[l], Wp[i * NB + l], vk[l]);
-                            }
+                            for (int l = 0; l < NB; ++l)
+                                if (l < j) P::mac2(u, vr[l], wk[l], wr[l], vk[l]);
+                        }
                         const V a = P::get(t, elem_off(lane, kc));
                         S x;
                         if constexpr (kFix) x = P::upd_ll(a, u);
@@ -665,11 +680,14 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                     for (int I = I0 + o + C * (kWarps - 1 - warp); I < nt; I += C * kWarps) {
                         const int i = I * kTile + lane;
                         const V vi = vv[i];
+                        V vr[NB], wr[NB];
+                        ld_row<NB>(Vp + i * NB, vr);
+                        ld_row<NB>(Wp + i * NB, wr);
 #pragma unroll
                         for (int l = 0; l < NB; ++l)
                             if (l < j) {
-                                P::mac(cacc[l], Wp[i * NB + l], vi);
-                                P::mac(cacc[NB + l], Vp[i * NB + l], vi);
+                                P::mac(cacc[l], wr[l], vi);
+                                P::mac(cacc[NB + l], vr[l], vi);
                             }
                     }
                     S x[2 * NB];
@@ -771,11 +789,14 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                             for (int r = 1; r < C; ++r) q = add_mod(q, pex[r * max_ld + i]);
                             Acc u;
                             P::zero(u);
+                            if (j > 0) {
+                                V vr[NB], wr[NB];
+                                ld_row<NB>(Vp + i * NB, vr);
+                                ld_row<NB>(Wp + i * NB, wr);
 #pragma unroll
-                            for (int l = 0; l < NB; ++l)
-                                if (l < j) {
-                                    P::mac2(u, Vp[i * NB + l], c1[l], Wp[i * NB + l], c2[l]);
-                                }
+                                for (int l = 0; l < NB; ++l)
+                                    if (l < j) P::mac2(u, vr[l], c1[l], wr[l], c2[l]);
+                            }
                             if constexpr (kFix) {
                                 q -= P::sum(u) << 2;  // 2^-58 S -> 2^-60 S
                                 Acc kv;
@@ -802,35 +823,34 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                 const int I0 = (k0 + nbk) >> 5, ntr = nt - I0, total = ntr * (ntr + 1) / 2;
                 const int active = (total - rank + cm) >> lc;
 #pragma unroll 1
-                for (int unit = warp; unit < 4 * active; unit += kWarps) {  // 8 columns of a tile
-                    const int ij = tab[unit >> 2], I = ij >> 8, Jt = ij & 255, q = unit & 3;
-                    void* t = tile(unit >> 2);
-                    const V* vi = Vp + (I * kTile + g) * NB;
-                    const V* wi = Wp + (I * kTile + g) * NB;
-                    const V* vj = Vp + (Jt * kTile + 8 * q + 2 * t4) * NB;
-                    const V* wj = Wp + (Jt * kTile + 8 * q + 2 * t4) * NB;
-                    Acc u[4][2];
+                for (int unit = warp; unit < 2 * active; unit += kWarps) {  // 16 rows of a tile
+                    const int ij = tab[unit >> 1], I = ij >> 8, Jt = ij & 255, mt = unit & 1;
+                    void* t = tile(unit >> 1);
+                    V a[4][4], vr[2][NB], wr[2][NB];
 #pragma unroll
-                    for (int m = 0; m < 4; ++m)
+                    for (int q = 0; q < 4; ++q) P::ld4(t, mt * 4 + q, lane, a[q]);
 #pragma unroll
-                        for (int c = 0; c < 2; ++c) P::zero(u[m][c]);
-#pragma unroll
-                    for (int l = 0; l < NB; ++l) {
-                        const V cv0 = vj[l], cw0 = wj[l], cv1 = vj[NB + l], cw1 = wj[NB + l];
-#pragma unroll
-                        for (int m = 0; m < 4; ++m) {
-                            const V rv = vi[8 * m * NB + l], rw = wi[8 * m * NB + l];
-                            P::mac2(u[m][0], rv, cw0, rw, cv0);
-                            P::mac2(u[m][1], rv, cw1, rw, cv1);
-                        }
+                    for (int h = 0; h < 2; ++h) {
+                        ld_row<NB>(Vp + (I * kTile + 16 * mt + 8 * h + g) * NB, vr[h]);
+                        ld_row<NB>(Wp + (I * kTile + 16 * mt + 8 * h + g) * NB, wr[h]);
                     }
 #pragma unroll
-                    for (int mt = 0; mt < 2; ++mt) {
-                        V a[4];
-                        P::ld4(t, mt * 4 + q, lane, a);
+                    for (int q = 0; q < 4; ++q) {
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) a[e] = P::upd(a[e], u[2 * mt + (e >> 1)][e & 1]);
-                        P::st4(t, mt * 4 + q, lane, a);
+                        for (int c = 0; c < 2; ++c) {
+                            V cv[NB], cw[NB];
+                            ld_row<NB>(Vp + (Jt * kTile + 8 * q + 2 * t4 + c) * NB, cv);
+                            ld_row<NB>(Wp + (Jt * kTile + 8 * q + 2 * t4 + c) * NB, cw);
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                Acc u;
+                                P::zero(u);
+#pragma unroll
+                                for (int l = 0; l < NB; ++l) P::mac2(u, vr[h][l], cw[l], wr[h][l], cv[l]);
+                                a[q][2 * h + c] = P::upd(a[q][2 * h + c], u);
+                            }
+                        }
+                        P::st4(t, mt * 4 + q, lane, a[q]);
                     }
                 }
             }
