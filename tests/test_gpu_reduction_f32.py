@@ -55,3 +55,22 @@ def test_orders_around_tiles(solver, n):
                                  (700, 60), (1000, 2), (1024, 17), (800, 100)])
 def test_cluster_sizes_and_warp_counts(solver, n, B):
     _run(solver, n, B, n + B)
+
+
+@pytest.mark.parametrize("sizes,variant", [((31, 32), 3), ((32, 12), 1)])
+def test_vector_solves_above_960(cuda_ok, fkg_lib, sizes, variant):
+    """Solves whose FP32 eigenvectors leave the library: with the shipped table they are, bit for bit, the two-stage
+    reduction's where every chain is above 960, and the width-8 one-stage reduction's in a batch of other orders."""
+    import fk_mc_gb300
+    res = []
+    for explicit in (False, True):
+        s = fk_mc_gb300.Solver(max_n=1024, max_batch=2, precision="mixed")
+        if explicit:
+            for n_max in (192, 1024):
+                s.set_tuning("mixed", n_max, variant)
+        f = np.concatenate([np.random.default_rng(L).integers(0, 2, s.set_lattice(i, "cubic2d", L))
+                            for i, L in enumerate(sizes)])
+        res.append(s.free_energy_grad(np.arange(2, dtype=np.int32), f, 2.0, 1.0, 1.0, 4.0))
+        s.close()
+    for k in ("F", "dU", "dt", "dmu", "dbeta"):
+        assert np.array_equal(res[0][k], res[1][k]), k
