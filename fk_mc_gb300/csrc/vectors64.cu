@@ -340,8 +340,15 @@ cluster_fix_kernel(const ChainDesc* __restrict__ descs, const double* __restrict
             // a perturbation of 2 eps ||T|| per rank keeps identical eigenvalues apart
             const double lam = w[jj] + sr[tid] * 2.0 * DBL_EPSILON * tnorm;
             factor(d, e, n, lam, pivmin, f);
-            for (int i = 0; i < n; ++i) x[i] = 1.0 + 0.25 * sin(0.7 * i + 1.3 * jj);  // fixed start vector
         }
+        // fixed start vectors, by the warps that factor nothing (nslots <= ld / 6 leaves some): a sine costs
+        // as much as a row's division, and a member's thread would evaluate n of them in turn
+        const int nf = (nslots + 31) / 32 * 32;
+        for (int q = tid - nf; q >= 0 && q < nslots * n; q += kCfThreads - nf) {
+            const int g = q / n, i = q - g * n, jj = sj[g];
+            base0[(size_t)g * 6 * ld + 5 * ld + i] = 1.0 + 0.25 * sin(0.7 * i + 1.3 * jj);
+        }
+        __syncthreads();
         for (int it = 0; it < 3; ++it) {
             if (tid < nslots) solve(f, n, x);
             __syncthreads();
