@@ -27,17 +27,21 @@ struct LU {
     int* piv;     // 1 where rows i and i+1 were interchanged
 };
 
+// |x| as an integer: comparisons of FP64 numbers off the FP64 pipe
+__device__ __forceinline__ long long abs_bits(double x) { return __double_as_longlong(x) & 0x7fffffffffffffffll; }
+
 // The pivots are kept as reciprocals: one FP64 division per elimination step
 // serves the multiplier and the three back substitutions, which then only
 // multiply (a division is a long dependent sequence on the FP64 pipe; the
 // solves are chains of n dependent steps). A pivot below pivmin is replaced by
 // +-pivmin before its reciprocal is taken.
 __device__ void factor(const double* d, const double* e, int n, double lam, double pivmin, LU f) {
-    auto guard = [&](double x) { return fabs(x) < pivmin ? (x < 0.0 ? -pivmin : pivmin) : x; };
+    const long long pivbits = abs_bits(pivmin);
+    auto guard = [&](double x) { return abs_bits(x) < pivbits ? (x < 0.0 ? -pivmin : pivmin) : x; };
     double cd = d[0] - lam, cs = n > 1 ? e[0] : 0.0;  // active row: diagonal and superdiagonal
     for (int i = 0; i + 1 < n; ++i) {
         const double sub = e[i], an = d[i + 1] - lam, en = i + 2 < n ? e[i + 1] : 0.0;
-        if (fabs(cd) >= fabs(sub)) {
+        if (abs_bits(cd) >= abs_bits(sub)) {
             const double r = 1.0 / guard(cd), mu = sub * r;
             f.r0[i] = r; f.u1[i] = cs; f.u2[i] = 0.0; f.m[i] = mu; f.piv[i] = 0;
             cd = an - mu * cs;
@@ -52,19 +56,70 @@ __device__ void factor(const double* d, const double* e, int n, double lam, doub
     f.r0[n - 1] = 1.0 / guard(cd);
 }
 
-// x <- (P L U)^{-1} x, in place
+// x <- (P L U)^{-1} x, in place. The recurrences run in registers, with the rows
+// of the next four steps loaded ahead.
 __device__ void solve(LU f, int n, double* x) {
-    for (int i = 0; i + 1 < n; ++i) {
-        if (f.piv[i]) { const double t = x[i]; x[i] = x[i + 1]; x[i + 1] = t; }
-        x[i + 1] -= f.m[i] * x[i];
+    double cur = x[0];
+    if (n > 1) {
+        double nm[4], nx[4];
+        int np[4];
+        auto fetch = [&](int i0) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = min(i0 + u, n - 2);
+                nm[u] = f.m[i]; np[u] = f.piv[i]; nx[u] = x[i + 1];
+            }
+        };
+        fetch(0);
+        for (int i0 = 0; i0 + 1 < n; i0 += 4) {
+            double tm[4], tx[4];
+            int tp[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) { tm[u] = nm[u]; tp[u] = np[u]; tx[u] = nx[u]; }
+            if (i0 + 5 < n) fetch(i0 + 4);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (i0 + u + 1 < n) {
+                    const double y = tp[u] ? tx[u] : cur, z = tp[u] ? cur : tx[u];
+                    x[i0 + u] = y;
+                    cur = z - tm[u] * y;
+                }
+        }
     }
-    x[n - 1] *= f.r0[n - 1];
-    if (n >= 2) x[n - 2] = (x[n - 2] - f.u1[n - 2] * x[n - 1]) * f.r0[n - 2];
-    for (int i = n - 3; i >= 0; --i) x[i] = (x[i] - f.u1[i] * x[i + 1] - f.u2[i] * x[i + 2]) * f.r0[i];
+    double x1 = cur * f.r0[n - 1], x2 = 0.0;
+    x[n - 1] = x1;
+    if (n < 2) return;
+    {
+        const double t = (x[n - 2] - f.u1[n - 2] * x1) * f.r0[n - 2];
+        x2 = x1;
+        x1 = t;
+        x[n - 2] = t;
+    }
+    if (n < 3) return;
+    double c0[4], c1[4], c2[4], cr[4];
+    auto fetch = [&](int i0) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = max(i0 - u, 0);
+            c0[u] = x[i]; c1[u] = f.u1[i]; c2[u] = f.u2[i]; cr[u] = f.r0[i];
+        }
+    };
+    fetch(n - 3);
+    for (int i0 = n - 3; i0 >= 0; i0 -= 4) {
+        double t0[4], t1[4], t2[4], tr[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) { t0[u] = c0[u]; t1[u] = c1[u]; t2[u] = c2[u]; tr[u] = cr[u]; }
+        if (i0 >= 4) fetch(i0 - 4);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (i0 >= u) {
+                const double t = (t0[u] - t1[u] * x1 - t2[u] * x2) * tr[u];
+                x2 = x1;
+                x1 = t;
+                x[i0 - u] = t;
+            }
+    }
 }
-
-// |x| as an integer: comparisons of FP64 numbers off the FP64 pipe
-__device__ __forceinline__ long long abs_bits(double x) { return __double_as_longlong(x) & 0x7fffffffffffffffll; }
 
 // x 2^-k by its exponent field; subnormal numbers, before or after, become 0
 __device__ __forceinline__ double scale_down(double x, int k) {
@@ -292,9 +347,16 @@ cluster_fix_kernel(const ChainDesc* __restrict__ descs, const double* __restrict
     // exactly these members)
     const double ortol = ctol[blockIdx.x], tnorm = ortol / kClusterTol;
     const double pivmin = DBL_EPSILON * tnorm + DBL_MIN;
+    __shared__ unsigned close[32];  // bit i: member i belongs to the cluster of i - 1
     int any = 0;
-    for (int i = tid + 1; i < n; i += blockDim.x) any |= (w[i] - w[i - 1] <= ortol);
+    for (int i = tid; i < (n + 31) / 32 * 32; i += blockDim.x) {
+        const bool c = i > 0 && i < n && w[i] - w[i - 1] <= ortol;
+        const unsigned b = __ballot_sync(0xffffffffu, c);
+        if (lane == 0) close[i >> 5] = b;
+        any |= c;
+    }
     if (!__syncthreads_or(any)) return;
+    auto joined = [&](int i) { return close[i >> 5] >> (i & 31) & 1; };
     float* Z = Zws + D.a_off;
     double* base0 = scratch + D.a_off;  // ld * ld doubles of this chain
     const int cap = min(kCfThreads, ld / 6);
@@ -309,7 +371,7 @@ cluster_fix_kernel(const ChainDesc* __restrict__ descs, const double* __restrict
             while (pos < n && g < cap) {
                 if (pos >= cend) {  // at a cluster boundary: find the next cluster
                     int end = pos + 1;
-                    while (end < n && w[end] - w[end - 1] <= ortol) ++end;
+                    while (end < n && joined(end)) ++end;
                     if (end - pos < 2) { pos = end; continue; }
                     cstart = pos;
                     cend = end;
