@@ -59,7 +59,7 @@ METRIC = "MC proposals/s at N=576: mixed+batched vs plain FP64 on GB300; dF erro
 NOMINAL_TFLOPS = {"fp32_fma": 152 * 128 * 2 * 2.07e9 / 1e12, "fp64": 1.25, "tf32_dense": 1100.0}
 W_FWD = 4.0 / 3.0 * N ** 3      # Householder tridiagonalisation flops per proposal
 W_BT = 2.0 * N ** 3              # back-transformation X = Q Z flops per proposal
-NB32 = 8                         # panel width of the FP32 reduction at N = 576 (tuning table)
+NB32 = 4                         # panel width of the FP32 reduction at N = 576
 # Compulsory matrix bytes of one FP32 reduction: the lower triangle of the
 # m x m trailing matrix read by the matrix-vector product of every column, and
 # read + written by the rank-2k update after every panel of NB32 columns.
@@ -198,7 +198,7 @@ def roofline(res, head, B):
             "traffic": traffic_per_launch(f"sytrd_{'f32' if f32 else 'f64'}_B{B}"),
             "traffic_source": "ncu capture committed under profiles/ (dram__bytes_read.sum + dram__bytes_write.sum "
                               "per launch), not measured by this run",
-            "kernel": "sytrd_v3<%s> (Householder reduction, one CTA per chain)" % ("float,8" if f32 else "double,4"),
+            "kernel": "sytrd_cluster<%s> (Householder reduction, a CTA or cluster per chain)" % ("F32" if f32 else "Fix"),
             "flops_per_unit": W_FWD, "units_per_launch": B, "launch_ms": red_s * 1e3 if red_s else None,
             "peak_source": f"MEASURED_PEAKS.json bf16_tflops_sustained (of {pk['of']})"}
     other = []
@@ -216,8 +216,8 @@ def roofline(res, head, B):
         m, n = res["f64"]["stages"]["reduce"]
         if n:
             a64 = W_FWD * B / (m / n * 1e-3) / 1e12
-            other.append({"kernel": "sytrd_v3<double,4> (plain FP64 path)", "view": "against the nominal FP64 "
-                          "pipe rate (not measured)", "achieved": a64, "peak": NOMINAL_TFLOPS["fp64"],
+            other.append({"kernel": "sytrd_cluster<Fix> (plain FP64 path, fixed point on the integer pipes)",
+                          "view": "against the nominal FP64 pipe rate (not measured)", "achieved": a64, "peak": NOMINAL_TFLOPS["fp64"],
                           "unit": "TFLOP/s", "frac": a64 / NOMINAL_TFLOPS["fp64"], "launch_ms": m / n})
     bt_ms, bt_n = hr["stages"].get("back", (0.0, 0))
     if bt_n:

@@ -134,7 +134,7 @@ __device__ __forceinline__ double scale_down(double x, int k) {
 // the scaling between solves (by powers of two) are integer work. Rows are stored [i][vector] (coalesced) and read
 // four ahead.
 // Measured (one thread's rows apart, branches, divisions and sines before): 32 chains of N = 225 1.41 -> 0.45 ms,
-// 256 of N = 576 27.5 -> 8.3 ms, one of N = 64 0.31 -> 0.11 ms.
+// 256 of N = 576 27.6 -> 6.5 ms, one of N = 64 0.31 -> 0.11 ms.
 __global__ void __launch_bounds__(32)
 stein_kernel(const ChainDesc* __restrict__ descs, const double* __restrict__ dd, const double* __restrict__ ee,
              const double* __restrict__ ww, double* __restrict__ Zws, double* __restrict__ scratch) {

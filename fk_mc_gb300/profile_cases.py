@@ -2,11 +2,12 @@
 
     python -m fk_mc_gb300.profile_cases all [B]        every kernel family once, cubic2d L=24 (N=576), B chains
     python -m fk_mc_gb300.profile_cases reduce [B] [V] one mixed-path solve of B chains (two warm-up solves first)
-                                                       with reduction variant V (0..2 panel widths, 3 two-stage)
+                                                       with reduction variant V (0..2 one-stage, 3 two-stage)
 
 `all` runs, in order: the plain FP64 solve with eigenvectors (reduction,
-tridiagonal eigenvalues, inverse iteration, compact-WY factors,
-back-transformation), the mixed-precision solve with eigenvectors, the
+tridiagonal eigenvalues, inverse iteration, reflectors in fixed point,
+back-transformation), its stiffness measure, the mixed-precision solve with
+eigenvectors, a values-only one, the
 stiffness measure with a 64-point conductivity grid, the IPR measure, the
 free-energy gradients with the full dF/dH, two proposal steps of
 device-resident chains (the step graph, logZ fused with the decision), and the
@@ -35,8 +36,10 @@ def run_all(B=16):
     s, rng, f, diag, ids = _setup(B, "f64")
     s.set_stiffness_ops(0, "cubic2d", L, 1.0)
     s.eigh_logz(ids, diag, 4.0, vectors=True)
+    s.measure_stiffness(ids, diag, 4.0, np.linspace(-4, 4, 64), 0.05)
     s.set_precision("mixed")
     s.eigh_logz(ids, diag, 4.0, vectors=True)
+    s.eigh_logz(ids, diag, 4.0)
     s.measure_stiffness(ids, diag, 4.0, np.linspace(-4, 4, 64), 0.05)
     s.measure_ipr(ids, diag, 4.0)
     s.free_energy_grad(ids, f.ravel(), 2.0, 1.0, 1.0, 4.0, rho=True)
