@@ -330,7 +330,13 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
     __shared__ FixRefl s_refl;
     cg::cluster_group cl = cg::this_cluster();
     const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-    const int lc = 31 - __clz(C), cm = C - 1;  // C is a power of two
+    const int inv_c = 65536 / C + 1;  // exact quotients by C below 8192
+    auto div_c = [&](int x) { return x * inv_c >> 16; };
+    auto mod_c = [&](int x) { return x - div_c(x) * C; };
+    auto first_of = [&](int x) {  // distance from item x to the next one that belongs to this CTA
+        const int o = rank - mod_c(x);
+        return o < 0 ? o + C : o;
+    };
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
     const Smem L = smem_layout<P, NB>(max_ld, C, max_slots);
     V* Vp = (V*)(sm + L.vp);  // [ld][NB]
@@ -351,7 +357,7 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
     };
     auto at = [&](auto* p, int r) { return C > 1 ? cl.map_shared_rank(p, r) : p; };
 
-    for (int item = blockIdx.x >> lc;;) {
+    for (int item = blockIdx.x / C;;) {
         if (order) {
             __syncthreads();
             if (rank == 0 && tid == 0) {
@@ -368,7 +374,7 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
         typename P::G* __restrict__ A = Aout + D.a_off;
         unsigned char* gt = (unsigned char*)spill + (size_t)D.a_off * sizeof(V);
         const int ntiles = nt * (nt + 1) / 2;
-        const int nslots = (ntiles - rank + cm) >> lc;
+        const int nslots = div_c(ntiles - rank + C - 1);
         auto tile = [&](int slot) -> unsigned char* {
             return slot < cap ? sm + L.tiles + (size_t)slot * kTileBytes : gt + (size_t)(slot * C + rank) * kTileBytes;
         };
@@ -443,7 +449,7 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
         __syncthreads();
         auto owner_slot = [&](int I, int J) {  // slot of tile (I, J) if this CTA owns it, else -1
             const int id = (nt - 1 - J) * (nt - J) / 2 + I - J;
-            return (id & cm) == rank ? id >> lc : -1;
+            return mod_c(id) == rank ? div_c(id) : -1;
         };
         auto add_elem = [&](int i, int j, double a) {
             const int I = i >> 5, J = j >> 5, slot = owner_slot(I, J);
@@ -471,6 +477,9 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
         }
         csync();  // no CTA writes into another one that is still building
 
+        // of tile column J: this CTA's first tile row (from J) and its slot; of the live tiles from row I0: their number
+        // and the first row. They change every 32 columns.
+        int at_J = -1, first_J = 0, slot_J = 0, at_I0 = -1, active = 0, first_I0 = 0;
 #pragma unroll 1
         for (int k0 = 0; k0 < n - 2; k0 += NB) {
             const int nbk = min(NB, n - 2 - k0);
@@ -479,14 +488,19 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                 const int k = k0 + j, s = k + 1, J = k >> 5, kc = k & 31;
                 // ---- (1) column k with the panel's pending updates, to every CTA ----
                 {
-                    const int id0 = (nt - 1 - J) * (nt - J) / 2;
-                    const int o = (rank - id0) & cm;
+                    if (J != at_J) {
+                        const int id0 = (nt - 1 - J) * (nt - J) / 2;
+                        at_J = J;
+                        first_J = J + first_of(id0);
+                        slot_J = div_c(id0 + first_J - J);
+                    }
+                    int slot = slot_J + warp;
                     V vk[NB], wk[NB];
                     ld_row<NB>(Vp + k * NB, vk);
                     ld_row<NB>(Wp + k * NB, wk);
 #pragma unroll 1
-                    for (int I = J + o + C * warp; I < nt; I += C * kWarps) {
-                        const unsigned char* t = tile((id0 + I - J) >> lc);
+                    for (int I = first_J + C * warp; I < nt; I += C * kWarps, slot += kWarps) {
+                        const unsigned char* t = tile(slot);
                         const int i = I * kTile + lane;
                         Acc u;
                         P::zero(u);
@@ -585,9 +599,9 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                     vv[i] = vi;
                     Vp[i * NB + j] = vi;
                     if (flat) Wp[i * NB + j] = P::vzero();
-                    if (i > s && i < n && ((i >> 5) & cm) == rank) {
+                    if ((!kFix || Aout) && i > s && i < n && mod_c(i >> 5) == rank) {
                         if constexpr (kFix) {
-                            if (Aout) A[(size_t)k * ld + i] = (double)P::join(vi) * (1.0 / (1ll << (30 + P::kLo)));
+                            A[(size_t)k * ld + i] = (double)P::join(vi) * (1.0 / (1ll << (30 + P::kLo)));
                         } else {
                             A[(size_t)k * ld + i] = vi;
                         }
@@ -600,9 +614,13 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                 __syncthreads();
                 // ---- (3a) partial p = A22 v over this CTA's tiles (stale trailing matrix) ----
                 const int I0 = s >> 5;
+                if (I0 != at_I0) {
+                    const int ntr = nt - I0;
+                    at_I0 = I0;
+                    active = div_c(ntr * (ntr + 1) / 2 - rank + C - 1);
+                    first_I0 = I0 + first_of(I0);
+                }
                 {
-                    const int ntr = nt - I0, total = ntr * (ntr + 1) / 2;
-                    const int active = (total - rank + cm) >> lc;
                     const int per = (active + kWarps - 1) / kWarps;
                     const int b0 = warp * per, b1 = min(active, b0 + per);
                     auto flush = [&](int i, S p) {
@@ -675,9 +693,8 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                     Acc cacc[2 * NB];
 #pragma unroll
                     for (int l = 0; l < 2 * NB; ++l) P::zero(cacc[l]);
-                    const int o = (rank - I0) & cm;
 #pragma unroll 1
-                    for (int I = I0 + o + C * (kWarps - 1 - warp); I < nt; I += C * kWarps) {
+                    for (int I = first_I0 + C * (kWarps - 1 - warp); I < nt; I += C * kWarps) {
                         const int i = I * kTile + lane;
                         const V vi = vv[i];
                         V vr[NB], wr[NB];
@@ -821,7 +838,7 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
             }
             {
                 const int I0 = (k0 + nbk) >> 5, ntr = nt - I0, total = ntr * (ntr + 1) / 2;
-                const int active = (total - rank + cm) >> lc;
+                const int active = div_c(total - rank + C - 1);
 #pragma unroll 1
                 for (int unit = warp; unit < 2 * active; unit += kWarps) {  // 16 rows of a tile
                     const int ij = tab[unit >> 1], I = ij >> 8, Jt = ij & 255, mt = unit & 1;
@@ -892,7 +909,7 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
 
 }  // namespace
 
-// Cluster size and grid of a launch. The time of one chain's column was fitted
+// Cluster size (any of 1 .. 8) and grid of a launch. The time of one chain's column was fitted
 // on the GPU (N = 64 .. 1024, one chain per cluster) as P::kBase + P::kPerRow n
 // + P::kPerTile times a CTA's mean share of tiles (a third of the chain's over
 // C), +0.8 for the cluster barriers, in k cycles; `fit` clusters run at once
@@ -908,8 +925,8 @@ static double cluster_cost(int n, int nt, int C) {
 template <class P, int NB>
 static cudaError_t launch_cluster(const ChainDesc* h_desc, const ChainDesc* d_desc, int batch, int max_ld,
                                   const double* d_diag, typename P::G* d_A, void* d_spill, double* d_d, double* d_e,
-                                  typename P::G* d_tau, const int* d_order, int* d_counter, int* d_status,
-                                  cudaStream_t st) {
+                                  typename P::G* d_tau, const int* d_order, int* d_counter, int num_sms,
+                                  int* d_status, cudaStream_t st) {
     if (batch <= 0) return cudaSuccess;
     auto* kern = sytrd_cluster_kernel<P, NB>;
     const size_t tile_bytes = sizeof(typename P::V) * kTileElems, limit = 226 * 1024 / P::kOcc;
@@ -925,22 +942,17 @@ static cudaError_t launch_cluster(const ChainDesc* h_desc, const ChainDesc* d_de
     int best_slots = 0, best_cap = 0, best_fit = 0, best_C = 0;
     size_t best_smem = 0;
     double best = 0.0;
-    for (int C = 1; C <= (d_order ? 8 : 1); C *= 2) {
+    // from the largest down: with the fewest chains the first is the best, and the others need no query
+    for (int C = d_order ? 8 : 1; C >= 1; --C) {
         const int slots = slots_of(max_ld / kTile, C);
         const size_t head = smem_layout<P, NB>(max_ld, C, slots).tiles;
         if (head > limit) continue;
         const int cap = (int)min((size_t)slots, (limit - head) / tile_bytes);
         if (cap < slots && !d_spill) continue;
         const size_t smem = head + cap * tile_bytes;
-        if ((err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))) return err;
         int fit = batch;
         double cost = 0.0;
         if (d_order) {
-            at.val.clusterDim.x = C;
-            cfg.gridDim = dim3(batch * C);
-            cfg.dynamicSmemBytes = smem;
-            if ((err = cudaOccupancyMaxActiveClusters(&fit, kern, &cfg))) return err;
-            if (fit < 1) continue;
             double sum = 0.0, mx = 0.0, mn = 1e300;
             for (int c = 0; c < batch; ++c) {
                 const double t = cluster_cost<P>(h_desc[c].n, h_desc[c].ld / kTile, C);
@@ -949,7 +961,15 @@ static cudaError_t launch_cluster(const ChainDesc* h_desc, const ChainDesc* d_de
                 mn = min(mn, t);
             }
             // equal chains run in whole rounds, uneven ones (longest first) end within about half the longest
-            cost = mn == mx ? mx * ((batch + fit - 1) / fit) : max(mx, sum / fit + 0.5 * mx);
+            auto total = [&](int f) { return mn == mx ? mx * ((batch + f - 1) / f) : max(mx, sum / f + 0.5 * mx); };
+            if (best_C && total(max(1, num_sms * P::kOcc / C)) >= best) continue;
+            if ((err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))) return err;
+            at.val.clusterDim.x = C;
+            cfg.gridDim = dim3(batch * C);
+            cfg.dynamicSmemBytes = smem;
+            if ((err = cudaOccupancyMaxActiveClusters(&fit, kern, &cfg))) return err;
+            if (fit < 1) continue;
+            cost = total(fit);
         }
         if (best_C && cost >= best) continue;
         best = cost;

@@ -27,8 +27,8 @@ cudaError_t launch_sytrd_f32(const ChainDesc* h_desc, const ChainDesc* d_desc, i
                    : narrow                     ? launch_cluster<F32<8>, 4>
                    : max_ld > 768 && batch > 96 ? launch_cluster<F32<16>, 8>
                                                    : launch_cluster<F32<16>, 4>;
-    return launch(h_desc, d_desc, batch, max_ld, d_diag, d_A, d_spill, d_d, d_e, d_tau, d_order, d_counter, d_status,
-                  st);
+    return launch(h_desc, d_desc, batch, max_ld, d_diag, d_A, d_spill, d_d, d_e, d_tau, d_order, d_counter, num_sms,
+                  d_status, st);
 }
 
 }  // namespace fkg

@@ -24,8 +24,8 @@ cudaError_t launch_sytrd_f64(const ChainDesc* h_desc, const ChainDesc* d_desc, i
     const bool narrow = max_ld <= 384 && batch > num_sms;
     auto* launch = variant == 0 ? (narrow ? launch_cluster<Fix<27, 4>, 2> : launch_cluster<Fix<27, 8>, 2>)
                                 : (narrow ? launch_cluster<Fix<27, 4>, 4> : launch_cluster<Fix<27, 8>, 4>);
-    return launch(h_desc, d_desc, batch, max_ld, d_diag, d_A, d_spill, d_d, d_e, d_tau, d_order, d_counter, d_status,
-                  st);
+    return launch(h_desc, d_desc, batch, max_ld, d_diag, d_A, d_spill, d_d, d_e, d_tau, d_order, d_counter, num_sms,
+                  d_status, st);
 }
 
 }  // namespace fkg

@@ -1,4 +1,4 @@
-"""The cluster reduction of the FP64 path (sytrd_cluster.cu) at its edges: orders
+"""The cluster reduction of the FP64 path (sytrd_cluster.cuh) at its edges: orders
 around the tile and warp sizes, every cluster size (the batch decides it),
 tiles beyond shared memory, flat columns, scales far from 1, and errors.
 
@@ -56,7 +56,7 @@ def test_orders_around_tiles(solver, n):
     _check(solver, H, [rng.uniform(-2, 2, n) for _ in range(3)])
 
 
-@pytest.mark.parametrize("n,B", [(353, 1), (353, 20), (353, 60), (353, 160), (200, 170), (384, 170), (385, 153), (700, 1), (700, 40), (1000, 2), (1024, 17)])
+@pytest.mark.parametrize("n,B", [(353, 1), (353, 20), (353, 60), (353, 160), (200, 170), (384, 170), (385, 153), (700, 1), (700, 40), (1000, 2), (1024, 17), (400, 40), (576, 25), (784, 40), (1000, 22), (1024, 28)])
 def test_cluster_sizes_and_spilled_tiles(solver, n, B):
     rng = np.random.default_rng(n + B)
     H = _random_csr(n, rng)

@@ -52,7 +52,7 @@ def test_orders_around_tiles(solver, n):
 
 
 @pytest.mark.parametrize("n,B", [(200, 310), (256, 305), (130, 306), (256, 153), (350, 1), (350, 160), (480, 160), (481, 160), (600, 20),
-                                 (700, 60), (1000, 2), (1024, 17), (800, 100)])
+                                 (700, 60), (1000, 2), (1024, 17), (800, 100), (400, 40), (576, 25), (784, 40), (1024, 22)])
 def test_cluster_sizes_and_warp_counts(solver, n, B):
     _run(solver, n, B, n + B)
 
