@@ -30,71 +30,110 @@ namespace {
 constexpr int kKpmThreads = 256;
 
 // Eigenvalues of the k x k tridiagonal (al, b2 = squared off-diagonal, as
-// FP32 pairs) below x: the sign changes of the leading principal minors p_i
-// of T - x, p_0 = 1, p_i = (al_i - x) p_{i-1} - b2_{i-1} p_{i-2} (Sylvester's
-// inertia: the pivots p_i / p_{i-1} of the LDL^T factorisation of T - x), in
-// double-float. The minors are rescaled by a common power of two when they
-// leave [2^-60, 2^60]; an exact zero counts as a tiny pivot of the opposite
-// sign. No division, no FP64: GB300's FP64 pipe is ~60x narrower than FP32.
+// FP32 pairs) below x, by a pair of lanes from both ends: the even lane takes
+// the leading principal minors of the rows above m = k/2, p_0 = 1,
+// p_{i+1} = (al_i - x) p_i - b2_{i-1} p_{i-1}, the odd lane those of the rows
+// below it from the last one up (q). Their sign changes count the negative
+// pivots of the twisted LDL^T factorisation of T - x (Sylvester's inertia); the
+// twist's pivot is al_m - x - b2_{m-1} p_{m-1}/p_m - b2_m q'/q, its sign formed from
+// the products. Double-float; the minors are rescaled by a common power of two
+// when they leave [2^-60, 2^60]; an exact zero counts as a tiny pivot of the
+// opposite sign. No division, no FP64 (GB300's FP64 pipe is ~60x narrower than
+// FP32), and half the dependent steps of a count from one end (about 150 cycles
+// each).
 __device__ __forceinline__ int sturm_count(const dfl* al, const dfl* b2, int k, dfl x) {
+    const int m = k >> 1;
+    const bool odd = threadIdx.x & 1;
+    const int len = odd ? k - 1 - m : m;
     const dfl nx = {-x.hi, -x.lo};
-    dfl pm = {1.0f, 0.0f}, p = df_add(al[0], nx);
-    if (p.hi == 0.0f) p = {-1e-30f, 0.0f};
-    int cnt = p.hi < 0.0f;
-    for (int i = 1; i < k; ++i) {
-        const dfl u = df_mul(df_add(al[i], nx), p), v = df_mul(b2[i - 1], pm);
-        dfl q = df_add(u, {-v.hi, -v.lo});
-        if (q.hi == 0.0f) q = {p.hi > 0.0f ? -1e-30f * fabsf(p.hi) : 1e-30f * fabsf(p.hi), 0.0f};
-        cnt += (q.hi < 0.0f) != (p.hi < 0.0f);
-        pm = p;
-        p = q;
-        const float ap = fabsf(p.hi);
-        if (ap > 0x1p60f || ap < 0x1p-60f) {
-            const float sc = ap > 0x1p60f ? 0x1p-60f : 0x1p60f;
-            p = {p.hi * sc, p.lo * sc};
-            pm = {pm.hi * sc, pm.lo * sc};
+    dfl pm = {0.0f, 0.0f}, p = {1.0f, 0.0f};  // the minor before, the minor
+    int cnt = 0;
+    for (int t = 0; t < m; ++t)
+        if (t < len) {
+            const int i = odd ? k - 1 - t : t, c = odd ? i : i - 1;  // row, coupling to the row before
+            const dfl u = df_mul(df_add(al[i], nx), p);
+            dfl q = u;
+            if (t > 0) {
+                const dfl v = df_mul(b2[c], pm);
+                q = df_add(u, {-v.hi, -v.lo});
+            }
+            if (q.hi == 0.0f) q = {p.hi > 0.0f ? -1e-30f * fabsf(p.hi) : 1e-30f * fabsf(p.hi), 0.0f};
+            cnt += (q.hi < 0.0f) != (p.hi < 0.0f);
+            pm = p;
+            p = q;
+            const float ap = fabsf(p.hi);
+            if (ap > 0x1p60f || ap < 0x1p-60f) {
+                const float sc = ap > 0x1p60f ? 0x1p-60f : 0x1p60f;
+                p = {p.hi * sc, p.lo * sc};
+                pm = {pm.hi * sc, pm.lo * sc};
+            }
+        }
+    // larger of the two into [1, 2): the products below stay in range
+    const float sc = __int_as_float(0x7f000000 - (__float_as_int(fmaxf(fabsf(p.hi), fabsf(pm.hi))) & 0x7f800000));
+    p = {p.hi * sc, p.lo * sc};
+    pm = {pm.hi * sc, pm.lo * sc};
+    const dfl o = {__shfl_xor_sync(0xffffffffu, p.hi, 1), __shfl_xor_sync(0xffffffffu, p.lo, 1)};
+    const dfl om = {__shfl_xor_sync(0xffffffffu, pm.hi, 1), __shfl_xor_sync(0xffffffffu, pm.lo, 1)};
+    cnt += __shfl_xor_sync(0xffffffffu, cnt, 1);
+    const dfl P = odd ? o : p, Pm = odd ? om : pm, Q = odd ? p : o, Qm = odd ? pm : om;
+    dfl g = df_mul(df_add(al[m], nx), df_mul(P, Q));
+    if (m > 0) {
+        const dfl v = df_mul(b2[m - 1], df_mul(Pm, Q));
+        g = df_add(g, {-v.hi, -v.lo});
+    }
+    if (m + 1 < k) {
+        const dfl v = df_mul(b2[m], df_mul(Qm, P));
+        g = df_add(g, {-v.hi, -v.lo});
+    }
+    return cnt + (((g.hi < 0.0f) != (P.hi < 0.0f)) != (Q.hi < 0.0f));
+}
+
+constexpr int kRitzThreads = 64;               // threads per end of the spectrum
+constexpr int kPoints = kRitzThreads / 2;      // a pair of lanes per point
+
+// The first of the group's points (pair order) whose count reaches `want`, kPoints if none does. `slot`
+// alternates between calls, so that the next one may write while a slow warp still reads.
+__device__ __forceinline__ int first_point(bool reached, int group, int (*slot)[kRitzThreads / 32]) {
+    const unsigned mask = __ballot_sync(0xffffffffu, reached);
+    const int wid = (threadIdx.x & (kRitzThreads - 1)) >> 5;
+    if ((threadIdx.x & 31) == 0) (*slot)[wid] = mask ? wid * 16 + (__ffs(mask) - 1) / 2 : kPoints;
+    if (group) asm volatile("bar.sync 2, %0;" ::"n"(kRitzThreads) : "memory");
+    else asm volatile("bar.sync 1, %0;" ::"n"(kRitzThreads) : "memory");
+    int t = kPoints;
+#pragma unroll
+    for (int q = 0; q < kRitzThreads / 32; ++q) t = min(t, (*slot)[q]);
+    return t;
+}
+
+// Smallest (group 0) or largest (group 1) eigenvalue of the tridiagonal by
+// multisection, half of the CTA per end: a round counts at 64 points (6 bits).
+// It starts from the narrow bracket prev +- span around the previous Ritz value,
+// whose ends are two of the first round's points and must hold the eigenvalue,
+// else from the Gershgorin bracket, and goes on until the bracket is as narrow
+// as the double-float counts resolve (4e-14 relative).
+// One warp per end with counts from one side took 57 % of the bounds kernel.
+__device__ double ritz_extreme(const dfl* al, const dfl* b2, int k, double lo, double hi, double prev, double span,
+                               bool have_prev, int group, int (*slots)[kRitzThreads / 32]) {
+    const int point = (threadIdx.x & (kRitzThreads - 1)) >> 1, want = group ? k : 1;
+    int phase = 0;
+    if (have_prev) {
+        const double a = prev - span, step = 2.0 * span * (1.0 / (kPoints - 1));
+        const int t = first_point(sturm_count(al, b2, k, df_of(a + step * point)) >= want, group, slots);
+        phase = 1;
+        if (t > 0 && t < kPoints) {
+            lo = a + step * (t - 1);
+            hi = a + step * t;
         }
     }
-    return cnt;
-}
-
-// Smallest (largest = false) or largest eigenvalue of the tridiagonal in
-// the bracket [lo, hi] by multisection on one warp: every round each lane
-// counts at one of 32 interior points and the bracket shrinks to one
-// sub-interval (5 bits a round), until it is as narrow as the double-float
-// counts resolve (4e-14 relative).
-__device__ double warp_extreme(const dfl* al, const dfl* b2, int k, double lo, double hi, bool largest) {
-    const int lane = threadIdx.x & 31;
     for (int round = 0; round < 40; ++round) {
-        const double w = hi - lo;
+        const double w = hi - lo, step = w * (1.0 / (kPoints + 1));
         if (!(w > 4e-14 * fmax(fabs(lo), fabs(hi)))) break;
-        const double x = lo + w * (double)(lane + 1) / 33.0;
-        const int c = sturm_count(al, b2, k, df_of(x));
-        const unsigned mask = __ballot_sync(0xffffffffu, c >= (largest ? k : 1));
-        const int t = mask ? __ffs(mask) - 1 : 32;
-        const double nlo = t == 0 ? lo : lo + w * (double)t / 33.0;
-        const double nhi = t == 32 ? hi : lo + w * (double)(t + 1) / 33.0;
-        lo = nlo;
-        hi = nhi;
+        const int t = first_point(sturm_count(al, b2, k, df_of(lo + step * (point + 1))) >= want, group, slots + phase);
+        phase ^= 1;
+        if (t < kPoints) hi = lo + step * (t + 1);
+        lo += step * t;
     }
     return 0.5 * (lo + hi);
-}
-
-// Extreme eigenvalue of the tridiagonal, searched first in the narrow
-// bracket prev +- span around the previous Ritz value (Sturm counts at its ends
-// confirm that it holds the extreme eigenvalue), else in the Gershgorin bracket.
-__device__ double ritz_extreme(const dfl* al, const dfl* b2, int k, double glo, double ghi, double prev,
-                               double span, bool have_prev, bool largest) {
-    if (have_prev) {
-        const double lo = prev - span, hi = prev + span;
-        const int lane = threadIdx.x & 31;
-        int c = 0;
-        if (lane < 2) c = sturm_count(al, b2, k, df_of(lane == 0 ? lo : hi));
-        const int clo = __shfl_sync(0xffffffffu, c, 0), chi = __shfl_sync(0xffffffffu, c, 1);
-        const bool holds = largest ? (clo <= k - 1 && chi >= k) : (clo == 0 && chi >= 1);
-        if (holds) return warp_extreme(al, b2, k, lo, hi, largest);
-    }
-    return warp_extreme(al, b2, k, glo, ghi, largest);
 }
 
 // Block-wide double-float sum, to every thread: each warp's sum through shared
@@ -113,6 +152,26 @@ __device__ __forceinline__ dfl block_sum_df(dfl x, float2 (*red)[kKpmThreads / 3
     return warp_sum_df(t);
 }
 
+// Block-wide (minimum of lo, maximum of hi), to every thread; the caller's next barrier frees `red`
+__device__ __forceinline__ float2 block_range(float lo, float hi, float2* red) {
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    for (int pass = 0; pass < 2; ++pass) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        if (pass) break;
+        if (lane == 0) red[threadIdx.x >> 5] = make_float2(lo, hi);
+        __syncthreads();
+        if (lane < nw) {
+            lo = red[lane].x;
+            hi = red[lane].y;
+        }
+    }
+    return make_float2(lo, hi);
+}
+
 // sqrt(x), x > 0: the FP32 root corrected by one Newton step carried in
 // double-float (s + (x - s^2) / (2 s), the residual formed exactly by fma)
 __device__ __forceinline__ dfl df_sqrt(dfl x) {
@@ -129,7 +188,7 @@ __device__ __forceinline__ dfl df_sqrt(dfl x) {
 // step (alpha, beta, 1/beta) stay in double-float too: as FP64 numbers their square
 // root, division and conversions, done by every warp, kept the narrow FP64 pipe busy
 // for half of the kernel. Every 16
-// steps warp 0 and warp 1 compute the smallest and largest eigenvalue of the
+// steps each half of the CTA computes the smallest or largest eigenvalue of the
 // Lanczos tridiagonal; the run stops when both moved less than 1e-13 of the
 // spectral width in two consecutive checks, when the Krylov space is
 // exhausted, or at kmax (then kStatusNoConverge). Writes (e_min, e_max, a, b)
@@ -148,8 +207,9 @@ kpm_bounds_kernel(const KpmDesc* __restrict__ descs, const double* __restrict__ 
     dfl* dgd = V2 + D.ld;
     __shared__ float2 red[2][kKpmThreads / 32];
     int phase = 0;
-    __shared__ double redd[kKpmThreads / 32];
+    __shared__ float2 redd[kKpmThreads / 32];
     __shared__ double ext[2];
+    __shared__ int slots[2][2][kRitzThreads / 32];
     const double* dg = diag + D.v_off;
     dfl s2 = {0.0f, 0.0f};
     for (int i = tid; i < n; i += blockDim.x) {
@@ -210,25 +270,22 @@ kpm_bounds_kernel(const KpmDesc* __restrict__ descs, const double* __restrict__ 
         if (exhausted || (kdim >= 32 && kdim % 16 == 0) || kdim == kmax) {
             // Gershgorin bracket of the kdim x kdim tridiagonal (its last
             // off-diagonal b2[kdim-1] is the residual, not part of it)
-            double lo = 1e300, hi = -1e300;
+            // in FP32 with a margin for its rounding
+            float flo = 3e38f, fhi = -3e38f;
             for (int i = tid; i < kdim; i += blockDim.x) {
-                const double r = (i > 0 ? sqrt(df_val(b2[i - 1])) : 0.0) + (i + 1 < kdim ? sqrt(df_val(b2[i])) : 0.0);
-                const double a = df_val(al[i]);
-                lo = fmin(lo, a - r);
-                hi = fmax(hi, a + r);
+                const float r = (i > 0 ? sqrtf(b2[i - 1].hi) : 0.0f) + (i + 1 < kdim ? sqrtf(b2[i].hi) : 0.0f);
+                flo = fminf(flo, al[i].hi - r);
+                fhi = fmaxf(fhi, al[i].hi + r);
             }
-            lo = block_min(lo, redd);
-            hi = block_max(hi, redd);
-            const double width = hi - lo;
-            lo -= 1e-12 * width + 1e-300;
-            hi += 1e-12 * width + 1e-300;
-            const int wid = tid >> 5;
-            if (wid < 2) {
-                const bool largest = wid == 1;
-                const double prev = largest ? tmax : tmin;
-                const double span = fmax(4.0 * (largest ? dmax : dmin), 1e-11 * width);
-                const double e = ritz_extreme(al, b2, kdim, lo, hi, prev, span, have_prev, largest);
-                if ((tid & 31) == 0) ext[wid] = e;
+            const float2 be = block_range(flo, fhi, redd);
+            const double width = (double)be.y - (double)be.x, pad = 1e-6 * ((double)fabsf(be.x) + (double)fabsf(be.y)) + 1e-300;
+            const double lo = (double)be.x - pad, hi = (double)be.y + pad;
+            if (tid < 2 * kRitzThreads) {
+                const int group = tid / kRitzThreads;
+                const double span = fmax(4.0 * (group ? dmax : dmin), 1e-11 * width);
+                const double e = ritz_extreme(al, b2, kdim, lo, hi, group ? tmax : tmin, span, have_prev, group,
+                                              slots[group]);
+                if ((tid & (kRitzThreads - 1)) == 0) ext[group] = e;
             }
             __syncthreads();
             const double nmin = ext[0], nmax = ext[1];
