@@ -193,9 +193,11 @@ __device__ __forceinline__ dfl df_sqrt(dfl x) {
 // spectral width in two consecutive checks, when the Krylov space is
 // exhausted, or at kmax (then kStatusNoConverge). Writes (e_min, e_max, a, b)
 // and the number of Lanczos steps.
+// blockDim: 2 kRitzThreads .. kKpmThreads
 __global__ void __launch_bounds__(kKpmThreads)
 kpm_bounds_kernel(const KpmDesc* __restrict__ descs, const double* __restrict__ diag, int kmax,
-                  KpmAB* __restrict__ ab, int* __restrict__ steps, int* __restrict__ status) {
+                  KpmAB* __restrict__ ab, int* __restrict__ steps, float2* __restrict__ xdiag,
+                  float2* __restrict__ xinv, int* __restrict__ status) {
     extern __shared__ __align__(16) double ksm[];
     const KpmDesc D = descs[blockIdx.x];
     const int n = D.n, tid = threadIdx.x;
@@ -309,9 +311,17 @@ kpm_bounds_kernel(const KpmDesc* __restrict__ descs, const double* __restrict__ 
             if (!done && kdim == kmax && tid == 0) atomicOr(status, kStatusNoConverge);
         }
     }
+    // x = (H - b) / a for the moments: its diagonal and 1/a, as FP32 pairs, once per chain
+    const double a = (tmax - tmin) / 2., b = (tmax + tmin) / 2., inv_a = 1.0 / a;
+    auto pair = [](double v) {
+        const dfl d = df_of(v);
+        return make_float2(d.hi, d.lo);
+    };
+    for (int i = tid; i < n; i += blockDim.x) xdiag[D.v_off + i] = pair(((D.hdiag[i] + dg[i]) + -b) * inv_a);
     if (tid == 0) {
         if (!(tmax - tmin == tmax - tmin)) atomicOr(status, kStatusNaN);
-        ab[blockIdx.x] = KpmAB{tmin, tmax, (tmax - tmin) / 2., (tmax + tmin) / 2.};
+        xinv[blockIdx.x] = pair(inv_a);
+        ab[blockIdx.x] = KpmAB{tmin, tmax, a, b};
         if (steps) steps[blockIdx.x] = kdim;
     }
 }
@@ -320,8 +330,11 @@ kpm_bounds_kernel(const KpmDesc* __restrict__ descs, const double* __restrict__ 
 // j (local row 0 is j; rows in hop order, cnt[d] = rows within d hops).
 // Writes, per column, tr[m] = (T_m(x))_jj, p1[m] = T_{m-1}(x)e_j . T_m(x)e_j and
 // p2[m] = |T_m(x) e_j|^2 for m = 1..R at part[(v_off + j) * 3R + ...].
-__global__ void kpm_moments_kernel(const KpmDesc* __restrict__ descs, const double* __restrict__ diag,
-                                   const KpmAB* __restrict__ ab, double* __restrict__ part, int wpc) {
+// What needs FP64 was made once per chain (xdiag, xinv), and the lanes share the
+// conversions of the results: made row by row and result by result they took half
+// of the kernel (256 x N = 576 1.05 -> 0.67 ms).
+__global__ void kpm_moments_kernel(const KpmDesc* __restrict__ descs, const float2* __restrict__ xdiag,
+                                   const float2* __restrict__ xinv, double* __restrict__ part, int wpc) {
     extern __shared__ __align__(16) double ksm[];
     const int c = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const KpmDesc D = descs[c];
@@ -334,14 +347,22 @@ __global__ void kpm_moments_kernel(const KpmDesc* __restrict__ descs, const doub
     dfl* vp = reinterpret_cast<dfl*>(ksm) + (size_t)warp * 3 * D.bmax;
     dfl* vc = vp + D.bmax;
     dfl* xd = vc + D.bmax;
-    const KpmAB s = ab[c];
-    const double b = s.b, inv_a = 1.0 / s.a;
-    const dfl ia = df_of(inv_a);
-    const double* dg = diag + D.v_off;
+    const float2 iv = xinv[c];
+    const dfl ia = {iv.x, iv.y};
     double* out = part + (size_t)(D.v_off + j) * nq;
+    // result s = 3 (m - 1) + q is kept by lane s % 32 until 32 of them, or the last, are stored together
+    dfl kept = {0.0f, 0.0f};
+    int ns = 0;
+    auto put = [&](dfl v) {
+        if ((ns & 31) == lane) kept = v;
+        if ((++ns & 31) == 0 || ns == nq) {
+            const int s = ((ns - 1) & ~31) + lane;
+            if (s < ns) out[(s % 3) * R + s / 3] = df_val(kept);
+        }
+    };
     for (int r = lane; r < size; r += 32) {
-        const int site = D.bsite[base + r];
-        xd[r] = df_of(((D.hdiag[site] + dg[site]) + -b) * inv_a);
+        const float2 x = xdiag[D.v_off + D.bsite[base + r]];
+        xd[r] = {x.x, x.y};
         vp[r] = {r == 0 ? 1.0f : 0.0f, 0.0f};
         vc[r] = {0.0f, 0.0f};
     }
@@ -366,12 +387,9 @@ __global__ void kpm_moments_kernel(const KpmDesc* __restrict__ descs, const doub
     }
     __syncwarp();
     d2 = warp_sum_df(d2);
-    if (lane == 0) {
-        const double t1 = df_val(vc[0]);
-        out[0] = t1;             // tr[1]
-        out[R] = t1;             // p1[1] = e_j . x e_j
-        out[2 * R] = df_val(d2); // p2[1]
-    }
+    put(vc[0]);  // tr[1]
+    put(vc[0]);  // p1[1] = e_j . x e_j
+    put(d2);     // p2[1]
     for (int m = 1; m < R; ++m) {
         // T_{m+1} e_j = 2 x T_m e_j - T_{m-1} e_j, written over T_{m-1} e_j
         const int rows = cnt[m + 1];
@@ -390,11 +408,9 @@ __global__ void kpm_moments_kernel(const KpmDesc* __restrict__ descs, const doub
         }
         q1 = warp_sum_df(q1);
         q2 = warp_sum_df(q2);
-        if (lane == 0) {
-            out[m] = df_val(vc[0]);
-            out[R + m] = df_val(q1);
-            out[2 * R + m] = df_val(q2);
-        }
+        put(vc[0]);
+        put(q1);
+        put(q2);
         __syncwarp();
     }
 }
@@ -502,18 +518,23 @@ int kpm_warps_per_cta(int bmax) {
 
 cudaError_t launch_kpm(const KpmDesc* d_kdesc, int batch, int max_n, int max_ld, int max_bmax, int R, int M, int G,
                        int kmax, const double* d_diag, const double* d_beta, KpmAB* d_ab, int* d_steps,
-                       double* d_part, double* d_mu, double* d_logz, int* d_status, cudaStream_t st) {
+                       double* d_part, float2* d_xdiag, float2* d_xinv, double* d_mu, double* d_logz, int* d_status,
+                       cudaStream_t st) {
     if (batch <= 0) return cudaSuccess;
     if (batch > 65535) return cudaErrorInvalidValue;  // grid y limit of the moment kernel
     cudaError_t err;
     const size_t sm_b = sizeof(dfl) * (2 * (size_t)kmax + 4 * (size_t)max_ld);
     if ((err = cudaFuncSetAttribute(kpm_bounds_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_b))) return err;
-    kpm_bounds_kernel<<<batch, kKpmThreads, sm_b, st>>>(d_kdesc, d_diag, kmax, d_ab, d_steps, d_status);
+    // the threads that share the rows evenly: 256 for N = 576 left a third of them idle in the last pass, and for
+    // N = 144 barriers for warps without rows (512 chains of N = 144 2.61 -> 2.47 ms for three steps)
+    const int passes = (max_n + kKpmThreads - 1) / kKpmThreads;
+    const int bt = max(2 * kRitzThreads, ((max_n + passes - 1) / passes + 31) / 32 * 32);
+    kpm_bounds_kernel<<<batch, bt, sm_b, st>>>(d_kdesc, d_diag, kmax, d_ab, d_steps, d_xdiag, d_xinv, d_status);
     if ((err = cudaGetLastError())) return err;
     const int wpc = kpm_warps_per_cta(max_bmax);
     const size_t sm_m = kpm_moment_smem_bytes(max_bmax, wpc);
     if ((err = cudaFuncSetAttribute(kpm_moments_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_m))) return err;
-    kpm_moments_kernel<<<dim3((max_n + wpc - 1) / wpc, batch), 32 * wpc, sm_m, st>>>(d_kdesc, d_diag, d_ab, d_part,
+    kpm_moments_kernel<<<dim3((max_n + wpc - 1) / wpc, batch), 32 * wpc, sm_m, st>>>(d_kdesc, d_xdiag, d_xinv, d_part,
                                                                                       wpc);
     if ((err = cudaGetLastError())) return err;
     // moments per block of the T_m table: as many as fit in 64 KB

@@ -226,7 +226,8 @@ namespace fkg {
 // per chain; d_mu (may be null): M moments per chain.
 cudaError_t launch_kpm(const KpmDesc* d_kdesc, int batch, int max_n, int max_ld, int max_bmax, int R, int M, int G,
                        int kmax, const double* d_diag, const double* d_beta, KpmAB* d_ab, int* d_steps,
-                       double* d_part, double* d_mu, double* d_logz, int* d_status, cudaStream_t st);
+                       double* d_part, float2* d_xdiag, float2* d_xinv, double* d_mu, double* d_logz, int* d_status,
+                       cudaStream_t st);
 int kpm_warps_per_cta(int bmax);
 // One-stage reductions (sytrd_cluster.cuh). h_desc: host copy of the descriptors
 // (read only with a work list); d_A: the reflectors (FP64: null, neither they

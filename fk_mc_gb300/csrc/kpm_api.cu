@@ -131,7 +131,8 @@ int prepare_kpm(fkg_ctx* ctx, Workspace& ws, const Layout& L) {
     if ((rc = ensure_dev(ctx, ws.kdesc, sizeof(KpmDesc) * L.batch))) return rc;
     if ((rc = ensure_dev(ctx, ws.ksteps, sizeof(int) * L.batch))) return rc;
     if ((rc = ensure_dev(ctx, ws.kab, sizeof(KpmAB) * L.batch))) return rc;
-    if ((rc = ensure_dev(ctx, ws.kpart, sizeof(double) * 3 * (size_t)R * V))) return rc;
+    // per column 3 R results, the diagonal of x; per chain 1/a
+    if ((rc = ensure_dev(ctx, ws.kpart, sizeof(double) * (3 * (size_t)R * V + V + L.batch)))) return rc;
     if ((rc = ensure_dev(ctx, ws.kmu, sizeof(double) * (size_t)ctx->kpm_M * L.batch))) return rc;
     FKG_CUDA(ctx, cudaMemcpyAsync(ws.kdesc.p, kd.data(), sizeof(KpmDesc) * L.batch, cudaMemcpyHostToDevice, ctx->st));
     FKG_CUDA(ctx, cudaStreamSynchronize(ctx->st));  // kd is a local array
@@ -144,10 +145,12 @@ int enqueue_kpm(fkg_ctx* ctx, Workspace& ws, const Layout& L, double* d_mu) {
     int bmax = 1;
     for (int c = 0; c < L.batch; ++c) bmax = std::max(bmax, ctx->lat[L.desc[c].lattice].kpm_bmax);
     stage_begin(ctx, FKG_STAGE_LOGZ);
+    const size_t V = (size_t)L.v_total;
+    float2* xdiag = (float2*)((double*)ws.kpart.p + 3 * (size_t)(ctx->kpm_M / 2) * V);
     FKG_CUDA(ctx, launch_kpm((const KpmDesc*)ws.kdesc.p, L.batch, L.max_n, L.max_ld, bmax, ctx->kpm_M / 2,
                              ctx->kpm_M, ctx->kpm_G, kpm_kmax(L.max_n), (const double*)ws.diag.p,
                              (const double*)ws.beta.p, (KpmAB*)ws.kab.p, (int*)ws.ksteps.p, (double*)ws.kpart.p,
-                             d_mu, (double*)ws.logz.p, (int*)ctx->status.p, ctx->st));
+                             xdiag, xdiag + V, d_mu, (double*)ws.logz.p, (int*)ctx->status.p, ctx->st));
     stage_end(ctx, FKG_STAGE_LOGZ);
     ctx->launches += 3;
     return FKG_OK;
