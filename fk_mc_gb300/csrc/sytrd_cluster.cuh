@@ -258,9 +258,10 @@ __device__ __forceinline__ FixRefl fix_reflector(unsigned __int128 s2, ll alpha)
     const int z = lz & ~1;
     const ull M = (ull)((s2 << z) >> 64);  // Q64, in [1/4, 1)
     constexpr ull kMax = 0x7fffffffffffffffull;
-    // y = 1/sqrt(M): Newton (third order) from the FP32 estimate
-    const float mf = __ull2float_rn(M) * 0x1p-64f;
-    ull y = min(__float2ull_rn(rsqrtf(mf) * 0x1p62f), kMax);  // Q62
+    // y = 1/sqrt(M): Newton (third order) from the FP32 estimate; the estimates go through 32-bit conversions (a
+    // 64-bit one takes 64 cycles)
+    const float mf = __uint2float_rn((unsigned)(M >> 32)) * 0x1p-32f;
+    ull y = min((ull)__float2uint_rn(rsqrtf(mf) * 0x1p30f) << 32, kMax);  // Q62
     {
         const ll e = (1ll << 60) - (ll)__umul64hi(M, __umul64hi(y, y));  // Q60: 1 - M y^2
         const ll e2 = ((e >> 10) * (e >> 10)) >> 40;
@@ -268,8 +269,8 @@ __device__ __forceinline__ FixRefl fix_reflector(unsigned __int128 s2, ll alpha)
     }
     const ull xn = __umul64hi(M, y);               // Q62: sqrt(M)
     const ull D = (aa << (z / 2 - 2)) + xn;        // Q62, in [1/2, 2)
-    const float df = __ull2float_rn(D) * 0x1p-62f;
-    ull r = min(__float2ull_rn(__frcp_rn(df) * 0x1p62f), kMax);
+    const float df = __uint2float_rn((unsigned)(D >> 32)) * 0x1p-30f;
+    ull r = min((ull)__float2uint_rn(__fdividef(1.f, df) * 0x1p30f) << 32, kMax);
     {
         const ll e = (1ll << 60) - (ll)__umul64hi(D, r);
         const ll e2 = ((e >> 10) * (e >> 10)) >> 40;
