@@ -10,8 +10,8 @@
 // (no panels, no corrections). One warp forms the reflector from the column
 // (= the row that its owner wrote after the last update); four barriers a
 // column. Rows and columns that are done are skipped. Measured per solve (ms;
-// tiled kernel, this one): FP64 arithmetic N = 64 0.28, 0.157; 512 chains of N = 64
-// 1.08, 0.40; N = 121 0.68, 0.54; FP32 N = 64 0.158, 0.068; 512 chains 0.34, 0.142;
+// tiled kernel, this one): FP64 arithmetic N = 64 0.28, 0.152; 512 chains of N = 64
+// 1.08, 0.39; N = 121 0.68, 0.54; FP32 N = 64 0.158, 0.068; 512 chains 0.34, 0.142;
 // N = 121 0.34, 0.18.
 #pragma once
 #include "sytrd_cluster.cuh"
