@@ -358,6 +358,8 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
     };
     auto at = [&](auto* p, int r) { return C > 1 ? cl.map_shared_rank(p, r) : p; };
 
+    // the list's items go into every CTA's shared memory: only a CTA that runs has one
+    if (order) csync();
     for (int item = blockIdx.x / C;;) {
         if (order) {
             __syncthreads();
