@@ -443,6 +443,7 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                     }
                 }
                 if (!order) return;
+                csync();  // every CTA has read its item: CTA 0 writes the next one
                 continue;
             }
             eS = m > 0x1p-900 ? ilogb(m * (1.0 + 0x1p-30)) + 1 : -899;

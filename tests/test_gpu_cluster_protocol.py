@@ -37,3 +37,30 @@ def test_clusters_start_on_a_busy_gpu(solver, kind, L, B):
                 a = a * 1.0
         assert np.array_equal(solver.eigh_logz(ids, d, 1.5)["evals"], quiet)
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("n,B", [(353, 9), (353, 40), (1024, 17)])
+def test_rejected_chains_between_good_ones(solver, n, B, bad):
+    """Chains with an entry that is not finite among good ones: an error, and the next call's results are right."""
+    from fk_mc_gb300._lib import FkgError
+    rng = np.random.default_rng(n + B)
+    i = np.arange(n)
+    H = np.zeros((n, n))
+    for step in (1, 19):
+        H[i, (i + step) % n] += -1.0
+        H[(i + step) % n, i] += -1.0
+    nz = H != 0
+    solver.set_hopping(0, np.concatenate([[0], np.cumsum(nz.sum(1))]).astype(np.int32),
+                       np.nonzero(nz)[1].astype(np.int32), H[nz])
+    d = rng.uniform(-2, 2, (B, n))
+    ids = np.zeros(B, np.int32)
+    for rows in ([0], [B - 1], list(range(0, B, 2)), list(range(B))):
+        x = d.copy()
+        x[rows, rng.integers(0, n, len(rows))] = bad
+        with pytest.raises(FkgError, match="FKG_ERR_NUMERIC"):
+            solver.eigh_logz(ids, x.ravel(), 1.5)
+    w = solver.eigh_logz(ids, d.ravel(), 1.5)["evals"].reshape(B, n)
+    for c in sorted({0, B // 2, B - 1}):
+        A = H + np.diag(d[c])
+        assert np.abs(w[c] - np.linalg.eigvalsh(A)).max() <= 8 * n * EPS * np.abs(A).sum(1).max(), c
