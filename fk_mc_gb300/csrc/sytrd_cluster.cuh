@@ -633,6 +633,7 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                             atomicAdd(&pwi[3 * i + 1], (int)((p >> 21) & 0x1fffff));
                             atomicAdd(&pwi[3 * i + 2], (int)(p >> 42));
                         } else {
+                            __syncwarp();  // another lane may have added to this entry in the flush before
                             pwf[warp * max_ld + i] += p;
                         }
                     };

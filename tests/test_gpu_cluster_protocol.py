@@ -64,3 +64,16 @@ def test_rejected_chains_between_good_ones(solver, n, B, bad):
     for c in sorted({0, B // 2, B - 1}):
         A = H + np.diag(d[c])
         assert np.abs(w[c] - np.linalg.eigvalsh(A)).max() <= 8 * n * EPS * np.abs(A).sum(1).max(), c
+
+
+@pytest.mark.parametrize("kind,L,B", [("cubic2d", 15, 320), ("cubic2d", 19, 5), ("cubic2d", 31, 20)])
+def test_fp32_products_do_not_depend_on_timing(cuda_ok, fkg_lib, kind, L, B):
+    """Partial products that different lanes of a warp add to one entry: the FP32 sums have one order."""
+    import fk_mc_gb300
+    s = fk_mc_gb300.Solver(max_n=1024, max_batch=B, precision="mixed", tuning=None)
+    n = s.set_lattice(0, kind, L)
+    f = np.random.default_rng(L).integers(0, 2, (B, n))
+    runs = [s.eigh_logz(np.zeros(B, np.int32), (2.0 * f - 1.0).ravel(), 3.0)["evals"] for _ in range(4)]
+    s.close()
+    for w in runs[1:]:
+        assert np.array_equal(w, runs[0])
