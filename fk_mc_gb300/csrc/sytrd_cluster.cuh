@@ -327,7 +327,7 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
     constexpr size_t kTileBytes = sizeof(V) * kTileElems;
     extern __shared__ __align__(16) unsigned char sm[];
     __shared__ int s_item;
-    __shared__ double s_red[kWarps];
+    __shared__ double s_red[kWarps], s_rowsum;
     __shared__ FixRefl s_refl;
     cg::cluster_group cl = cg::this_cluster();
     const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
@@ -433,7 +433,15 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                 bad = bad || !(rs[i] < 0x1p900);
             }
             m = block_max(m, s_red);
-            if (__syncthreads_or(bad)) {  // NaN, Inf or out of the format's range
+            if (__syncthreads_or(bad)) m = NAN;
+            // The row sums' rounding depends on the order of the additions, and so, next to a power of two, does the
+            // scale: every CTA takes CTA 0's.
+            if (rank == 0 && tid == 0)
+#pragma unroll 1
+                for (int r = 0; r < C; ++r) *at(&s_rowsum, r) = m;
+            csync();
+            m = s_rowsum;
+            if (!(m < 0x1p900)) {  // NaN, Inf or out of the format's range
                 if (rank == 0) {
                     if (tid == 0 && status) atomicOr(status, kStatusNaN);
 #pragma unroll 1
@@ -443,8 +451,7 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                     }
                 }
                 if (!order) return;
-                csync();  // every CTA has read its item: CTA 0 writes the next one
-                continue;
+                continue;  // every CTA has read its item: CTA 0 writes the next one
             }
             eS = m > 0x1p-900 ? ilogb(m * (1.0 + 0x1p-30)) + 1 : -899;
             quant = scalbn(1.0, eS - 30 - P::kLo);

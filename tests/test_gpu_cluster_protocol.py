@@ -77,3 +77,26 @@ def test_fp32_products_do_not_depend_on_timing(cuda_ok, fkg_lib, kind, L, B):
     s.close()
     for w in runs[1:]:
         assert np.array_equal(w, runs[0])
+
+
+@pytest.mark.parametrize("n,B", [(200, 1), (353, 1), (600, 20)])
+def test_scale_at_a_rounding_edge(solver, n, B):
+    """A row whose absolute sum lies on either side of a power of two's threshold, as the order of its additions
+    has it: all CTAs of a cluster still work in one scale."""
+    a, b, c = 0.6870830067379103, 0.23316528022862978, 1.0797517111708146
+    assert {((a + b) + c) * (1 + 2.0 ** -30) >= 2.0, ((a + c) + b) * (1 + 2.0 ** -30) >= 2.0} == {True, False}
+    H = np.zeros((n, n))
+    i = np.arange(3, n - 1)
+    H[i, i + 1] = H[i + 1, i] = 0.1
+    H[0, 1] = H[1, 0] = b
+    H[0, 2] = H[2, 0] = c
+    H[2, 3] = H[3, 2] = 0.05
+    nz = H != 0
+    solver.set_hopping(0, np.concatenate([[0], np.cumsum(nz.sum(1))]).astype(np.int32),
+                       np.nonzero(nz)[1].astype(np.int32), H[nz])
+    d = np.zeros(n)
+    d[0] = a
+    ref = np.linalg.eigvalsh(H + np.diag(d))
+    for _ in range(10):
+        w = solver.eigh_logz(np.zeros(B, np.int32), np.tile(d, B), 1.5)["evals"].reshape(B, n)
+        assert np.abs(w - ref).max() <= 8 * n * EPS * np.abs(H + np.diag(d)).sum(1).max()
