@@ -19,9 +19,9 @@
 //      polynomial p_n(x) = det(T - x I) (three-term recurrence, rescaled by
 //      powers of two, no divisions) in double-float and one last step with
 //      p_n in FP64;
-//   4. otherwise (eigenvalues closer than the FP32 resolution) a warp per
-//      eigenvalue: FP64 Sturm counts at the ends, then safeguarded Newton in
-//      FP64 or 32-point multisection.
+//   4. otherwise (eigenvalues closer than the FP32 resolution) FP64 Sturm counts
+//      at the ends, then safeguarded Newton in FP64, or bisection (multisection
+//      where a warp has lanes to spare).
 // One thread per eigenvalue index; d and e of the chain sit in shared memory.
 #include <cfloat>
 
@@ -268,34 +268,45 @@ __device__ double newton64(const TriShared& S, int n, int ca, double tnorm, doub
     return fmin(fmax(x, a), b);
 }
 
-// FP64 eigenvalue j of a bracket that nothing confirms yet, by a whole warp (an
-// FP64 instruction costs the narrow pipe the same for one lane as for 32):
-// Sturm counts at both ends; if it holds exactly lambda_j Newton, else
-// multisection with 32 points a round (five bisections each).
-__device__ double refine64_warp(const TriShared& S, int n, int j, const TriBounds& B, float lo, float hi,
-                                int* status) {
+// FP64 eigenvalue j of a bracket that nothing confirms yet, by a group of p
+// lanes (p a power of two, the group's lanes adjacent; `active`: the group has
+// an eigenvalue; a whole warp calls): Sturm counts at both ends; if it holds
+// exactly lambda_j Newton, else multisection with p points a round (p = 1:
+// bisection).
+__device__ double refine64_group(const TriShared& S, int n, int j, const TriBounds& B, float lo, float hi, int p,
+                                 bool active, int* status) {
     const double eps = DBL_EPSILON;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, k = lane & (p - 1), base = lane - k;
+    const unsigned group = p == 32 ? 0xffffffffu : (1u << p) - 1;
     const double delta = bracket_slack(B);
     double a = fmax((double)lo - delta, B.gl), b = fmin((double)hi + delta, B.gu);
-    const int c = count64(S.d, S.e2, n, lane == 0 ? a : b, B.pivmin);
-    int ca = __shfl_sync(0xffffffffu, c, 0), cb = __shfl_sync(0xffffffffu, c, 1);
+    int ca = active ? count64(S.d, S.e2, n, k == 0 ? a : b, B.pivmin) : 0, cb;
+    if (p == 1) {
+        cb = active ? count64(S.d, S.e2, n, b, B.pivmin) : 0;
+    } else {
+        cb = __shfl_sync(0xffffffffu, ca, base + 1);
+        ca = __shfl_sync(0xffffffffu, ca, base);
+    }
     if (!(ca <= j && j < cb)) {
         a = B.gl; b = B.gu; ca = 0; cb = n;
     }
-    if (ca == j && cb == j + 1) return newton64(S, n, ca, B.tnorm, a, b);
-    for (int it = 0; it < 64; ++it) {
+    const bool newton = active && ca == j && cb == j + 1;
+    bool run = active && !newton;
+    for (int it = 0; it < 128; ++it) {
         const double w = b - a, mid = 0.5 * (a + b);
-        if (w <= 2.0 * eps * fmax(fabs(a), fabs(b)) + 0.5 * eps * B.tnorm || mid <= a || mid >= b) break;
-        const double x = fmin(fmax(a + w * ((lane + 1) * (1.0 / 33.0)), a), b);
-        const unsigned up = __ballot_sync(0xffffffffu, count64(S.d, S.e2, n, x, B.pivmin) > j);
-        const int f = up ? __ffs(up) - 1 : 32;  // first point above lambda_j
-        const double nb = __shfl_sync(0xffffffffu, x, min(f, 31)), na = __shfl_sync(0xffffffffu, x, max(f - 1, 0));
-        if (f < 32) b = nb;
-        if (f > 0) a = na;
-        if (it == 63) { if (lane == 0) atomicOr(status, kStatusNoConverge); }
+        if (w <= 2.0 * eps * fmax(fabs(a), fabs(b)) + 0.5 * eps * B.tnorm || mid <= a || mid >= b) run = false;
+        if (!__any_sync(0xffffffffu, run)) break;
+        const double x = p == 1 ? mid : fmin(fmax(a + w * ((double)(k + 1) / (p + 1)), a), b);
+        const bool above = run && count64(S.d, S.e2, n, x, B.pivmin) > j;
+        const unsigned up = __ballot_sync(0xffffffffu, above) >> base & group;
+        const int f = up ? __ffs(up) - 1 : p;  // first point above lambda_j
+        const double nb = __shfl_sync(0xffffffffu, x, base + min(f, p - 1));
+        const double na = __shfl_sync(0xffffffffu, x, base + max(f - 1, 0));
+        if (run && f < p) b = nb;
+        if (run && f > 0) a = na;
+        if (it == 127 && run) atomicOr(status, kStatusNoConverge);
     }
-    return 0.5 * (a + b);
+    return newton ? newton64(S, n, ca, B.tnorm, a, b) : 0.5 * (a + b);
 }
 
 // Gaps between the widened FP32 bracket of this thread's eigenvalue and its
@@ -324,8 +335,9 @@ __device__ __forceinline__ void neighbour_gaps(float* br, int n, int j, bool act
 // which GB300 runs about ten times faster than FP64: the FP32 bracket, then
 // safeguarded Newton on p_n in double-float (p_n'(x) in FP32 is accurate
 // enough for the step); converged at 1e-13 ||T||, far below what the FP32
-// twisted factorisation can resolve. FP64 (refine64) remains only for the
-// rare brackets the double-float Sturm counts cannot confirm.
+// twisted factorisation can resolve. FP64 (list64) remains for the brackets
+// that the double-float Sturm counts cannot confirm: none for random
+// configurations, all of them where every eigenvalue belongs to a multiplet.
 
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
     s = a + b;
@@ -463,15 +475,22 @@ __device__ bool shift_df(const float* d, const float* e2h, const float* e2l, int
     return false;
 }
 
-// The listed eigenvalues in FP64, one warp each.
+// The listed eigenvalues in FP64, packed onto the first warps: a warp's FP64
+// instruction costs the narrow pipe the same for one lane as for 32, so a warp
+// works on up to 32 eigenvalues at once, and on fewer with more lanes each. The
+// spectra of ordered configurations are all multiplets and all of them listed:
+// 256 chains of the N = 576 checkerboard 243 ms with a warp per eigenvalue.
 __device__ void list64(const ChainDesc& D, const TriShared& S, int n, const TriBounds& B, int count, const int* list,
                        const float* lbr, double* __restrict__ ww, int* __restrict__ status) {
-    for (int q = threadIdx.x >> 5; q < count; q += blockDim.x >> 5) {
-        const double lam = refine64_warp(S, n, list[q], B, lbr[2 * q], lbr[2 * q + 1], status);
-        if ((threadIdx.x & 31) == 0) {
-            ww[D.v_off + list[q]] = lam;
-            if (!isfinite(lam)) atomicOr(status, kStatusNaN);
-        }
+    if (count == 0) return;
+    int p = 1;
+    while (2 * p * count <= 32) p *= 2;
+    if ((int)(threadIdx.x & ~31u) / p >= count) return;  // nothing for this warp
+    const int q = threadIdx.x / p, i = min(q, count - 1);
+    const double lam = refine64_group(S, n, list[i], B, lbr[2 * i], lbr[2 * i + 1], p, q < count, status);
+    if (q < count && (threadIdx.x & (p - 1)) == 0) {
+        ww[D.v_off + list[i]] = lam;
+        if (!isfinite(lam)) atomicOr(status, kStatusNaN);
     }
 }
 
