@@ -110,18 +110,19 @@ struct TriShared {
     float2* de;   // (d_i, e_{i-1}^2) for the FP32 counts
     float* e2l;   // e_i^2 - e232[i]
     float* dl;    // d_i - d32[i] (null: T is FP32-exact)
+    int k;        // with dl: d32, dl and e232, e2l hold 2^-k T, of norm 1 .. 2 (else 0)
 };
 
 // shared-memory layout of one chain's tridiagonal (pairs: d as FP32 pairs too)
 __device__ __forceinline__ TriShared tri_shared(double* sm, int ld, bool pairs) {
     float* f = (float*)(sm + 2 * ld);
-    return TriShared{sm, sm + ld, f, f + ld, (float2*)(f + 2 * ld), f + 4 * ld, pairs ? f + 5 * ld : nullptr};
+    return TriShared{sm, sm + ld, f, f + ld, (float2*)(f + 2 * ld), f + 4 * ld, pairs ? f + 5 * ld : nullptr, 0};
 }
 
 // Loads d, e^2 (FP64 and FP32 copies) of chain D into shared memory and
 // returns the Gershgorin interval, max e^2 and the norm estimate.
 __device__ void load_tridiag(const ChainDesc& D, const double* __restrict__ dd, const double* __restrict__ ee,
-                             TriShared S, double& gl, double& gu, double& emax2) {
+                             TriShared& S, double& gl, double& gu, double& emax2) {
     const int n = D.n;
     __shared__ double red[3][kEigThreads / 32];
     gl = DBL_MAX; gu = -DBL_MAX; emax2 = 0.0;
@@ -131,10 +132,11 @@ __device__ void load_tridiag(const ChainDesc& D, const double* __restrict__ dd, 
         const double er = i + 1 < n ? fabs(ee[D.v_off + i]) : 0.0;
         S.d[i] = di;
         S.e2[i] = er * er;
-        S.d32[i] = (float)di;
-        S.e232[i] = i + 1 < n ? fmaxf((float)(er * er), FLT_MIN) : 0.f;
-        S.e2l[i] = (float)(er * er - (double)S.e232[i]);
-        if (S.dl) S.dl[i] = (float)(di - (double)S.d32[i]);
+        if (!S.dl) {
+            S.d32[i] = (float)di;
+            S.e232[i] = i + 1 < n ? fmaxf((float)(er * er), FLT_MIN) : 0.f;
+            S.e2l[i] = (float)(er * er - (double)S.e232[i]);
+        }
         S.de[i] = make_float2((float)di, i > 0 ? fmaxf((float)(el * el), FLT_MIN) : 0.f);
         gl = fmin(gl, di - el - er);
         gu = fmax(gu, di + el + er);
@@ -149,6 +151,19 @@ __device__ void load_tridiag(const ChainDesc& D, const double* __restrict__ dd, 
     gl = red[0][0]; gu = red[1][0]; emax2 = red[2][0];
     for (int q = 1; q < (int)(blockDim.x / 32); ++q) {
         gl = fmin(gl, red[0][q]); gu = fmax(gu, red[1][q]); emax2 = fmax(emax2, red[2][q]);
+    }
+    if (!S.dl) return;
+    // The pairs' recurrence is rescaled every four rows, by at most 2^50: away from norms around 1 it would leave
+    // FP32's range in between, and every eigenvalue go to the FP64 list.
+    const double tnorm = fmax(fabs(gl), fabs(gu));
+    S.k = tnorm >= 0x1p-900 && tnorm <= 0x1p900 ? ilogb(tnorm) : 0;
+    const double sc = scalbn(1.0, -S.k);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const double di = S.d[i] * sc, er = i + 1 < n ? ee[D.v_off + i] * sc : 0.0;
+        S.d32[i] = (float)di;
+        S.dl[i] = (float)(di - (double)S.d32[i]);
+        S.e232[i] = i + 1 < n ? fmaxf((float)(er * er), FLT_MIN) : 0.f;
+        S.e2l[i] = (float)(er * er - (double)S.e232[i]);
     }
 }
 
@@ -522,22 +537,23 @@ __device__ void charpoly_df2(const TriShared& S, int n, float xh, float xl, floa
 }
 
 // Newton in double-float from the middle of an isolated FP32 bracket, until the
-// next step would be below 1e-13 ||T||; returns the point, and p_n' there (to FP32
-// accuracy, up to 2^edp). False when the iteration cannot be trusted.
+// next step would be below 1e-13 ||T||; returns the point, and the derivative of
+// 2^-k T's polynomial there (to FP32 accuracy, up to 2^edp). False when the
+// iteration cannot be trusted.
 __device__ bool newton_df(const TriShared& S, int n, const TriBounds& B, float lo, float hi, double& x, double& dpx,
                           int& edp) {
-    const double delta = bracket_slack(B), tol = 1e-13 * B.tnorm;
-    const double x0 = 0.5 * ((double)lo + (double)hi);
+    const double delta = bracket_slack(B), sc = scalbn(1.0, -S.k), inv = scalbn(1.0, S.k), tol = 1e-13 * B.tnorm * sc;
+    const double x0 = 0.5 * ((double)lo + (double)hi) * sc;
     float xh = (float)x0, xl = (float)(x0 - (double)xh), prev = 0.f;
     for (int it = 0; it < kDfIters; ++it) {
         float p, dp;
         charpoly_df2(S, n, xh, xl, p, dp, edp);
         const float step = p / dp;
-        if (!(dp != 0.f) || !isfinite(step)) return false;
+        if (!(dp != 0.f) || !isfinite(dp) || !isfinite(step)) return false;
         float sh, se, nh, nl;
         two_sum(xh, -step, sh, se);
         fast_two_sum(sh, se + xl, nh, nl);
-        x = (double)nh + (double)nl;
+        x = ((double)nh + (double)nl) * inv;
         if (!(x >= (double)lo - delta && x <= (double)hi + delta)) return false;
         const float as = fabsf(step);
         if ((double)as <= tol || (prev > 0.f && (double)as * as * as <= 0.25 * tol * (double)prev * prev)) {
@@ -591,7 +607,7 @@ trieig_values_kernel(const ChainDesc* __restrict__ descs, const double* __restri
     const ChainDesc D = descs[blockIdx.x];
     const int n = D.n;
     if ((int)(blockIdx.y * blockDim.x) >= n) return;
-    const TriShared S = tri_shared(sm, D.ld, true);
+    TriShared S = tri_shared(sm, D.ld, true);
     double gl, gu, emax2;
     load_tridiag(D, dd, ee, S, gl, gu, emax2);
     const TriBounds B = tri_bounds(n, gl, gu, emax2);
@@ -615,7 +631,7 @@ trieig_values_kernel(const ChainDesc* __restrict__ descs, const double* __restri
             if (newton_df(S, n, B, lo, hi, x, dp, edp)) {
                 int ep;
                 const double p = charpoly_value(S.d, S.e2, n, x, ep);
-                const double step = scalbn(p / dp, max(-2000, min(2000, ep - edp)));
+                const double step = scalbn(p / dp, max(-2000, min(2000, ep - edp - S.k * (n - 1))));
                 const double lam = x - step;
                 if (fabs(step) <= 1e-11 * B.tnorm && lam >= (double)lo - delta && lam <= (double)hi + delta) {
                     ww[D.v_off + j] = lam;
@@ -642,7 +658,7 @@ trieig_shift_kernel(const ChainDesc* __restrict__ descs, const double* __restric
     const ChainDesc D = descs[blockIdx.x];
     const int n = D.n;
     if ((int)(blockIdx.y * blockDim.x) >= n) return;
-    const TriShared S = tri_shared(sm, D.ld, false);
+    TriShared S = tri_shared(sm, D.ld, false);
     __shared__ float br[2 * kEigThreads];
     __shared__ int list[kEigThreads];
     __shared__ float lbr[2 * kEigThreads];
