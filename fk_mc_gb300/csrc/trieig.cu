@@ -18,7 +18,8 @@
 //   3. if the bracket holds exactly one eigenvalue, Newton on the characteristic
 //      polynomial p_n(x) = det(T - x I) (three-term recurrence, rescaled by
 //      powers of two, no divisions) in double-float and one last step with
-//      p_n in FP64;
+//      p_n in FP64, two where a neighbour is so close that the pairs'
+//      derivative is not good enough;
 //   4. otherwise (eigenvalues closer than the FP32 resolution) FP64 Sturm counts
 //      at the ends, then safeguarded Newton in FP64, or bisection (multisection
 //      where a warp has lanes to spare).
@@ -567,13 +568,14 @@ __device__ bool newton_df(const TriShared& S, int n, const TriBounds& B, float l
     return false;
 }
 
-// Does the widened bracket [lo - delta, hi + delta] hold exactly lambda_j? Decided
-// with FP32 counts a further 1.5 delta out: an FP32 count at y is the exact count at a
-// point within delta of y, so count32(lo - 2.5 delta) >= j puts lambda_{j-1}
-// below lo - delta, and likewise above.
-__device__ __forceinline__ bool isolated32(const TriShared& S, int n, int j, const TriBounds& B, float lo, float hi) {
-    const float d25 = (float)(2.5 * bracket_slack(B));
-    return (j == 0 || count32(S.de, n, lo - d25) >= j) && (j == n - 1 || count32(S.de, n, hi + d25) <= j + 1);
+// Does the widened bracket [lo - delta, hi + delta] hold exactly lambda_j, with no
+// other eigenvalue within (m - 2) delta of it? Decided with FP32 counts m delta out:
+// an FP32 count at y is the exact count at a point within delta of y, so count32(lo
+// - m delta) >= j puts lambda_{j-1} below lo - (m - 1) delta, and likewise above.
+__device__ __forceinline__ bool isolated32(const TriShared& S, int n, int j, const TriBounds& B, float lo, float hi,
+                                           double m) {
+    const float out = (float)(m * bracket_slack(B));
+    return (j == 0 || count32(S.de, n, lo - out) >= j) && (j == n - 1 || count32(S.de, n, hi + out) <= j + 1);
 }
 
 // p_n(x) in FP64 up to 2^e (no derivative: three FP64 operations a row).
@@ -593,6 +595,28 @@ __device__ __forceinline__ double charpoly_value(const double* __restrict__ d, c
         }
     }
     return p1;
+}
+
+// The last step: from x (an FP32-pair Newton point of the eigenvalue whose
+// neighbours are `gap` away) with p_n in FP64 and the pairs' derivative dp 2^edp of
+// 2^-k T's polynomial. dp is FP32: its relative error reaches 16 eps32 ||T|| / gap
+// (at most 12 of these 16 seen over disordered rings up to n = 900, 0.1 usually).
+// Where the step times that is not below eps ||T|| / 2, one more evaluation and
+// the secant's slope give a second step. False when the steps cannot be trusted.
+__device__ bool last_step(const TriShared& S, int n, const TriBounds& B, double x, double dp, int edp, double gap,
+                          double& lam) {
+    int e0, e1;
+    const double p0 = charpoly_value(S.d, S.e2, n, x, e0);
+    const double step = scalbn(p0 / dp, max(-2000, min(2000, e0 - edp - S.k * (n - 1))));
+    lam = x - step;
+    if (!(fabs(step) <= 1e-11 * B.tnorm)) return false;
+    if (fabs(step) * (32.0 * FLT_EPSILON / DBL_EPSILON) <= gap) return true;
+    const double p1 = charpoly_value(S.d, S.e2, n, lam, e1);
+    const double den = p1 - scalbn(p0, max(-2000, min(2000, e0 - e1)));
+    if (den == 0.0) return lam == x;
+    const double second = p1 * (lam - x) / den;
+    lam -= second;
+    return fabs(second) <= 0.5 * fabs(step);
 }
 
 // One thread per eigenvalue index, FP64 result for every index: Newton in
@@ -625,19 +649,17 @@ trieig_values_kernel(const ChainDesc* __restrict__ descs, const double* __restri
     neighbour_gaps(br, n, j, active, lo, hi, delta, lgap, rgap);
     if (active) {
         bool done = false;
-        if ((lgap > 2.0 * delta && rgap > 2.0 * delta) || isolated32(S, n, j, B, lo, hi)) {
-            double x, dp;
-            int edp;
-            if (newton_df(S, n, B, lo, hi, x, dp, edp)) {
-                int ep;
-                const double p = charpoly_value(S.d, S.e2, n, x, ep);
-                const double step = scalbn(p / dp, max(-2000, min(2000, ep - edp - S.k * (n - 1))));
-                const double lam = x - step;
-                if (fabs(step) <= 1e-11 * B.tnorm && lam >= (double)lo - delta && lam <= (double)hi + delta) {
-                    ww[D.v_off + j] = lam;
-                    done = true;
-                }
-            }
+        double gap = fmin(lgap, rgap);  // beyond 2 delta the neighbours' brackets are clear of this one's
+        if (!(gap > 2.0 * delta)) {
+            if (isolated32(S, n, j, B, lo, hi, 64.0)) gap = 62.0 * delta;  // the first or last of a block
+            else gap = isolated32(S, n, j, B, lo, hi, 2.5) ? 0.5 * delta : 0.0;
+        }
+        double x, dp, lam;
+        int edp;
+        if (gap > 0.0 && newton_df(S, n, B, lo, hi, x, dp, edp) && last_step(S, n, B, x, dp, edp, gap, lam) &&
+            lam >= (double)lo - delta && lam <= (double)hi + delta) {
+            ww[D.v_off + j] = lam;
+            done = true;
         }
         if (!done) {
             const int q = atomicAdd(&cnt, 1);
