@@ -103,6 +103,9 @@ __device__ __forceinline__ void charpoly(const double* __restrict__ d, const dou
     dp = dp1;
 }
 
+// 2^k, -1022 <= k <= 1023
+__device__ __forceinline__ double pow2(int k) { return __hiloint2double((1023 + k) << 20, 0); }
+
 struct TriShared {
     double* d;
     double* e2;
@@ -111,7 +114,7 @@ struct TriShared {
     float2* de;   // (d_i, e_{i-1}^2) for the FP32 counts
     float* e2l;   // e_i^2 - e232[i]
     float* dl;    // d_i - d32[i] (null: T is FP32-exact)
-    int k;        // with dl: d32, dl and e232, e2l hold 2^-k T, of norm 1 .. 2 (else 0)
+    int k;        // d32, dl and e232, e2l hold 2^-k T (0 unless with dl and ||T|| is far from 1)
 };
 
 // shared-memory layout of one chain's tridiagonal (pairs: d as FP32 pairs too)
@@ -133,11 +136,10 @@ __device__ void load_tridiag(const ChainDesc& D, const double* __restrict__ dd, 
         const double er = i + 1 < n ? fabs(ee[D.v_off + i]) : 0.0;
         S.d[i] = di;
         S.e2[i] = er * er;
-        if (!S.dl) {
-            S.d32[i] = (float)di;
-            S.e232[i] = i + 1 < n ? fmaxf((float)(er * er), FLT_MIN) : 0.f;
-            S.e2l[i] = (float)(er * er - (double)S.e232[i]);
-        }
+        S.d32[i] = (float)di;
+        S.e232[i] = i + 1 < n ? fmaxf((float)(er * er), FLT_MIN) : 0.f;
+        S.e2l[i] = (float)(er * er - (double)S.e232[i]);
+        if (S.dl) S.dl[i] = (float)(di - (double)S.d32[i]);
         S.de[i] = make_float2((float)di, i > 0 ? fmaxf((float)(el * el), FLT_MIN) : 0.f);
         gl = fmin(gl, di - el - er);
         gu = fmax(gu, di + el + er);
@@ -157,14 +159,15 @@ __device__ void load_tridiag(const ChainDesc& D, const double* __restrict__ dd, 
     // The pairs' recurrence is rescaled every four rows, by at most 2^50: away from norms around 1 it would leave
     // FP32's range in between, and every eigenvalue go to the FP64 list.
     const double tnorm = fmax(fabs(gl), fabs(gu));
-    S.k = tnorm >= 0x1p-900 && tnorm <= 0x1p900 ? ilogb(tnorm) : 0;
-    const double sc = scalbn(1.0, -S.k);
+    if ((tnorm >= 0.25 && tnorm < 32.0) || !(tnorm >= 0x1p-480 && tnorm <= 0x1p480)) return;
+    S.k = ilogb(tnorm);
+    const double sc = pow2(-S.k), sc2 = pow2(-2 * S.k);
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double di = S.d[i] * sc, er = i + 1 < n ? ee[D.v_off + i] * sc : 0.0;
+        const double di = S.d[i] * sc, e2 = S.e2[i] * sc2;
         S.d32[i] = (float)di;
         S.dl[i] = (float)(di - (double)S.d32[i]);
-        S.e232[i] = i + 1 < n ? fmaxf((float)(er * er), FLT_MIN) : 0.f;
-        S.e2l[i] = (float)(er * er - (double)S.e232[i]);
+        S.e232[i] = i + 1 < n ? fmaxf((float)e2, FLT_MIN) : 0.f;
+        S.e2l[i] = (float)(e2 - (double)S.e232[i]);
     }
 }
 
@@ -543,8 +546,8 @@ __device__ void charpoly_df2(const TriShared& S, int n, float xh, float xl, floa
 // iteration cannot be trusted.
 __device__ bool newton_df(const TriShared& S, int n, const TriBounds& B, float lo, float hi, double& x, double& dpx,
                           int& edp) {
-    const double delta = bracket_slack(B), sc = scalbn(1.0, -S.k), inv = scalbn(1.0, S.k), tol = 1e-13 * B.tnorm * sc;
-    const double x0 = 0.5 * ((double)lo + (double)hi) * sc;
+    const double delta = bracket_slack(B), sc = pow2(-S.k), tol = 1e-13 * B.tnorm * sc;
+    const double a = ((double)lo - delta) * sc, b = ((double)hi + delta) * sc, x0 = 0.5 * ((double)lo + (double)hi) * sc;
     float xh = (float)x0, xl = (float)(x0 - (double)xh), prev = 0.f;
     for (int it = 0; it < kDfIters; ++it) {
         float p, dp;
@@ -554,11 +557,12 @@ __device__ bool newton_df(const TriShared& S, int n, const TriBounds& B, float l
         float sh, se, nh, nl;
         two_sum(xh, -step, sh, se);
         fast_two_sum(sh, se + xl, nh, nl);
-        x = ((double)nh + (double)nl) * inv;
-        if (!(x >= (double)lo - delta && x <= (double)hi + delta)) return false;
+        x = (double)nh + (double)nl;
+        if (!(x >= a && x <= b)) return false;
         const float as = fabsf(step);
         if ((double)as <= tol || (prev > 0.f && (double)as * as * as <= 0.25 * tol * (double)prev * prev)) {
             dpx = (double)dp;
+            x *= pow2(S.k);
             return true;
         }
         prev = as;
@@ -605,18 +609,27 @@ __device__ __forceinline__ double charpoly_value(const double* __restrict__ d, c
 // the secant's slope give a second step. False when the steps cannot be trusted.
 __device__ bool last_step(const TriShared& S, int n, const TriBounds& B, double x, double dp, int edp, double gap,
                           double& lam) {
-    int e0, e1;
-    const double p0 = charpoly_value(S.d, S.e2, n, x, e0);
-    const double step = scalbn(p0 / dp, max(-2000, min(2000, e0 - edp - S.k * (n - 1))));
-    lam = x - step;
-    if (!(fabs(step) <= 1e-11 * B.tnorm)) return false;
-    if (fabs(step) * (32.0 * FLT_EPSILON / DBL_EPSILON) <= gap) return true;
-    const double p1 = charpoly_value(S.d, S.e2, n, lam, e1);
-    const double den = p1 - scalbn(p0, max(-2000, min(2000, e0 - e1)));
-    if (den == 0.0) return lam == x;
-    const double second = p1 * (lam - x) / den;
-    lam -= second;
-    return fabs(second) <= 0.5 * fabs(step);
+    double p0 = 0.0, step = 0.0;
+    int e0 = 0;
+    lam = x;
+#pragma unroll 1
+    for (int it = 0;; ++it) {
+        int e;
+        const double p = charpoly_value(S.d, S.e2, n, lam, e);
+        if (it == 1) {
+            const double den = p - scalbn(p0, max(-2000, min(2000, e0 - e)));
+            if (den == 0.0) return lam == x;
+            const double second = p * (lam - x) / den;
+            lam -= second;
+            return fabs(second) <= 0.5 * fabs(step);
+        }
+        p0 = p;
+        e0 = e;
+        step = scalbn(p / dp, max(-2000, min(2000, e - edp - S.k * (n - 1))));
+        lam = x - step;
+        if (!(fabs(step) <= 1e-11 * B.tnorm)) return false;
+        if (fabs(step) * (32.0 * FLT_EPSILON / DBL_EPSILON) <= gap) return true;
+    }
 }
 
 // One thread per eigenvalue index, FP64 result for every index: Newton in
