@@ -154,9 +154,10 @@ stein_kernel(const ChainDesc* __restrict__ descs, const double* __restrict__ dd,
     }
     const double tnorm = fmax(fabs(warp_min(gl)), fabs(warp_max(gu)));
     const double ortol = 1e-5 * tnorm, pivmin = DBL_EPSILON * tnorm + DBL_MIN;
-    if (j >= n) return;
     const double* w = ww + D.v_off;
-    if (j > 0 && w[j] - w[j - 1] <= ortol) return;  // not a cluster leader
+    int members = 0;  // of the cluster that this lane leads
+    if (j < n && !(j > 0 && w[j] - w[j - 1] <= ortol))
+        for (members = 1; j + members < n && w[j + members] - w[j + members - 1] <= ortol;) ++members;
     double* Z = Zws + D.a_off;
     // chain c owns [6 a_off_c, 6 a_off_c + 6 ld_c^2): planes of ld x ld, this thread's column j
     const size_t plane = (size_t)ld * ld;
@@ -169,143 +170,176 @@ stein_kernel(const ChainDesc* __restrict__ descs, const double* __restrict__ dd,
     const long long pivbits = abs_bits(pivmin);
     auto guard = [&](double x) { return abs_bits(x) < pivbits ? copysign(pivmin, x) : x; };
     const double rs = sin(0.7 * 32), rc = cos(0.7 * 32);
-    for (int jj = j; jj < n && (jj == j || w[jj] - w[jj - 1] <= ortol); ++jj) {
-        // a perturbation of 2 eps ||T|| keeps identical eigenvalues of a cluster apart
-        const double lam = w[jj] + (jj - j) * 2.0 * DBL_EPSILON * tnorm;
+    for (int r = 0; __any_sync(0xffffffffu, r < members); ++r) {
+        const bool on = r < members;
+        const int jj = j + r;
         double* const z = Z + jj;
-        // fixed start vector 1 + sin(0.7 i + 1.3 jj) / 4: ps, pc the sine and cosine at the last multiple of 32
-        double ps, pc;
-        sincos(1.3 * jj, &ps, &pc);
-        ps *= 0.25;
-        pc *= 0.25;
-        auto start = [&](int i) {
-            if ((i & 31) == 0 && i > 0) {
-                const double t = fma(ps, rc, pc * rs);
-                pc = fma(pc, rc, -ps * rs);
-                ps = t;
-            }
-            const double2 q = rot[i & 31];
-            return fma(pc, q.x, fma(ps, q.y, 1.0));
-        };
-        // factorisation, with the first forward elimination
-        double cd = de[0].x - lam, cs = de[0].y, cur = start(0);  // active row: diagonal, superdiagonal, right side
+        double cur, rl;
         unsigned bits = 0;
-        for (int i = 0; i + 1 < n; ++i) {
-            const double sub = de[i].y, an = de[i + 1].x - lam, en = de[i + 1].y, nx = start(i + 1);
-            const bool swap = abs_bits(cd) < abs_bits(sub);
-            const double r = recip64(guard(swap ? sub : cd)), mu = (swap ? cd : sub) * r;
-            const double a1 = swap ? an : cs, a2 = swap ? en : 0.0, y = swap ? nx : cur;
-            const size_t o = (size_t)i * ld;
-            r0[o] = r;
-            u1[o] = a1;
-            u2[o] = a2;
-            ml[o] = mu;
-            yy[o] = y;
-            bits |= (unsigned)swap << (i & 31);
-            if ((i & 31) == 31) {
-                pv[(size_t)(i >> 5) * ld] = bits;
-                bits = 0;
+        if (on) {
+            // a perturbation of 2 eps ||T|| keeps identical eigenvalues of a cluster apart
+            const double lam = w[jj] + r * 2.0 * DBL_EPSILON * tnorm;
+            // fixed start vector 1 + sin(0.7 i + 1.3 jj) / 4: ps, pc the sine and cosine at the last multiple of 32
+            double ps, pc;
+            sincos(1.3 * jj, &ps, &pc);
+            ps *= 0.25;
+            pc *= 0.25;
+            auto start = [&](int i) {
+                if ((i & 31) == 0 && i > 0) {
+                    const double t = fma(ps, rc, pc * rs);
+                    pc = fma(pc, rc, -ps * rs);
+                    ps = t;
+                }
+                const double2 q = rot[i & 31];
+                return fma(pc, q.x, fma(ps, q.y, 1.0));
+            };
+            // factorisation, with the first forward elimination
+            double cd = de[0].x - lam, cs = de[0].y;  // active row: diagonal, superdiagonal, right side (cur)
+            cur = start(0);
+            for (int i = 0; i + 1 < n; ++i) {
+                const double sub = de[i].y, an = de[i + 1].x - lam, en = de[i + 1].y, nx = start(i + 1);
+                const bool swap = abs_bits(cd) < abs_bits(sub);
+                const double rp = recip64(guard(swap ? sub : cd)), mu = (swap ? cd : sub) * rp;
+                const double a1 = swap ? an : cs, a2 = swap ? en : 0.0, y = swap ? nx : cur;
+                const size_t o = (size_t)i * ld;
+                r0[o] = rp;
+                u1[o] = a1;
+                u2[o] = a2;
+                ml[o] = mu;
+                yy[o] = y;
+                bits |= (unsigned)swap << (i & 31);
+                if ((i & 31) == 31) {
+                    pv[(size_t)(i >> 5) * ld] = bits;
+                    bits = 0;
+                }
+                cur = fma(-mu, y, swap ? cur : nx);
+                cd = fma(-mu, a1, swap ? cs : an);
+                cs = fma(-mu, a2, swap ? 0.0 : en);
             }
-            cur = fma(-mu, y, swap ? cur : nx);
-            cd = fma(-mu, a1, swap ? cs : an);
-            cs = fma(-mu, a2, swap ? 0.0 : en);
+            if ((n - 1) & 31) pv[(size_t)((n - 1) >> 5) * ld] = bits;
+            rl = recip64(guard(cd));
         }
-        if ((n - 1) & 31) pv[(size_t)((n - 1) >> 5) * ld] = bits;
-        const double rl = recip64(guard(cd));
         double nrm, sg;  // squared norm, a component with the vector's sign
+        long long best;  // the largest component (the first of equal ones)
         for (int it = 0;; ++it) {
-            // back substitution
-            double x1 = cur * rl, x2 = 0.0;
-            long long best = abs_bits(x1);  // the largest component (the first of equal ones) and its sign
-            sg = x1;
-            double sq[4] = {x1 * x1, 0.0, 0.0, 0.0};  // four sums round less than one
-            z[(size_t)(n - 1) * ld] = x1;
-            double cy[4], c1[4], c2[4], cr[4];
-            auto fetch = [&](int i0) {
+            if (on) {
+                // back substitution
+                double x1 = cur * rl, x2 = 0.0;
+                best = abs_bits(x1);
+                sg = x1;
+                double sq[4] = {x1 * x1, 0.0, 0.0, 0.0};  // four sums round less than one
+                z[(size_t)(n - 1) * ld] = x1;
+                double cy[4], c1[4], c2[4], cr[4];
+                auto fetch = [&](int i0) {
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const size_t o = (size_t)max(i0 - u, 0) * ld;
-                    cy[u] = yy[o]; c1[u] = u1[o]; c2[u] = u2[o]; cr[u] = r0[o];
-                }
-            };
-            if (n > 1) fetch(n - 2);
-            for (int i0 = n - 2; i0 >= 0; i0 -= 4) {
-                double ty[4], t1[4], t2[4], tr[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) { ty[u] = cy[u]; t1[u] = c1[u]; t2[u] = c2[u]; tr[u] = cr[u]; }
-                if (i0 >= 4) fetch(i0 - 4);
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (i0 >= u) {
-                        const double x = fma(-t1[u], x1, fma(-t2[u], x2, ty[u])) * tr[u];
-                        x2 = x1;
-                        x1 = x;
-                        z[(size_t)(i0 - u) * ld] = x;
-                        const long long ab = abs_bits(x);
-                        if (ab >= best) { best = ab; sg = x; }
-                        if (it == 2) sq[u] = fma(x, x, sq[u]);
+                    for (int u = 0; u < 4; ++u) {
+                        const size_t o = (size_t)max(i0 - u, 0) * ld;
+                        cy[u] = yy[o]; c1[u] = u1[o]; c2[u] = u2[o]; cr[u] = r0[o];
                     }
-            }
-            nrm = (sq[0] + sq[1]) + (sq[2] + sq[3]);
-            if (jj > j) {  // orthogonalise against the cluster's earlier vectors
-                for (int q = j; q < jj; ++q) {
-                    double dot = 0.0;
-                    for (int i = 0; i < n; ++i) dot += Z[(size_t)i * ld + q] * z[(size_t)i * ld];
-                    for (int i = 0; i < n; ++i) z[(size_t)i * ld] -= dot * Z[(size_t)i * ld + q];
+                };
+                if (n > 1) fetch(n - 2);
+                for (int i0 = n - 2; i0 >= 0; i0 -= 4) {
+                    double ty[4], t1[4], t2[4], tr[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) { ty[u] = cy[u]; t1[u] = c1[u]; t2[u] = c2[u]; tr[u] = cr[u]; }
+                    if (i0 >= 4) fetch(i0 - 4);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (i0 >= u) {
+                            const double x = fma(-t1[u], x1, fma(-t2[u], x2, ty[u])) * tr[u];
+                            x2 = x1;
+                            x1 = x;
+                            z[(size_t)(i0 - u) * ld] = x;
+                            const long long ab = abs_bits(x);
+                            if (ab >= best) { best = ab; sg = x; }
+                            if (it == 2) sq[u] = fma(x, x, sq[u]);
+                        }
                 }
-                best = -1;
-                nrm = 0.0;
-                for (int i = 0; i < n; ++i) {
-                    const double x = z[(size_t)i * ld];
-                    if (abs_bits(x) > best) { best = abs_bits(x); sg = x; }
-                    nrm = fma(x, x, nrm);
-                }
+                nrm = (sq[0] + sq[1]) + (sq[2] + sq[3]);
             }
-            const int k = (int)(best >> 52) - 1023;  // 1024: not a number, which stays so
-            if (it == 2) {
-                if (!(nrm > 1e-280 && nrm < 1e280) && k < 1024) {  // squares out of range: the scaled vector
-                    nrm = 0.0;
-                    for (int i = 0; i < n; ++i) {
-                        const double x = scale_down(z[(size_t)i * ld], k);
-                        z[(size_t)i * ld] = x;
-                        nrm = fma(x, x, nrm);
+            if (r > 0) {
+                // orthogonalise against the cluster's earlier vectors, the whole warp on one vector after the other
+                // (a lane that works alone takes as much of the FP64 pipe as 32), a lane's rows lane + 32 q
+                __syncwarp();
+                for (unsigned todo = __ballot_sync(0xffffffffu, on); todo; todo &= todo - 1) {
+                    const int l = __ffs(todo) - 1, first = j - lane + l;
+                    double* const x = Z + first + r;
+                    for (int q = first; q < first + r; ++q) {
+                        double dot = 0.0;
+                        for (int i = lane; i < n; i += 32) dot = fma(Z[(size_t)i * ld + q], x[(size_t)i * ld], dot);
+                        dot = warp_sum(dot);
+                        for (int i = lane; i < n; i += 32) x[(size_t)i * ld] -= dot * Z[(size_t)i * ld + q];
+                    }
+                    long long top = -1;
+                    double tx = 0.0, sum = 0.0;
+                    int ti = n;
+                    for (int i = lane; i < n; i += 32) {
+                        const double y = x[(size_t)i * ld];
+                        if (abs_bits(y) > top) { top = abs_bits(y); tx = y; ti = i; }
+                        sum = fma(y, y, sum);
+                    }
+                    sum = warp_sum(sum);
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        const long long ot = __shfl_xor_sync(0xffffffffu, top, o);
+                        const double ox = __shfl_xor_sync(0xffffffffu, tx, o);
+                        const int oi = __shfl_xor_sync(0xffffffffu, ti, o);
+                        if (ot > top || (ot == top && oi < ti)) { top = ot; tx = ox; ti = oi; }
+                    }
+                    if (lane == l) { best = top; sg = tx; nrm = sum; }
+                }
+                __syncwarp();
+            }
+            if (on) {
+                const int k = (int)(best >> 52) - 1023;  // 1024: not a number, which stays so
+                if (it == 2) {
+                    if (!(nrm > 1e-280 && nrm < 1e280) && k < 1024) {  // squares out of range: the scaled vector
+                        nrm = 0.0;
+                        for (int i = 0; i < n; ++i) {
+                            const double x = scale_down(z[(size_t)i * ld], k);
+                            z[(size_t)i * ld] = x;
+                            nrm = fma(x, x, nrm);
+                        }
+                    }
+                } else {
+                    // scaled forward elimination
+                    const double nan = k == 1024 ? (double)NAN : 0.0;
+                    cur = scale_down(z[0], k) + nan;
+                    double cz[4], cm[4];
+                    auto fetch2 = [&](int i0) {
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const size_t o = (size_t)min(i0 + u, n - 2) * ld;
+                            cm[u] = ml[o];
+                            cz[u] = z[o + ld];
+                        }
+                    };
+                    if (n > 1) fetch2(0);
+                    for (int i0 = 0; i0 + 1 < n; i0 += 4) {
+                        double tm[4], tz[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) { tm[u] = cm[u]; tz[u] = cz[u]; }
+                        if (i0 + 5 < n) fetch2(i0 + 4);
+                        if ((i0 & 31) == 0) bits = pv[(size_t)(i0 >> 5) * ld];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (i0 + u + 1 < n) {
+                                const bool swap = bits >> ((i0 + u) & 31) & 1;
+                                const double nx = scale_down(tz[u], k), y = swap ? nx : cur;
+                                yy[(size_t)(i0 + u) * ld] = y;
+                                cur = fma(-tm[u], y, swap ? cur : nx);
+                            }
                     }
                 }
-                break;
             }
-            // scaled forward elimination
-            const double nan = k == 1024 ? (double)NAN : 0.0;
-            cur = scale_down(z[0], k) + nan;
-            double cz[4], cm[4];
-            auto fetch2 = [&](int i0) {
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const size_t o = (size_t)min(i0 + u, n - 2) * ld;
-                    cm[u] = ml[o];
-                    cz[u] = z[o + ld];
-                }
-            };
-            if (n > 1) fetch2(0);
-            for (int i0 = 0; i0 + 1 < n; i0 += 4) {
-                double tm[4], tz[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) { tm[u] = cm[u]; tz[u] = cz[u]; }
-                if (i0 + 5 < n) fetch2(i0 + 4);
-                if ((i0 & 31) == 0) bits = pv[(size_t)(i0 >> 5) * ld];
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (i0 + u + 1 < n) {
-                        const bool swap = bits >> ((i0 + u) & 31) & 1;
-                        const double nx = scale_down(tz[u], k), y = swap ? nx : cur;
-                        yy[(size_t)(i0 + u) * ld] = y;
-                        cur = fma(-tm[u], y, swap ? cur : nx);
-                    }
-            }
+            if (it == 2) break;
         }
         // sign: largest component positive (deterministic output)
-        const double sc = copysign(1.0 / sqrt(nrm), sg);
+        if (on) {
+            const double sc = copysign(1.0 / sqrt(nrm), sg);
 #pragma unroll 4
-        for (int i = 0; i < n; ++i) z[(size_t)i * ld] *= sc;
+            for (int i = 0; i < n; ++i) z[(size_t)i * ld] *= sc;
+        }
     }
 }
 

@@ -64,3 +64,45 @@ def test_multiplets_cost_no_warp_each(cuda_ok, fkg_lib, precision):
         s.profile(False)
     s.close()
     assert ms[1] <= 35 * ms[0], ms
+
+
+@pytest.mark.parametrize("kind,L", [("cubic2d", 4), ("cubic2d", 8), ("cubic3d", 6), ("cubic2d", 24)])
+def test_vectors_of_multiplets(cuda_ok, fkg_lib, kind, L):
+    """Inverse iteration with the members of a multiplet orthogonalised against each other: residual below
+    8 n eps ||H||, orthogonal to 1e-10 (the FP64 path's stated accuracy)."""
+    import fk_mc_gb300
+    from fk_mc_gb300.lattice import dense
+    n = L ** NDIM[kind]
+    cb = _checkerboard(kind, L)
+    one = cb.copy()
+    one[n // 3] ^= 1
+    fs = [cb, np.zeros(n, int), one]
+    s = fk_mc_gb300.Solver(max_n=n, max_batch=len(fs), precision="f64")
+    s.set_lattice(0, kind, L)
+    out = s.eigh_logz(np.zeros(len(fs), np.int32), np.concatenate([4.0 * (f - 0.5) for f in fs]), 8.0, vectors=True)
+    s.close()
+    for c, f in enumerate(fs):
+        A, X, w = dense(kind, L) + np.diag(4.0 * (f - 0.5)), out["evecs"][c], out["evals"][c * n:(c + 1) * n]
+        assert np.abs(A @ X - X * w).max() <= 8 * n * EPS * np.abs(A).sum(1).max()
+        assert np.abs(X.T @ X - np.eye(n)).max() <= 1e-10
+
+
+def test_vectors_of_multiplets_use_whole_warps(cuda_ok, fkg_lib):
+    """The N = 576 lattice without f: multiplets of 4, 8 and 46. Members are solved one after the other (a lane at
+    work: ~4 times the time of single eigenvalues); their orthogonalisation, n multiply-adds for every pair, must not
+    take a lane's time each as well (then 40 times)."""
+    import time
+    import fk_mc_gb300
+    L, B = 24, 16
+    n = L * L
+    s = fk_mc_gb300.Solver(max_n=n, max_batch=B, precision="f64")
+    s.set_lattice(0, "cubic2d", L)
+    ms = []
+    for f in (np.random.default_rng(1).integers(0, 2, (B, n)), np.zeros((B, n))):
+        ids, d = np.zeros(B, np.int32), (4.0 * (f - 0.5)).ravel()
+        s.measure_ipr(ids, d, 4.0)
+        t = time.perf_counter()
+        s.measure_ipr(ids, d, 4.0)
+        ms.append(time.perf_counter() - t)
+    s.close()
+    assert ms[1] <= 18 * ms[0], ms
