@@ -15,8 +15,10 @@ eigenvectors (the panel widths matter only for the latter; the values-only
 one-stage reduction has one width). It then times the mixed path's two back-transformation
 kernels (mma.sync with the block of Z in shared memory, tcgen05 with
 tensor-memory accumulators; fkg_set_tuning_back) per size class under the
-chosen reduction. `Solver(..., tuning=path)` (default: the table shipped next
-to this file, when present) applies it with fkg_set_tuning.
+chosen reduction, and the proposal steps of resident chains, which need
+eigenvalues only, under the one-stage and the two-stage reduction
+(fkg_set_tuning_chains). `Solver(..., tuning=path)` (default: the table shipped
+next to this file, when present) applies it with these setters.
 
 Run on the GPU:  python -m fk_mc_gb300.autotune --out fk_mc_gb300/tuning_gb300.json
 """
@@ -63,8 +65,9 @@ def tune(batch=None, reps=3, seed=1):
                 times.append(sum(s.stage_time(st)[0] for st in STAGES) / reps)
                 s.profile(False)
             best = int(np.argmin(times))
-            table["entries"].append({"precision": prec, "n_max": n, "variant": best, "panel_width": widths[best],
-                                     "ms_per_solve": [round(t, 4) for t in times], "batch": batch})
+            reduction = {"precision": prec, "n_max": n, "variant": best, "panel_width": widths[best],
+                         "ms_per_solve": [round(t, 4) for t in times], "batch": batch}
+            table["entries"].append(reduction)
             if prec == "mixed":
                 s.set_tuning(prec, n, best)
                 bt = []
@@ -80,6 +83,16 @@ def tune(batch=None, reps=3, seed=1):
                 table["entries"].append({"stage": "back", "n_max": n, "variant": best,
                                          "kernel": BACK_VARIANTS[best], "ms_per_solve": [round(t, 4) for t in bt],
                                          "batch": batch})
+                s.chains_init(ids, f.ravel(), 2.0, 1.0, 1.0, 4.0)
+                st = []
+                for v in (0, 1):
+                    s.set_tuning_chains(n, v)
+                    s.propose_accept(rng.integers(0, n, (1, batch)), np.full((1, batch), 0.5))  # warm
+                    s.profile(True)
+                    s.propose_accept(rng.integers(0, n, (reps, batch)), np.full((reps, batch), 0.5))
+                    st.append(sum(s.stage_time(x)[0] for x in STAGES) / reps)
+                    s.profile(False)
+                reduction.update(chains=int(np.argmin(st)), ms_per_step=[round(t, 4) for t in st])
                 s.set_tuning_back(n, -1)
             s.set_tuning(prec, n, -1)
         s.close()
@@ -96,6 +109,8 @@ def apply(solver, path=DEFAULT_TABLE):
             solver.set_tuning_back(e["n_max"], e["variant"])
         else:
             solver.set_tuning(e["precision"], e["n_max"], e["variant"])
+            if "chains" in e:
+                solver.set_tuning_chains(e["n_max"], e["chains"])
     return True
 
 

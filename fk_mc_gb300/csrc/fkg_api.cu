@@ -120,16 +120,22 @@ int upload_layout(fkg_ctx* ctx, Workspace& ws, const Layout& L) {
 // one-stage kernel, whose persistent longest-first schedule balances them
 // (measured on the uneven batch of n = 144 .. 1024: 14.7k against 12.7k
 // proposals/s).
-static int pick_variant(const fkg_ctx* ctx, const Layout& L, bool f32) {
+// chains: the layout of the device-resident chains, whose choice can be set apart.
+static int pick_variant(const fkg_ctx* ctx, const Layout& L, bool f32, bool chains = false) {
+    auto set = [&](int b) {
+        if (!f32) return ctx->tune_f64[b];
+        if (chains && ctx->tune_chains[b] >= 0) return ctx->tune_chains[b] ? kTwoStageVariant : 1;
+        return ctx->tune_f32[b];
+    };
     double work[17] = {0};
     for (const ChainDesc& d : L.desc) work[std::min(16, (d.n + 63) / 64)] += (double)d.n * d.n * d.n;
     int best = 0;
     for (int b = 1; b < 17; ++b)
         if (work[b] > work[best]) best = b;
-    const int v = f32 ? ctx->tune_f32[best] : ctx->tune_f64[best];
+    const int v = set(best);
     if (f32 && v == kTwoStageVariant)
         for (const ChainDesc& d : L.desc)
-            if (ctx->tune_f32[std::min(16, (d.n + 63) / 64)] != kTwoStageVariant) return 1;
+            if (set(std::min(16, (d.n + 63) / 64)) != kTwoStageVariant) return 1;
     return v >= 0 ? v : 1;
 }
 
@@ -239,7 +245,7 @@ int enqueue_solve(fkg_ctx* ctx, Workspace& ws, const Layout& L, bool want_exp, c
         // the two-stage reduction where every chain is in the class above 960 and a table is set for it, else
         // sytrd_v3 (any other order of summation moves dF/dU by the path's own error, 1e-7). Values-only solves
         // take the faster sytrd_cluster kernel: 256 chains of N = 576 9.9 -> 7.9 ms, 16 of N = 1024 14.9 -> 7.2.
-        const int variant = pick_variant(ctx, L, true);
+        const int variant = pick_variant(ctx, L, true, &ws == &ctx->chain);
         two_stage = variant == kTwoStageVariant || (want_q && L.min_n > 960 && ctx->tune_f32[16] >= 0);
         if (two_stage) {
             const int rc = upload_tensor_maps(ctx, ws, L);
@@ -469,6 +475,16 @@ int fkg_set_tuning(fkg_ctx* ctx, int precision, int n_max, int variant) {
     if (variant < -1 || variant >= nvar) return set_err(ctx, FKG_ERR_ARG, "variant out of range");
     int* tune = precision == FKG_PREC_MIXED ? ctx->tune_f32 : ctx->tune_f64;
     tune[std::min(16, (n_max + 63) / 64)] = variant;
+    if (precision == FKG_PREC_MIXED) ctx->tune_chains[std::min(16, (n_max + 63) / 64)] = -1;
+    ctx->drop_graph();
+    return FKG_OK;
+}
+
+int fkg_set_tuning_chains(fkg_ctx* ctx, int n_max, int variant) {
+    if (!ctx) return FKG_ERR_ARG;
+    if (n_max < 1 || n_max > kMaxN) return set_err(ctx, FKG_ERR_ARG, "n_max out of range");
+    if (variant < -1 || variant > 1) return set_err(ctx, FKG_ERR_ARG, "variant out of range");
+    ctx->tune_chains[std::min(16, (n_max + 63) / 64)] = variant;
     ctx->drop_graph();
     return FKG_OK;
 }

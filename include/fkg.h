@@ -235,6 +235,13 @@ int fkg_set_stream(fkg_ctx* ctx, void* cuda_stream);
  * Written by the autotuner (fk_mc_gb300/autotune.py) from measured times. */
 int fkg_set_tuning(fkg_ctx* ctx, int precision, int n_max, int variant);
 
+/* Reduction of the device-resident chains (fkg_chains_init and the proposal
+ * steps: eigenvalues only) on the mixed path for matrices of order up to n_max
+ * (size buckets of 64): 0 = one-stage, 1 = two-stage; -1 (the default, and what
+ * fkg_set_tuning restores for its bucket) = as fkg_set_tuning says. A batch is
+ * two-stage only if every chain's bucket selects it. Written by the autotuner. */
+int fkg_set_tuning_chains(fkg_ctx* ctx, int n_max, int variant);
+
 /* Back-transformation kernel of the mixed path for matrices of order up to
  * n_max (size buckets of 64): 0 = mma.sync 3xTF32 with the column block of Z
  * in shared memory (the default), 1 = tcgen05 3xTF32 with tensor-memory

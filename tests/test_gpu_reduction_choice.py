@@ -1,0 +1,61 @@
+"""Which reduction the mixed path takes: the caller's settings per size bucket, for
+solves and for resident chains, by the number of launches (a two-stage solve has
+two more than a one-stage one) and by results.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture()
+def solver(cuda_ok, fkg_lib):
+    import fk_mc_gb300
+    s = fk_mc_gb300.Solver(max_n=1024, max_batch=2, precision="mixed", tuning=None)
+    s.set_graphs(False)
+    yield s
+    s.close()
+
+
+def _launches(s, call):
+    call()  # workspaces
+    n0 = s.launch_count()
+    call()
+    return s.launch_count() - n0
+
+
+def _lattices(s, *sizes):
+    return [s.set_lattice(i, "cubic2d", L) for i, L in enumerate(sizes)]
+
+
+def _diag(ns, seed=3):
+    return np.random.default_rng(seed).integers(0, 2, sum(ns)) * 2.0 - 1.0
+
+
+def test_chains_can_be_set_apart(solver):
+    s = solver
+    ns = _lattices(s, 9, 9)
+    ids, rng = [0, 1], np.random.default_rng(1)
+    f, site, u = rng.integers(0, 2, sum(ns)), rng.integers(0, 81, (1, 2)), np.full((1, 2), 2.0)  # u = 2: none accepted
+    solve = lambda: s.eigh_logz(ids, _diag(ns), 4.0)
+    step = lambda: s.propose_accept(site, u)
+    init = lambda: s.chains_init(ids, f, 2.0, 1.0, 1.0, 4.0)
+    init()
+    one_solve, one_step, one_init, dl = _launches(s, solve), _launches(s, step), _launches(s, init), step()[1]
+    for solves, chains, more_solve, more_step in [(3, None, 2, 2), (3, 0, 2, 0), (3, -1, 2, 2), (1, None, 0, 0),
+                                                  (1, 1, 0, 2), (3, None, 2, 2), (-1, None, 0, 0)]:
+        s.set_tuning("mixed", 81, solves)  # takes the chains' bucket back to its own choice
+        if chains is not None:
+            s.set_tuning_chains(81, chains)
+        case = (solves, chains)
+        assert _launches(s, solve) == one_solve + more_solve, case
+        assert _launches(s, init) == one_init + more_step, case
+        assert _launches(s, step) == one_step + more_step, case
+        assert np.abs(step()[1] - dl).max() < 1e-8, case
+
+
+def test_chains_setting_rejects_what_it_does_not_know(solver):
+    from fk_mc_gb300._lib import FkgError
+    for n_max, v in [(0, 0), (1025, 0), (64, 2), (64, -2)]:
+        with pytest.raises(FkgError, match="FKG_ERR_ARG"):
+            solver.set_tuning_chains(n_max, v)
