@@ -15,9 +15,9 @@ eigenvectors (the panel widths matter only for the latter; the values-only
 one-stage reduction has one width). It then times the mixed path's two back-transformation
 kernels (mma.sync with the block of Z in shared memory, tcgen05 with
 tensor-memory accumulators; fkg_set_tuning_back) per size class under the
-chosen reduction, and the proposal steps of resident chains, which need
-eigenvalues only, under the one-stage and the two-stage reduction
-(fkg_set_tuning_chains). `Solver(..., tuning=path)` (default: the table shipped
+chosen reduction. Where that is the two-stage one, it times the proposal steps of
+resident chains, which need eigenvalues only, under both reductions: with few
+chains the one-stage kernel gives each several SMs (fkg_set_tuning_chains). `Solver(..., tuning=path)` (default: the table shipped
 next to this file, when present) applies it with these setters.
 
 Run on the GPU:  python -m fk_mc_gb300.autotune --out fk_mc_gb300/tuning_gb300.json
@@ -33,6 +33,20 @@ CLASSES = [("cubic2d", 12), ("cubic2d", 16), ("triangular", 18), ("cubic2d", 20)
 VARIANTS = {"mixed": [4, 8, 16, "two-stage"], "f64": [2, 4]}  # panel widths (or two-stage), index = variant
 STAGES = ("reduce", "trieig", "back", "refine")
 BACK_VARIANTS = {0: "mma.sync", 1: "tcgen05"}       # back-transformation kernels of the mixed path
+
+
+def _step_ms(s, n, f, most, reps, rng):
+    """Stage times of a proposal step of resident chains reduced in one stage (most >= their number) or two."""
+    B = len(f)
+    s.set_tuning_chains(n, most)
+    s.chains_init(np.zeros(B, np.int32), f.ravel(), 2.0, 1.0, 1.0, 4.0)
+    step = lambda k: s.propose_accept(rng.integers(0, n, (k, B)), np.full((k, B), 0.5))
+    step(1)  # warm
+    s.profile(True)
+    step(reps)
+    ms = sum(s.stage_time(st)[0] for st in STAGES) / reps
+    s.profile(False)
+    return ms
 
 
 def tune(batch=None, reps=3, seed=1):
@@ -83,16 +97,12 @@ def tune(batch=None, reps=3, seed=1):
                 table["entries"].append({"stage": "back", "n_max": n, "variant": best,
                                          "kernel": BACK_VARIANTS[best], "ms_per_solve": [round(t, 4) for t in bt],
                                          "batch": batch})
-                s.chains_init(ids, f.ravel(), 2.0, 1.0, 1.0, 4.0)
-                st = []
-                for v in (0, 1):
-                    s.set_tuning_chains(n, v)
-                    s.propose_accept(rng.integers(0, n, (1, batch)), np.full((1, batch), 0.5))  # warm
-                    s.profile(True)
-                    s.propose_accept(rng.integers(0, n, (reps, batch)), np.full((reps, batch), 0.5))
-                    st.append(sum(s.stage_time(x)[0] for x in STAGES) / reps)
-                    s.profile(False)
-                reduction.update(chains=int(np.argmin(st)), ms_per_step=[round(t, 4) for t in st])
+                if widths[reduction["variant"]] == "two-stage":
+                    s.set_tuning_back(n, best)
+                    steps = [(b, [_step_ms(s, n, f[:b], most, reps, rng) for most in (b, 0)])
+                             for b in (batch // 4, batch // 2, batch)]
+                    reduction.update(chains=max([b for b, (one, two) in steps if one < two], default=0),
+                                     ms_per_step=[[b, round(one, 4), round(two, 4)] for b, (one, two) in steps])
                 s.set_tuning_back(n, -1)
             s.set_tuning(prec, n, -1)
         s.close()

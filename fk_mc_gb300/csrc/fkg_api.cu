@@ -124,7 +124,7 @@ int upload_layout(fkg_ctx* ctx, Workspace& ws, const Layout& L) {
 static int pick_variant(const fkg_ctx* ctx, const Layout& L, bool f32, bool chains = false) {
     auto set = [&](int b) {
         if (!f32) return ctx->tune_f64[b];
-        if (chains && ctx->tune_chains[b] >= 0) return ctx->tune_chains[b] ? kTwoStageVariant : 1;
+        if (chains && ctx->tune_chains[b] >= 0) return L.batch > ctx->tune_chains[b] ? kTwoStageVariant : 1;
         return ctx->tune_f32[b];
     };
     double work[17] = {0};
@@ -480,11 +480,11 @@ int fkg_set_tuning(fkg_ctx* ctx, int precision, int n_max, int variant) {
     return FKG_OK;
 }
 
-int fkg_set_tuning_chains(fkg_ctx* ctx, int n_max, int variant) {
+int fkg_set_tuning_chains(fkg_ctx* ctx, int n_max, int most) {
     if (!ctx) return FKG_ERR_ARG;
     if (n_max < 1 || n_max > kMaxN) return set_err(ctx, FKG_ERR_ARG, "n_max out of range");
-    if (variant < -1 || variant > 1) return set_err(ctx, FKG_ERR_ARG, "variant out of range");
-    ctx->tune_chains[std::min(16, (n_max + 63) / 64)] = variant;
+    if (most < -1) return set_err(ctx, FKG_ERR_ARG, "number of chains out of range");
+    ctx->tune_chains[std::min(16, (n_max + 63) / 64)] = most;
     ctx->drop_graph();
     return FKG_OK;
 }

@@ -145,7 +145,7 @@ struct fkg_ctx {
     // (bucket b covers n in (64 (b-1), 64 b]); -1 = default
     int tune_f32[17], tune_f64[17];
     int tune_bt[17];  // back-transformation kernel of the mixed path per size bucket (-1: default)
-    int tune_chains[17];  // reduction of device-resident chains, mixed path: 0 one-stage, 1 two-stage, -1 as tune_f32
+    int tune_chains[17];  // mixed path: the most resident chains that are reduced in one stage (-1: as tune_f32 says)
     // CUDA graph of one proposal step (fkg_propose_accept*), replayed per step
     bool use_graphs = true;
     int graph_kernels = 0;  // kernel launches in one replay of the step graph

@@ -237,9 +237,10 @@ class Solver:
     def set_tuning(self, precision, n_max, variant):
         self._check(self.lib.fkg_set_tuning(self.ctx, _lib.PREC[precision], int(n_max), int(variant)), "fkg_set_tuning")
 
-    def set_tuning_chains(self, n_max, variant):
-        """Mixed path, reduction of the resident chains for orders up to n_max: 0 one-stage, 1 two-stage, -1 as solves."""
-        self._check(self.lib.fkg_set_tuning_chains(self.ctx, int(n_max), int(variant)), "fkg_set_tuning_chains")
+    def set_tuning_chains(self, n_max, most):
+        """Mixed path, orders up to n_max: batches of at most `most` resident chains are reduced in one stage, larger
+        ones in two; -1: as set_tuning says."""
+        self._check(self.lib.fkg_set_tuning_chains(self.ctx, int(n_max), int(most)), "fkg_set_tuning_chains")
 
     def set_tuning_back(self, n_max, variant):
         """Back-transformation kernel of the mixed path for orders up to n_max: 0 mma.sync, 1 tcgen05, -1 default."""

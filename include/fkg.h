@@ -237,10 +237,11 @@ int fkg_set_tuning(fkg_ctx* ctx, int precision, int n_max, int variant);
 
 /* Reduction of the device-resident chains (fkg_chains_init and the proposal
  * steps: eigenvalues only) on the mixed path for matrices of order up to n_max
- * (size buckets of 64): 0 = one-stage, 1 = two-stage; -1 (the default, and what
+ * (size buckets of 64): one-stage for batches of at most `most` chains (several
+ * SMs share a chain), two-stage for larger ones; -1 (the default, and what
  * fkg_set_tuning restores for its bucket) = as fkg_set_tuning says. A batch is
  * two-stage only if every chain's bucket selects it. Written by the autotuner. */
-int fkg_set_tuning_chains(fkg_ctx* ctx, int n_max, int variant);
+int fkg_set_tuning_chains(fkg_ctx* ctx, int n_max, int most);
 
 /* Back-transformation kernel of the mixed path for matrices of order up to
  * n_max (size buckets of 64): 0 = mma.sync 3xTF32 with the column block of Z

@@ -42,8 +42,9 @@ def test_chains_can_be_set_apart(solver):
     init = lambda: s.chains_init(ids, f, 2.0, 1.0, 1.0, 4.0)
     init()
     one_solve, one_step, one_init, dl = _launches(s, solve), _launches(s, step), _launches(s, init), step()[1]
-    for solves, chains, more_solve, more_step in [(3, None, 2, 2), (3, 0, 2, 0), (3, -1, 2, 2), (1, None, 0, 0),
-                                                  (1, 1, 0, 2), (3, None, 2, 2), (-1, None, 0, 0)]:
+    for solves, chains, more_solve, more_step in [(3, None, 2, 2), (3, 2, 2, 0), (3, 1, 2, 2), (3, -1, 2, 2),
+                                                  (1, None, 0, 0), (1, 0, 0, 2), (1, 100, 0, 0), (3, None, 2, 2),
+                                                  (-1, None, 0, 0)]:  # two chains
         s.set_tuning("mixed", 81, solves)  # takes the chains' bucket back to its own choice
         if chains is not None:
             s.set_tuning_chains(81, chains)
@@ -56,6 +57,6 @@ def test_chains_can_be_set_apart(solver):
 
 def test_chains_setting_rejects_what_it_does_not_know(solver):
     from fk_mc_gb300._lib import FkgError
-    for n_max, v in [(0, 0), (1025, 0), (64, 2), (64, -2)]:
+    for n_max, v in [(0, 0), (1025, 0), (64, -2)]:
         with pytest.raises(FkgError, match="FKG_ERR_ARG"):
             solver.set_tuning_chains(n_max, v)
