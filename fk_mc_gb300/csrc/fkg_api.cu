@@ -241,12 +241,11 @@ int enqueue_solve(fkg_ctx* ctx, Workspace& ws, const Layout& L, bool want_exp, c
     } else {
         if (!ws.A32.p || !ws.Z.p || !ws.Tf.p || !ws.VT.p || !ws.zsc.p || !ws.Q2.p || !ws.S1.p)
             return set_err(ctx, FKG_ERR_STATE, "mixed workspace not allocated");
-        // FP32 eigenvectors that leave the library keep the rounding of the kernels they have always come from:
-        // the two-stage reduction where every chain is in the class above 960 and a table is set for it, else
-        // sytrd_v3 (any other order of summation moves dF/dU by the path's own error, 1e-7). Values-only solves
-        // take the faster sytrd_cluster kernel: 256 chains of N = 576 9.9 -> 7.9 ms, 16 of N = 1024 14.9 -> 7.2.
+        // The setting decides between one and two stages. One-stage solves whose FP32 eigenvectors leave the library
+        // keep sytrd_v3's rounding (another order of summation moves dF/dU by the path's own error, 1e-7); values-only
+        // ones take the faster sytrd_cluster kernel: 256 chains of N = 576 9.9 -> 7.9 ms, 16 of N = 1024 14.9 -> 6.6.
         const int variant = pick_variant(ctx, L, true, &ws == &ctx->chain);
-        two_stage = variant == kTwoStageVariant || (want_q && L.min_n > 960 && ctx->tune_f32[16] >= 0);
+        two_stage = variant == kTwoStageVariant;
         if (two_stage) {
             const int rc = upload_tensor_maps(ctx, ws, L);
             if (rc) return rc;
@@ -263,8 +262,8 @@ int enqueue_solve(fkg_ctx* ctx, Workspace& ws, const Layout& L, bool want_exp, c
             if (want_q)
                 FKG_CUDA(ctx, launch_sytrd_v3_f32(dd, L.batch, L.max_ld, (const double*)ws.diag.p, (float*)ws.A32.p,
                                                   (double*)ws.d.p, (double*)ws.e.p, (float*)ws.aux32.p, ctx->st,
-                                                  L.max_n > 960 ? 1 : variant, (const int*)ws.order.p,
-                                                  (int*)ws.counter.p, ctx->num_sms, (int*)ctx->status.p));
+                                                  variant, (const int*)ws.order.p, (int*)ws.counter.p, ctx->num_sms,
+                                                  (int*)ctx->status.p));
             else
                 FKG_CUDA(ctx, launch_sytrd_f32(L.desc.data(), dd, L.batch, L.max_ld, (const double*)ws.diag.p,
                                                (float*)ws.A32.p, ws.VT.p /* written by larft later */,

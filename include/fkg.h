@@ -229,9 +229,9 @@ int fkg_set_stream(fkg_ctx* ctx, void* cuda_stream);
  * (FKG_PREC_MIXED) or {2, 4} (FKG_PREC_F64); FKG_PREC_MIXED 3 selects the
  * two-stage reduction; -1 restores the default. On the mixed path the widths
  * apply to solves whose eigenvectors are used (gradients, measures,
- * eigenvectors); values-only solves have one one-stage reduction. Such solves
- * take the two-stage reduction where every order is above 960 and a variant is
- * set there, and width 8 in a batch that holds other orders too.
+ * eigenvectors); values-only solves have one one-stage reduction. The setting of
+ * the bucket with most of a batch's work holds; two-stage only if every chain's
+ * bucket selects it (else width 8).
  * Written by the autotuner (fk_mc_gb300/autotune.py) from measured times. */
 int fkg_set_tuning(fkg_ctx* ctx, int precision, int n_max, int variant);
 

@@ -60,3 +60,46 @@ def test_chains_setting_rejects_what_it_does_not_know(solver):
     for n_max, v in [(0, 0), (1025, 0), (64, -2)]:
         with pytest.raises(FkgError, match="FKG_ERR_ARG"):
             solver.set_tuning_chains(n_max, v)
+
+
+def test_shipped_table_by_size_and_kind(cuda_ok, fkg_lib):
+    """With the shipped table: solves of chains that are all above 960 take two stages, with eigenvectors or without;
+    solves of an uneven batch one; two resident chains of N = 1024 one (their entry's number of chains is above two)."""
+    import fk_mc_gb300
+    s = fk_mc_gb300.Solver(max_n=1024, max_batch=2, precision="mixed")
+    s.set_graphs(False)
+    launches = {}
+    for name, sizes in (("uniform", (32, 32)), ("uneven", (32, 12))):
+        ns = _lattices(s, *sizes)
+        f = np.random.default_rng(1).integers(0, 2, sum(ns))
+        launches["values", name] = _launches(s, lambda: s.eigh_logz([0, 1], _diag(ns), 4.0))
+        launches["vectors", name] = _launches(s, lambda: s.free_energy_grad([0, 1], f, 2.0, 1.0, 1.0, 4.0))
+        launches["chains", name] = _launches(s, lambda: s.chains_init([0, 1], f, 2.0, 1.0, 1.0, 4.0))
+    s.close()
+    assert launches["values", "uniform"] == launches["values", "uneven"] + 2, launches
+    assert launches["vectors", "uniform"] == launches["vectors", "uneven"] + 2, launches
+    assert launches["chains", "uniform"] == launches["chains", "uneven"], launches
+
+
+@pytest.mark.parametrize("sizes", [(32, 32), (32, 12)])
+def test_settings_hold_for_vector_solves_above_960(solver, sizes):
+    """Every setting of the bucket above 960 reaches solves with eigenvectors: the two-stage reduction by its
+    launches, the panel widths by their different roundings, all by the free energy's derivative."""
+    s = solver
+    ns = _lattices(s, *sizes)
+    f = np.random.default_rng(2).integers(0, 2, sum(ns))
+    grad = lambda: s.free_energy_grad([0, 1], f, 2.0, 1.0, 1.0, 4.0)
+    two_stage = sizes[0] == sizes[1]
+    res, launches = {}, {}
+    for v in (0, 1, 2, 3):
+        s.set_tuning("mixed", 1024, v)
+        launches[v] = _launches(s, grad)
+        res[v] = grad()["dU"]
+    assert launches[0] == launches[1] == launches[2] == launches[3] - 2 * two_stage, launches
+    for a in range(4):
+        for b in range(a):
+            if two_stage or a < 3:  # width 8 where two stages are not for every chain
+                assert not np.array_equal(res[a], res[b]), (a, b)
+            assert np.allclose(res[a], res[b], rtol=1e-5, atol=0), (a, b)
+    if not two_stage:
+        assert np.array_equal(res[3], res[1])
