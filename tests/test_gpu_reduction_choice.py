@@ -103,3 +103,47 @@ def test_settings_hold_for_vector_solves_above_960(solver, sizes):
             assert np.allclose(res[a], res[b], rtol=1e-5, atol=0), (a, b)
     if not two_stage:
         assert np.array_equal(res[3], res[1])
+
+
+@pytest.mark.parametrize("variant", [0, 1, 2, 3])
+@pytest.mark.parametrize("L", [5, 10, 20, 31])
+def test_every_variant_of_a_solve_with_vectors(solver, L, variant):
+    """Eigenvalues to 1e-9 ||H||, residuals to 1e-5 ||H|| (the mixed path's stated accuracy) with every panel width and
+    the two-stage reduction."""
+    from fk_mc_gb300.lattice import dense
+    s = solver
+    ns = _lattices(s, L, L)
+    n = ns[0]
+    s.set_tuning("mixed", n, variant)
+    d = _diag(ns, L)
+    out = s.eigh_logz([0, 1], d, 4.0, vectors=True)
+    for c in range(2):
+        A = dense("cubic2d", L) + np.diag(d[c * n:(c + 1) * n])
+        w, X = out["evals"][c * n:(c + 1) * n], out["evecs"][c]
+        norm = np.abs(A).sum(1).max()
+        assert np.abs(w - np.linalg.eigvalsh(A)).max() <= 1e-9 * norm
+        assert np.abs(A @ X - X * w).max() <= 1e-5 * norm
+
+
+@pytest.mark.parametrize("variant", [0, 1])
+@pytest.mark.parametrize("n,B", [(129, 153), (200, 165), (353, 170), (384, 153), (385, 3)])
+def test_both_panel_widths_in_large_fp64_batches(cuda_ok, fkg_lib, n, B, variant):
+    """More chains than SMs take the kernel of 4 warps up to n = 384. Bound 8 n eps ||H||_inf, as a backward-stable
+    reduction and LAPACK's leave together."""
+    import fk_mc_gb300
+    s = fk_mc_gb300.Solver(max_n=n, max_batch=B, precision="f64", tuning=None)
+    i = np.arange(n)
+    H = np.zeros((n, n))
+    for step in (1, 11):
+        H[i, (i + step) % n] -= 1.0
+        H[(i + step) % n, i] -= 1.0
+    nz = H != 0
+    s.set_hopping(0, np.concatenate([[0], np.cumsum(nz.sum(1))]).astype(np.int32), np.nonzero(nz)[1].astype(np.int32),
+                  H[nz])
+    s.set_tuning("f64", n, variant)
+    d = np.random.default_rng(n).uniform(-2, 2, (B, n))
+    w = s.eigh_logz(np.zeros(B, np.int32), d.ravel(), 1.5)["evals"].reshape(B, n)
+    s.close()
+    for c in sorted({0, B // 2, B - 1}):
+        A = H + np.diag(d[c])
+        assert np.abs(w[c] - np.linalg.eigvalsh(A)).max() <= 8 * n * np.finfo(float).eps * np.abs(A).sum(1).max(), c
