@@ -94,11 +94,20 @@ __device__ __forceinline__ T reduce_scatter(T (&x)[VN], int lane, int& idx) {
     return x[0];
 }
 
+// time of a column in k cycles, see launch_cluster: base, per row, per tile of a CTA's mean share and per tile of it in
+// global memory, for a cluster's barriers and for each CTA beyond the first; its relative increase for each further CTA
+// on an SM
+struct ColumnCost {
+    double base, row, tile, spill, cluster, cta, shared;
+};
+
 // W warps a CTA; four CTAs of 4 warps, two of 8 or one of 16 share an SM
 template <int W>
 struct F32 {
     static constexpr int kWarps = W, kOcc = 16 / W;
-    static constexpr double kBase = 6.0, kPerRow = 0.0035, kPerTile = 0.115;  // column time, see launch_cluster
+    static constexpr ColumnCost kCost = W == 4   ? ColumnCost{3.99, 0.0, 0.398, 0.0, 1.25, 0.214, 0.15}
+                                        : W == 8 ? ColumnCost{4.72, 0.00248, 0.080, 0.095, 0.70, 0.139, 0.15}
+                                                 : ColumnCost{5.23, 0.00152, 0.095, 0.041, 0.93, 0.166, 0.15};
     using V = float;  // matrix / vector entry
     using S = float;  // sum
     using G = float;  // reflectors in global memory
@@ -134,7 +143,7 @@ struct F32 {
 template <int LO, int W>
 struct Fix {
     static constexpr int kWarps = W, kOcc = 8 / W;
-    static constexpr double kBase = 8.8, kPerRow = 0.0034, kPerTile = 0.68;
+    static constexpr ColumnCost kCost = {8.8, 0.0034, 0.68, 0.0, 0.8, 0.0, 0.0};
     static constexpr int kLo = LO;
     using V = int2;  // (hi, lo)
     using S = ll;
@@ -921,17 +930,18 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
 
 }  // namespace
 
-// Cluster size (any of 1 .. 8) and grid of a launch. The time of one chain's column was fitted
-// on the GPU (N = 64 .. 1024, one chain per cluster) as P::kBase + P::kPerRow n
-// + P::kPerTile times a CTA's mean share of tiles (a third of the chain's over
-// C), +0.8 for the cluster barriers, in k cycles; `fit` clusters run at once
-// (152, 76, 36, 15 for C = 1, 2, 4, 8). Measured ms behind the choice (C = 1, 2,
-// 4, 8), FP64 path: 256 chains of N = 576 30.4, 34.2, 46.6, 85; 16 chains 13.8, 8.6,
-// 5.9, 9.5 (two rounds); one chain of N = 343 4.2, 3.0, 2.4, 2.1. FP32: 256 chains
-// of N = 576 7.9, 12.8, 21.3, 47.6; 16 chains of N = 1024 15.3, 10.1, 7.4, 12.7.
+// Cluster size (any of 1 .. 8) and grid of a launch. The time of one chain's column was fitted on the GPU (one chain
+// per cluster) as P::kCost has it: FP64 over N = 64 .. 1024; FP32 for each number of warps over N = 130 .. 1024 and C = 1
+// .. 8, 2 % rms, and two CTAs on an SM 14 .. 24 % slower than one (one set for all warps took C = 8 where 1 or 4 is better: 32 chains of N = 216 0.86 -> 0.70 ms, one of
+// N = 256 0.94 -> 0.88). `fit` clusters run at once (152, 76, 36, 15 for C = 1, 2, 4, 8). Measured ms behind the choice (C =
+// 1, 2, 4, 8), FP64 path: 256 chains of N = 576 30.4, 34.2, 46.6, 85; 16 chains 13.8, 8.6, 5.9, 9.5 (two rounds); one
+// chain of N = 343 4.2, 3.0, 2.4, 2.1. FP32: 256 chains of N = 576 7.9, 12.8, 21.3, 47.6; 16 chains of N = 1024 15.3, 10.1,
+// 7.4, 12.7.
 template <class P>
-static double cluster_cost(int n, int nt, int C) {
-    return n * (P::kBase + P::kPerRow * n + (C > 1 ? 0.8 : 0.0) + P::kPerTile * (nt * (nt + 1) / 2) / (3.0 * C));
+static double cluster_cost(int n, int nt, int C, int cap) {
+    constexpr ColumnCost k = P::kCost;
+    const double share = nt * (nt + 1) / 2 / (3.0 * C), spilled = max(0, slots_of(nt, C) - cap) / 3.0;
+    return n * (k.base + k.row * n + k.tile * share + k.spill * spilled + (C > 1 ? k.cluster + k.cta * (C - 1) : 0.0));
 }
 
 template <class P, int NB>
@@ -967,13 +977,17 @@ static cudaError_t launch_cluster(const ChainDesc* h_desc, const ChainDesc* d_de
         if (d_order) {
             double sum = 0.0, mx = 0.0, mn = 1e300;
             for (int c = 0; c < batch; ++c) {
-                const double t = cluster_cost<P>(h_desc[c].n, h_desc[c].ld / kTile, C);
+                const double t = cluster_cost<P>(h_desc[c].n, h_desc[c].ld / kTile, C, cap);
                 sum += t;
                 mx = max(mx, t);
                 mn = min(mn, t);
             }
             // equal chains run in whole rounds, uneven ones (longest first) end within about half the longest
-            auto total = [&](int f) { return mn == mx ? mx * ((batch + f - 1) / f) : max(mx, sum / f + 0.5 * mx); };
+            auto total = [&](int f) {
+                const int ctas = (min(batch, f) * P::kOcc + f - 1) / f;  // on the fullest SM
+                return (mn == mx ? mx * ((batch + f - 1) / f) : max(mx, sum / f + 0.5 * mx)) *
+                       (1.0 + P::kCost.shared * (ctas - 1));
+            };
             if (best_C && total(max(1, num_sms * P::kOcc / C)) >= best) continue;
             if ((err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))) return err;
             at.val.clusterDim.x = C;

@@ -147,3 +147,24 @@ def test_both_panel_widths_in_large_fp64_batches(cuda_ok, fkg_lib, n, B, variant
     for c in sorted({0, B // 2, B - 1}):
         A = H + np.diag(d[c])
         assert np.abs(w[c] - np.linalg.eigvalsh(A)).max() <= 8 * n * np.finfo(float).eps * np.abs(A).sum(1).max(), c
+
+
+@pytest.mark.parametrize("n,B", [(200, 24), (216, 32), (240, 100), (256, 24), (256, 48), (256, 152)])
+def test_values_reduce_no_slower_than_vectors(cuda_ok, fkg_lib, n, B):
+    """The cluster kernel's size per chain is chosen by a fitted time: at every order and number of chains it must not
+    be slower than the one-CTA kernel that solves with vectors keep (5 % for the clock's noise)."""
+    import fk_mc_gb300
+    s = fk_mc_gb300.Solver(max_n=n, max_batch=B, precision="mixed", tuning=None)
+    s.set_lattice(0, "cubic1d", n)
+    f, ids = np.random.default_rng(n).integers(0, 2, (B, n)), np.zeros(B, np.int32)
+    ms = []
+    for call in (lambda: s.eigh_logz(ids, (2.0 * f - 1.0).ravel(), 4.0),
+                 lambda: s.free_energy_grad(ids, f.ravel(), 2.0, 1.0, 1.0, 4.0)):
+        call()
+        s.profile(True)
+        for _ in range(5):
+            call()
+        ms.append(s.stage_time("reduce")[0])
+        s.profile(False)
+    s.close()
+    assert ms[0] <= 1.05 * ms[1], ms
