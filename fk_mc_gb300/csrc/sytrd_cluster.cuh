@@ -952,7 +952,9 @@ static cudaError_t launch_cluster(const ChainDesc* h_desc, const ChainDesc* d_de
     if (batch <= 0) return cudaSuccess;
     auto* kern = sytrd_cluster_kernel<P, NB>;
     const size_t tile_bytes = sizeof(typename P::V) * kTileElems, limit = 226 * 1024 / P::kOcc;
-    cudaError_t err;
+    // the attribute belongs to the process: one value, whatever another thread's context launches meanwhile
+    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
+    if (err != cudaSuccess) return err;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeClusterDimension;
@@ -989,7 +991,6 @@ static cudaError_t launch_cluster(const ChainDesc* h_desc, const ChainDesc* d_de
                        (1.0 + P::kCost.shared * (ctas - 1));
             };
             if (best_C && total(max(1, num_sms * P::kOcc / C)) >= best) continue;
-            if ((err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))) return err;
             at.val.clusterDim.x = C;
             cfg.gridDim = dim3(batch * C);
             cfg.dynamicSmemBytes = smem;
@@ -1006,7 +1007,6 @@ static cudaError_t launch_cluster(const ChainDesc* h_desc, const ChainDesc* d_de
         best_smem = smem;
     }
     if (!best_C) return cudaErrorInvalidValue;
-    if ((err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)best_smem))) return err;
     if (d_order && (err = cudaMemsetAsync(d_counter, 0, sizeof(int), st))) return err;
     at.val.clusterDim.x = best_C;
     cfg.gridDim = dim3(min(batch, best_fit) * best_C);

@@ -100,3 +100,29 @@ def test_scale_at_a_rounding_edge(solver, n, B):
     for _ in range(10):
         w = solver.eigh_logz(np.zeros(B, np.int32), np.tile(d, B), 1.5)["evals"].reshape(B, n)
         assert np.abs(w - ref).max() <= 8 * n * EPS * np.abs(H + np.diag(d)).sum(1).max()
+
+
+def test_two_threads_with_contexts_of_different_size(cuda_ok, fkg_lib):
+    """Launches of one kernel with different shared memory from two threads: neither changes the other's limit."""
+    import threading
+    import fk_mc_gb300
+    errors = []
+
+    def work(L, B, seed):
+        try:
+            s = fk_mc_gb300.Solver(max_n=L * L, max_batch=B, precision="f64")
+            n = s.set_lattice(0, "cubic2d", L)
+            d = np.random.default_rng(seed).uniform(-2, 2, B * n)
+            first = s.eigh_logz(np.zeros(B, np.int32), d, 2.0)["evals"]
+            for _ in range(60):
+                assert np.array_equal(s.eigh_logz(np.zeros(B, np.int32), d, 2.0)["evals"], first)
+            s.close()
+        except Exception as e:  # noqa: BLE001 - reported below
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=a) for a in ((12, 1, 1), (23, 2, 2), (15, 9, 3))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
