@@ -455,7 +455,8 @@ sytrd_cluster_kernel(const ChainDesc* __restrict__ descs, const double* __restri
                     if (tid == 0 && status) atomicOr(status, kStatusNaN);
 #pragma unroll 1
                     for (int i = tid; i < n; i += kThreads) {
-                        dout[D.v_off + i] = eout[D.v_off + i] = 0.0;
+                        dout[D.v_off + i] = NAN;  // and so every eigenvalue and logZ
+                        eout[D.v_off + i] = 0.0;
                         tauout[D.v_off + i] = 0;
                     }
                 }

@@ -81,7 +81,8 @@ sytrd_small_kernel(const ChainDesc* __restrict__ descs, const double* __restrict
         if (__syncthreads_or(bad)) {  // NaN, Inf or out of the format's range
             if (tid == 0 && status) atomicOr(status, kStatusNaN);
             for (int i = tid; i < n; i += kThreads) {
-                dout[D.v_off + i] = eout[D.v_off + i] = 0.0;
+                dout[D.v_off + i] = NAN;  // and so every eigenvalue and logZ
+                eout[D.v_off + i] = 0.0;
                 tauout[D.v_off + i] = 0;
             }
             return;

@@ -655,6 +655,10 @@ trieig_values_kernel(const ChainDesc* __restrict__ descs, const double* __restri
     if (threadIdx.x == 0) cnt = 0;
     const int j = blockIdx.y * blockDim.x + threadIdx.x;
     const bool active = j < n;
+    if (S.d[0] != S.d[0]) {  // a chain that the reduction rejected
+        if (active) ww[D.v_off + j] = NAN;
+        return;
+    }
     float lo = 0.f, hi = 0.f;
     block_brackets(S, n, j, active, B, lo, hi);
     double lgap, rgap;
