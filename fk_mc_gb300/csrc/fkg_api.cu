@@ -225,14 +225,15 @@ int enqueue_solve(fkg_ctx* ctx, Workspace& ws, const Layout& L, bool want_exp, c
     double* A = (double*)ws.A.p;
     bool two_stage = false;
     if (ctx->precision == FKG_PREC_F64) {
-        // with eigenvectors A holds the reflectors, else the tiles beyond shared memory
+        // the tiles beyond shared memory: in A, or, with eigenvectors, whose reflectors A holds, in the eigenvectors' own
+        // buffer, which inverse iteration fills later
         if (want_q) {
-            const int rc = ensure_dev(ctx, ws.tiles, sizeof(double) * (size_t)L.a_total);
+            const int rc = ensure_dev(ctx, ws.Z64, sizeof(double) * (size_t)L.a_total);
             if (rc) return rc;
         }
         stage_begin(ctx, FKG_STAGE_REDUCE);
         FKG_CUDA(ctx, launch_sytrd_f64(L.desc.data(), dd, L.batch, L.max_ld, (const double*)ws.diag.p,
-                                       want_q ? A : nullptr, want_q ? ws.tiles.p : ws.A.p, (double*)ws.d.p,
+                                       want_q ? A : nullptr, want_q ? ws.Z64.p : ws.A.p, (double*)ws.d.p,
                                        (double*)ws.e.p, (double*)ws.tau.p, ctx->st, pick_variant(ctx, L, false),
                                        (const int*)ws.order.p, (int*)ws.counter.p, ctx->num_sms,
                                        (int*)ctx->status.p));
