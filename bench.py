@@ -18,8 +18,8 @@ roofline of the dominant kernel (the Householder reduction: W_fwd = 4/3 N^3
 flops per proposal times the chains of one launch, over the launch's
 CUDA-event duration, against the measured dense bf16 tensor peak of
 MEASURED_PEAKS.json; DRAM traffic per launch from the committed ncu capture),
-with the other views of the same kernels (nominal FP32 / FP64 pipe rates, the
-one-stage algorithm's matrix re-reads against HBM) as labelled context; the CPU
+with the other views of the same kernels (nominal FP32 / FP64 pipe rates) as
+labelled context; the CPU
 baseline (the oracle restatement of the reference path on all host cores);
 `chebyshev`: the same chains and proposals with logZ from the reference's
 Chebyshev expansion (cheb_moves; int(log N * 2.2) moments) instead of the
@@ -59,12 +59,6 @@ METRIC = "MC proposals/s at N=576: mixed+batched vs plain FP64 on GB300; dF erro
 NOMINAL_TFLOPS = {"fp32_fma": 152 * 128 * 2 * 2.07e9 / 1e12, "fp64": 1.25, "tf32_dense": 1100.0}
 W_FWD = 4.0 / 3.0 * N ** 3      # Householder tridiagonalisation flops per proposal
 W_BT = 2.0 * N ** 3              # back-transformation X = Q Z flops per proposal
-NB32 = 4                         # panel width of the FP32 reduction at N = 576
-# Compulsory matrix bytes of one FP32 reduction: the lower triangle of the
-# m x m trailing matrix read by the matrix-vector product of every column, and
-# read + written by the rank-2k update after every panel of NB32 columns.
-A_BYTES = 4.0 * (sum(m * (m + 1) / 2 for m in range(2, N))
-                 + sum(2 * m * (m + 1) / 2 for m in range(N - NB32, 2, -NB32)))
 
 
 def parse():
@@ -184,8 +178,8 @@ def roofline(res, head, B):
     algorithmic work of one launch (W_fwd = 4/3 N^3 flops per chain, B chains) over its mean CUDA-event
     duration (stage timers on the library's stream), against the dense bf16 tensor peak of
     MEASURED_PEAKS.json (the sustained figure: the kernel is timed inside a run of many steps). The
-    other views are context: the same kernels against the nominal FP32 / FP64 pipe rates, the one-stage
-    reduction's matrix re-reads against HBM, the back-transformation's FP32-equivalent rate."""
+    other views are context: the same kernels against the nominal FP32 / FP64 pipe rates, the
+    back-transformation's FP32-equivalent rate."""
     pk = measured_peaks()
     peak = pk["bf16_tflops_sustained"]
     hr = res[head]
@@ -207,11 +201,6 @@ def roofline(res, head, B):
         other.append({"kernel": roof["kernel"], "view": f"against the nominal {pipe} pipe rate (not measured)",
                       "achieved": achieved, "peak": NOMINAL_TFLOPS[pipe], "unit": "TFLOP/s",
                       "frac": achieved / NOMINAL_TFLOPS[pipe]})
-        if f32:
-            other.append({"kernel": roof["kernel"], "view": "one-stage reduction's own matrix re-reads (every "
-                          "column's matrix-vector product plus the rank-2k update per panel) against HBM; not "
-                          "compulsory traffic", "achieved": A_BYTES * B / red_s / 1e9, "peak": pk["hbm_gbs"],
-                          "unit": "GB/s", "frac": A_BYTES * B / red_s / 1e9 / pk["hbm_gbs"]})
     if "f64" in res and head != "f64":
         m, n = res["f64"]["stages"]["reduce"]
         if n:

@@ -133,9 +133,11 @@ __device__ __forceinline__ double scale_down(double x, int k) {
 // inside the factorisation, reciprocals take the hardware's approximation and one third-order step, comparisons and
 // the scaling between solves (by powers of two) are integer work. Rows are stored [i][vector] (coalesced) and read
 // four ahead.
+// A cluster's members follow one another on the lane that leads it; their orthogonalisation is the whole warp's.
 // Measured (one thread's rows apart, branches, divisions and sines before): 32 chains of N = 225 1.41 -> 0.45 ms,
-// 256 of N = 576 27.6 -> 6.5 ms, one of N = 64 0.31 -> 0.11 ms.
-__global__ void __launch_bounds__(32)
+// 256 of N = 576 27.4 -> 6.0 ms, one of N = 64 0.31 -> 0.11 ms; clusters of 4, 8 and 30 (64 chains of N = 256 without f)
+// 57 -> 17 ms, 54 with the leading lane orthogonalising.
+__global__ void __launch_bounds__(32, 16)  // 12 CTAs an SM (168 registers): 7.3 ms
 stein_kernel(const ChainDesc* __restrict__ descs, const double* __restrict__ dd, const double* __restrict__ ee,
              const double* __restrict__ ww, double* __restrict__ Zws, double* __restrict__ scratch) {
     extern __shared__ double2 de[];  // d_i, e_i
