@@ -19,10 +19,13 @@
 //        power of two above the largest row sum of |H| (so ||H||_2 <= S), held as
 //        two limbs x = hi 2^LO + lo (hi 32 bits, |lo| <= 2^(LO - 1); formats at
 //        struct Fix). A product is three integer multiplications: hi hi into one
-//        64-bit sum, hi lo + lo hi into another; lo lo is dropped. Every sum is
+//        64-bit sum, hi lo + lo hi into another; lo lo is dropped. The sums are
 //        exact: the results are bounded by the norms (|A v| <= sqrt(2) S, |w| <=
 //        2 S, the cross sums by sqrt(n) times the limbs' ranges), and
-//        intermediate wrap-around modulo 2^64 is harmless. Orthogonal
+//        intermediate wrap-around modulo 2^64 is harmless. Where a partial sum leaves
+//        its lane its cross sum is rounded to the other's unit, so a result's last bits
+//        depend on how many warps and CTAs share the chain (but not on their timing).
+//        Orthogonal
 //        transformations keep ||A||_2, so no entry outgrows its format. The
 //        rounding is half a quantum per entry and panel where FP64 rounds every
 //        product; the norm of a column is an exact integer sum,

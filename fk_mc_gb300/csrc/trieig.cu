@@ -494,16 +494,19 @@ __device__ bool shift_df(const float* d, const float* e2h, const float* e2l, int
     return false;
 }
 
-// The listed eigenvalues in FP64, packed onto the first warps: a warp's FP64
-// instruction costs the narrow pipe the same for one lane as for 32, so a warp
-// works on up to 32 eigenvalues at once, and on fewer with more lanes each. The
-// spectra of ordered configurations are all multiplets and all of them listed:
-// 256 chains of the N = 576 checkerboard 243 ms with a warp per eigenvalue.
+// The listed eigenvalues in FP64. A warp's FP64 instruction costs the narrow pipe
+// the same for one lane as for 32, so eigenvalues share a warp: in ordered
+// configurations all of them belong to multiplets and are listed, and a warp for
+// each took 243 ms for 256 checkerboards of N = 576 (37 now). A short list gets
+// more lanes an eigenvalue, whose rounds are fewer (32 lanes 7, 4 lanes 15, one 35), as
+// far as two warps reach (128 chains of cubic3d L = 8 with 5 % defects 8.9 ms with one
+// warp, 9.3 with two, 9.9 with four; 64 of cubic1d L = 343 1.28, 1.10, 0.98). The number of
+// lanes changes an eigenvalue's last bits, so it depends on nothing but the list.
 __device__ void list64(const ChainDesc& D, const TriShared& S, int n, const TriBounds& B, int count, const int* list,
                        const float* lbr, double* __restrict__ ww, int* __restrict__ status) {
     if (count == 0) return;
     int p = 1;
-    while (2 * p * count <= 32) p *= 2;
+    while (p < 32 && 2 * p * count <= 64) p *= 2;
     if ((int)(threadIdx.x & ~31u) / p >= count) return;  // nothing for this warp
     const int q = threadIdx.x / p, i = min(q, count - 1);
     const double lam = refine64_group(S, n, list[i], B, lbr[2 * i], lbr[2 * i + 1], p, q < count, status);
