@@ -1,10 +1,9 @@
 // sytrd_v3.cu — blocked Householder tridiagonalisation in FP32, one CTA per
 // chain: the mixed path's reduction where FP32 eigenvectors leave the library
-// (gradients, measures, eigenvectors). Values-only solves use the faster
-// sytrd_cluster.cuh; its other order of summation would change every output
-// that is computed from the FP32 vectors by the path's own error (1e-7 of
-// dF/dU), so those solves keep this kernel's rounding (and the two-stage one's where
-// every chain is above n = 960).
+// (gradients, measures, eigenvectors) and the settings do not ask for two stages.
+// Values-only solves use the faster sytrd_cluster.cuh; its other order of summation
+// would change every output that is computed from the FP32 vectors by the path's own
+// error (1e-7 of dF/dU), so those solves keep this kernel's rounding.
 //
 // Replaces the first half of Eigen::SelfAdjointEigenSolver at
 // src/configuration.cpp:213; the Hamiltonian build (src/configuration.cpp:79-91)

@@ -502,7 +502,9 @@ __device__ bool shift_df(const float* d, const float* e2h, const float* e2l, int
 // far as two warps reach (128 chains of cubic3d L = 8 with 5 % defects 8.9 ms with one
 // warp, 9.3 with two, 9.9 with four; 64 of cubic1d L = 343 1.28, 1.10, 0.98). The number of
 // lanes changes an eigenvalue's last bits, so it depends on nothing but the list.
-__device__ void list64(const ChainDesc& D, const TriShared& S, int n, const TriBounds& B, int count, const int* list,
+// A function of its own, as last_step, with its arguments by value: inlined, they
+// cost the kernels' FP32 recurrences 5 % (16 chains of N = 576 0.505 -> 0.480 ms mixed).
+__device__ __noinline__ void list64(const ChainDesc D, const TriShared S, int n, const TriBounds B, int count, const int* list,
                        const float* lbr, double* __restrict__ ww, int* __restrict__ status) {
     if (count == 0) return;
     int p = 1;
@@ -610,7 +612,7 @@ __device__ __forceinline__ double charpoly_value(const double* __restrict__ d, c
 // (at most 12 of these 16 seen over disordered rings up to n = 900, 0.1 usually).
 // Where the step times that is not below eps ||T|| / 2, one more evaluation and
 // the secant's slope give a second step. False when the steps cannot be trusted.
-__device__ bool last_step(const TriShared& S, int n, const TriBounds& B, double x, double dp, int edp, double gap,
+__device__ __noinline__ bool last_step(const TriShared S, int n, const TriBounds B, double x, double dp, int edp, double gap,
                           double& lam) {
     double p0 = 0.0, step = 0.0;
     int e0 = 0;

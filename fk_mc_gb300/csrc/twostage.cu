@@ -3,7 +3,7 @@
 // the back-transformation. The first stage (dense -> band) is sy2sb.cu.
 //
 // Replaces, with sy2sb.cu, the first half of Eigen::SelfAdjointEigenSolver at
-// src/configuration.cpp:213. The one-stage reduction (sytrd_f32.cu) reads the
+// src/configuration.cpp:213. The one-stage reductions (sytrd_f32.cu, sytrd_v3.cu) read the
 // whole trailing matrix for every column (a matrix-vector product per
 // reflector); the two-stage reduction passes over it once per panel of kBand
 // columns on the tensor cores and leaves O(b n^2) work to the band stage:
