@@ -47,3 +47,20 @@ def test_mean_error_of_the_bounds(cuda_ok, fkg_lib):
             means.append(e.mean())
         s.close()
     assert np.exp(np.mean(np.log(means))) <= 2.0 ** -48, means
+
+
+def test_bounds_of_converged_spectra(cuda_ok, fkg_lib):
+    """The Krylov space of cubic2d L = 8 is exhausted long after its ends have converged; copies of them come up, whose
+    distance is the scalars' rounding. Bound: two roundings of a pair; a twice rounded 1 / beta left 1.3e-14."""
+    import fk_mc_gb300
+    from fk_mc_gb300.lattice import dense
+    B, n = 25, 64
+    s = fk_mc_gb300.Solver(max_n=n, max_batch=B, precision="f64")
+    s.set_lattice(0, "cubic2d", 8)
+    s.set_chebyshev(10, 20)
+    d = 0.5 * (np.random.default_rng(0).integers(0, 2, (B, n)) - 0.5)
+    r = s.chebyshev_logz(np.zeros(B, np.int32), d.ravel(), 5.0)
+    s.close()
+    w = np.array([np.linalg.eigvalsh(dense("cubic2d", 8) + np.diag(x))[[0, -1]] for x in d])
+    assert np.mean(np.abs(r["e_min"] - w[:, 0]) / np.abs(w).max(1)) <= 2.0 * 2.0 ** -48
+    assert np.mean(np.abs(r["e_max"] - w[:, 1]) / np.abs(w).max(1)) <= 2.0 * 2.0 ** -48
