@@ -76,7 +76,6 @@ int make_layout(fkg_ctx* ctx, int batch, const int32_t* lattice_id, Layout& L) {
     L.a_total = 0;
     L.max_n = 0;
     L.max_ld = 0;
-    L.min_n = 1 << 30;
     for (int c = 0; c < batch; ++c) {
         int id = lattice_id[c];
         if (id < 0 || id >= kMaxLattices || ctx->lat[id].n <= 0)
@@ -97,7 +96,6 @@ int make_layout(fkg_ctx* ctx, int batch, const int32_t* lattice_id, Layout& L) {
         L.v_total += d.ld;
         L.n_total += d.n;
         if (d.n > L.max_n) L.max_n = d.n;
-        if (d.n < L.min_n) L.min_n = d.n;
         if (d.ld > L.max_ld) L.max_ld = d.ld;
     }
     L.order.resize(batch);

@@ -68,7 +68,7 @@ struct LatticeDev {
 
 // Host copy of a batch layout.
 struct Layout {
-    int batch = 0, max_n = 0, max_ld = 0, min_n = 0;
+    int batch = 0, max_n = 0, max_ld = 0;
     long long n_total = 0, v_total = 0, a_total = 0;
     std::vector<ChainDesc> desc;
     std::vector<int> order;  // chain indices by decreasing n (work list of the persistent reduction)
