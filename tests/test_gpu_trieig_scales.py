@@ -54,3 +54,26 @@ def test_time_does_not_depend_on_the_scale(cuda_ok, fkg_lib):
         s.profile(False)
     s.close()
     assert max(ms) <= 2 * ms[0], ms
+
+
+@pytest.mark.parametrize("n,small", [(96, 2.0 ** -20), (300, 2.0 ** -20), (300, 2.0 ** -45)])
+def test_uncoupled_blocks_of_different_scale(cuda_ok, fkg_lib, n, small):
+    """Values to 8 n eps ||H||, residuals of the vectors to the same, and vectors orthonormal to 1e-9 (clusters, into which
+    the small block's values may fall, are orthogonalised)."""
+    import fk_mc_gb300
+    A = np.zeros((n, n))
+    i = np.arange(n // 2 - 1)
+    for o, t in ((0, 1.0), (n // 2, small)):
+        A[o + i, o + i + 1] = A[o + i + 1, o + i] = -t
+    nz = A != 0
+    s = fk_mc_gb300.Solver(max_n=n, max_batch=1, precision="f64")
+    s.set_hopping(0, np.concatenate([[0], np.cumsum(nz.sum(1))]).astype(np.int32), np.nonzero(nz)[1].astype(np.int32),
+                  A[nz])
+    d = np.random.default_rng(n).uniform(-2, 2, n) * np.where(np.arange(n) < n // 2, 1.0, small)
+    out = s.eigh_logz([0], d, 3.0, vectors=True)
+    s.close()
+    A += np.diag(d)
+    w, X, bound = out["evals"], out["evecs"][0], 8 * n * EPS * np.abs(A).sum(1).max()
+    assert np.abs(w - np.linalg.eigvalsh(A)).max() <= bound
+    assert np.abs(A @ X - X * w).max() <= bound
+    assert np.abs(X.T @ X - np.eye(n)).max() <= 1e-9
