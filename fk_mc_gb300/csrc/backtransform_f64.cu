@@ -216,7 +216,7 @@ cudaError_t launch_fix(const ChainDesc* d_desc, int batch, int max_n, const doub
                        double* d_Z, cudaStream_t st) {
     const size_t smem = sizeof(int2) * 2 * 32 * R * kBlk;
     auto* kern = backtransform_fix_kernel<R, W, NC, OCC>;
-    const cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t err = allow_smem<backtransform_fix_kernel<R, W, NC, OCC>>();
     if (err != cudaSuccess) return err;
     kern<<<dim3((max_n + NC * W - 1) / (NC * W), batch), W * 32, smem, st>>>(d_desc, d_A, d_Tf, d_Z);
     return cudaGetLastError();

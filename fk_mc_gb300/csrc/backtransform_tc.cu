@@ -271,7 +271,7 @@ cudaError_t launch_backtransform_tc(const ChainDesc* d_desc, int batch, int max_
     if (batch <= 0) return cudaSuccess;
     if (batch > 65535) return cudaErrorInvalidValue;  // grid y limit
     const size_t smem = backtransform_tc_smem_bytes(max_ld);
-    cudaError_t err = cudaFuncSetAttribute(backtransform_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t err = allow_smem<backtransform_tc_kernel>();
     if (err != cudaSuccess) return err;
     backtransform_tc_kernel<<<dim3((max_n + kNC - 1) / kNC, batch), kTcThreads, smem, st>>>(d_desc, d_VT, plane, d_Z,
                                                                                                 d_zscale, shift);

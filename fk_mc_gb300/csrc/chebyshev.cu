@@ -563,7 +563,7 @@ cudaError_t launch_kpm(const KpmDesc* d_kdesc, int batch, int max_n, int max_ld,
     if (batch > 65535) return cudaErrorInvalidValue;  // grid y limit of the moment kernel
     cudaError_t err;
     const size_t sm_b = sizeof(dfl) * (2 * (size_t)kmax + 4 * (size_t)max_ld);
-    if ((err = cudaFuncSetAttribute(kpm_bounds_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_b))) return err;
+    if ((err = allow_smem<kpm_bounds_kernel>())) return err;
     // the threads that share the rows evenly: 256 for N = 576 left a third of them idle in the last pass, and for
     // N = 144 barriers for warps without rows (512 chains of N = 144 2.61 -> 2.47 ms for three steps)
     const int passes = (max_n + kKpmThreads - 1) / kKpmThreads;
@@ -572,14 +572,14 @@ cudaError_t launch_kpm(const KpmDesc* d_kdesc, int batch, int max_n, int max_ld,
     if ((err = cudaGetLastError())) return err;
     const int wpc = kpm_warps_per_cta(max_bmax);
     const size_t sm_m = kpm_moment_smem_bytes(max_bmax, wpc);
-    if ((err = cudaFuncSetAttribute(kpm_moments_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_m))) return err;
+    if ((err = allow_smem<kpm_moments_kernel>())) return err;
     kpm_moments_kernel<<<dim3((max_n + wpc - 1) / wpc, batch), 32 * wpc, sm_m, st>>>(d_kdesc, d_xdiag, d_xinv, d_part,
                                                                                       wpc);
     if ((err = cudaGetLastError())) return err;
     // moments per block of the T_m table: as many as fit in 64 KB
     const int mblk = max(1, min(M, (int)(8192 / G)));
     const size_t sm_f = sizeof(double) * (3 * (size_t)R + 2 * (size_t)M + (2 + (size_t)mblk) * (size_t)G);
-    if ((err = cudaFuncSetAttribute(kpm_final_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_f))) return err;
+    if ((err = allow_smem<kpm_final_kernel>())) return err;
     kpm_final_kernel<<<batch, kKpmThreads, sm_f, st>>>(d_kdesc, d_part, d_ab, d_beta, M, G, mblk, d_mu, d_logz,
                                                      d_status);
     return cudaGetLastError();

@@ -219,6 +219,17 @@ __device__ __forceinline__ void two_sum(double a, double b, double& s, double& e
 
 // Host-side launch wrappers implemented in the .cu files.
 namespace fkg {
+// Lets a kernel have all the shared memory of an SM. The limit is an attribute of the process: one value for every
+// launch of a kernel, whatever another thread's context launches between this call and the launch.
+template <auto kern>
+cudaError_t allow_smem() {
+    static const size_t fixed = [] {
+        cudaFuncAttributes a{};
+        return cudaFuncGetAttributes(&a, kern) == cudaSuccess ? a.sharedSizeBytes : (size_t)16 * 1024;
+    }();
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024 - fixed));
+}
+
 // Chebyshev-expansion logZ (chebyshev.cu): bounds by Lanczos (at most kmax
 // steps; d_steps, may be null: the steps each chain took), moments of M (even)
 // Chebyshev polynomials on balls of radius R = M/2 (d_part: 3R doubles per

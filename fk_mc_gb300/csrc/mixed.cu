@@ -392,7 +392,7 @@ cudaError_t launch_mixed_refine(const ChainDesc* d_desc, int batch, int max_n, i
     if ((err = cudaEventRecord(ev_join, aux)) != cudaSuccess) return err;
     stage(sctx, 1, 0);
     const size_t sm_tw = (size_t)max_ld * 3 * sizeof(float);
-    if ((err = cudaFuncSetAttribute(twisted_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_tw))) return err;
+    if ((err = allow_smem<twisted_kernel>())) return err;
     twisted_kernel<<<dim3(batch, (max_n + 127) / 128), 128, sm_tw, st>>>(d_desc, d_d, d_e, d_w, d_ctol, d_Z, d_zscale);
     if ((err = cudaGetLastError()) != cudaSuccess) return err;
     stage(sctx, 1, 1);
@@ -412,7 +412,7 @@ cudaError_t launch_mixed_refine(const ChainDesc* d_desc, int batch, int max_n, i
         d_desc, d_Z, d_diag, d_theta);
     if ((err = cudaGetLastError()) != cudaSuccess) return err;
     const size_t sm_s = (sizeof(double) + sizeof(int)) * max_ld;
-    if ((err = cudaFuncSetAttribute(sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_s))) return err;
+    if ((err = allow_smem<sort_kernel>())) return err;
     sort_kernel<<<batch, 128, sm_s, st>>>(d_desc, d_theta, d_w, d_perm, d_status);
     if ((err = cudaGetLastError()) != cudaSuccess) return err;
     stage(sctx, 3, 1);

@@ -372,7 +372,7 @@ cudaError_t launch_rank1(int batch, int n, const double* d_evals, const double* 
                          const double* d_beta, double* d_logz, double* d_ev_out, int* d_status, cudaStream_t st) {
     if (batch <= 0) return cudaSuccess;
     const size_t sm = rank1_smem_bytes(n);
-    cudaError_t e = cudaFuncSetAttribute(rank1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_smem<rank1_kernel>();
     if (e != cudaSuccess) return e;
     // one root per thread and pass, with whole passes where n exceeds a block
     const int passes = (n + kR1MaxThreads - 1) / kR1MaxThreads, threads = ((n + passes - 1) / passes + 31) / 32 * 32;

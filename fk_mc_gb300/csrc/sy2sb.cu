@@ -813,7 +813,7 @@ cudaError_t launch_sy2sb(const ChainDesc* d_desc, int batch, int max_ld, const d
     const size_t smem = sy2sb_smem_bytes(max_ld);
     // three panel rows per thread up to n = 768 (fewer registers held through the QR), four beyond
     auto kern = max_ld <= 3 * kS1Threads ? sy2sb_kernel<3> : sy2sb_kernel<4>;
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t err = max_ld <= 3 * kS1Threads ? allow_smem<sy2sb_kernel<3>>() : allow_smem<sy2sb_kernel<4>>();
     if (err != cudaSuccess) return err;
     // the largest shared-memory configuration: two CTAs per SM
     err = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);

@@ -454,7 +454,7 @@ cudaError_t launch_v3(const ChainDesc* d_desc, int batch, int max_ld, const doub
                       int* d_status) {
     if (batch <= 0) return cudaSuccess;
     const size_t smem = v3_smem<T, NB>(max_ld);
-    cudaError_t err = cudaFuncSetAttribute(sytrd_v3_kernel<T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t err = allow_smem<sytrd_v3_kernel<T, NB>>();
     if (err != cudaSuccess) return err;
     int grid = batch;
     if (d_order) {  // persistent: as many CTAs as fit on the GPU at once

@@ -748,7 +748,7 @@ cudaError_t launch_trieig_shifts(const ChainDesc* d_desc, int batch, int max_n, 
                                  const double* d_e, double* d_w, double* d_ctol, int* d_status, cudaStream_t st) {
     if (batch <= 0) return cudaSuccess;
     const size_t smem = trieig_smem_bytes(max_ld);
-    cudaError_t err = cudaFuncSetAttribute(trieig_shift_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t err = allow_smem<trieig_shift_kernel>();
     if (err != cudaSuccess) return err;
     dim3 grid(batch, (max_n + kEigThreads - 1) / kEigThreads);
     trieig_shift_kernel<<<grid, kEigThreads, smem, st>>>(d_desc, d_d, d_e, d_w, d_ctol, d_status);
@@ -759,7 +759,7 @@ cudaError_t launch_trieig_values(const ChainDesc* d_desc, int batch, int max_n, 
                                  const double* d_e, double* d_w, int* d_status, cudaStream_t st) {
     if (batch <= 0) return cudaSuccess;
     const size_t smem = trieig_smem_bytes(max_ld);
-    cudaError_t err = cudaFuncSetAttribute(trieig_values_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t err = allow_smem<trieig_values_kernel>();
     if (err != cudaSuccess) return err;
     dim3 grid(batch, (max_n + kEigThreads - 1) / kEigThreads);
     trieig_values_kernel<<<grid, kEigThreads, smem, st>>>(d_desc, d_d, d_e, d_w, d_status);

@@ -334,7 +334,7 @@ cudaError_t launch_sb2st(const ChainDesc* d_desc, int batch, int max_n, const fl
                          float* d_Q2, long long q2t_off, cudaStream_t st) {
     if (batch <= 0) return cudaSuccess;
     const size_t smem = sizeof(float) * (size_t)(max_n + kB) * kLdb;
-    cudaError_t err = cudaFuncSetAttribute(sb2st_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t err = allow_smem<sb2st_kernel>();
     if (err != cudaSuccess) return err;
     sb2st_kernel<<<batch, kS2Warps * 32, smem, st>>>(d_desc, d_A, d_d, d_e, d_Q2, q2t_off);
     return cudaGetLastError();

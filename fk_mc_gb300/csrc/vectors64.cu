@@ -498,7 +498,7 @@ cudaError_t launch_cluster_fix_f32(const ChainDesc* d_desc, int batch, int max_l
                                    float* d_zscale, double* d_scratch, cudaStream_t st) {
     if (batch <= 0) return cudaSuccess;
     const size_t smem = sizeof(double) * 3 * (size_t)max_ld;
-    cudaError_t err = cudaFuncSetAttribute(cluster_fix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t err = allow_smem<cluster_fix_kernel>();
     if (err != cudaSuccess) return err;
     cluster_fix_kernel<<<batch, kCfThreads, smem, st>>>(d_desc, d_d, d_e, d_w, d_ctol, d_Z, d_zscale,
                                                          d_scratch);
