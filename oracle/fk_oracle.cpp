@@ -3,7 +3,7 @@
 // TEST INFRASTRUCTURE ONLY. This file restates, in plain C++ (no Eigen, no
 // ALPSCore, no Boost), the reference algorithm of aeantipov/fk_mc for the path
 // that the GPU library replaces. Only tests/, __graft_entry__.smoke() and the
-// CPU-baseline legs of bench.py load it, and only as the checker / the timed
+// CPU-baseline legs of bench.py load it, and only as the oracle / the timed
 // CPU baseline. The product (fk_mc_gb300/) never links or calls it.
 //
 // What is restated, with the reference lines it follows:

@@ -1,7 +1,7 @@
 """ctypes wrapper around the CPU oracle (oracle/fk_oracle.cpp).
 
 TEST INFRASTRUCTURE ONLY: imported by tests/, by __graft_entry__.smoke() as the
-checker, and by bench.py's CPU-baseline legs. The product package
+oracle, and by bench.py's CPU-baseline legs. The product package
 (fk_mc_gb300) never imports this module.
 """
 import ctypes
